@@ -45,7 +45,8 @@ __device__ __forceinline__ double cr_powi(double x, int n) {
         n >>= 1;
         if (n) a = (a.lo == 0.0) ? dd_sq(a.hi) : dd_mul(a, a);
     }
-    if (!isfinite(r.hi)) return r.hi;
+    // overflow (the low parts are NaN then): infinity, as the reference's powf
+    if (!isfinite(r.hi)) return (n & 1) && x < 0.0 ? -INFINITY : INFINITY;
     return __dadd_rn(r.hi, r.lo);
 }
 // x^(1/4): sqrt(sqrt(x)) is within one ulp; of it and its two neighbours pick
