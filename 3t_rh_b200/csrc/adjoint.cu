@@ -681,7 +681,7 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
     }
 }
 
-__global__ void __launch_bounds__(FLUX_THREADS, 2) k_adj_flux(const Inst* __restrict__ insts,
+__global__ void __launch_bounds__(ADJ_FLUX_THREADS, 2) k_adj_flux(const Inst* __restrict__ insts,
                                                            const Tile* __restrict__ tx, int ntx,
                                                            const Tile* __restrict__ ty, int nty,
                                                            const double* __restrict__ Xb,
@@ -1550,7 +1550,7 @@ void launch_adj_l(cudaStream_t s, const Inst* insts, int k0, int n, long long ma
                                                                                                   X, slots);
     const unsigned cb = (unsigned)((max_cells + 127) / 128);
     if (ntx + nty > 0)
-        k_adj_flux<<<ntx + nty, FLUX_THREADS, sizeof(AdjFluxShared), s>>>(insts, tx, ntx, ty, nty, X, rbar, W);
+        k_adj_flux<<<ntx + nty, ADJ_FLUX_THREADS, sizeof(AdjFluxShared), s>>>(insts, tx, ntx, ty, nty, X, rbar, W);
     if (ntr > 0) k_adj_cells<<<ntr, RHS_THREADS, ADJ_CELL_SMEM, s>>>(insts, tr, ntr, X, rbar, W, pbar);
     const int nbh = (nh + AG_WARPS - 1) / AG_WARPS, nbc = (nc + AG_WARPS * 32 - 1) / (AG_WARPS * 32);
     if (nbh + nbc > 0)

@@ -131,7 +131,14 @@ int make_tiles(rh3t_ctx* c) {
 int enqueue_flux(rh3t_ctx* c, cudaStream_t s, int stage, Span r) {
     const HostInst &a = c->hi[r.k0], &b = c->hi[r.k1 - 1];
     const int ntx = b.tx0 + b.ntx - a.tx0, nty = b.ty0 + b.nty - a.ty0;
-    launch_flux(s, c->d_inst, c->d_tx + a.tx0, ntx, c->d_ty + a.ty0, nty, stage);
+    FluxSize z{0, 0, false};
+    for (int k = r.k0; k < r.k1; ++k) {
+        const HostInst& H = c->hi[k];
+        z.npx = std::max(z.npx, flux_points(0, H.shape.lgx));
+        z.npy = std::max(z.npy, flux_points(1, H.shape.lgy));
+        z.diffusion = z.diffusion || H.diffusion;
+    }
+    launch_flux(s, c->d_inst, c->d_tx + a.tx0, ntx, c->d_ty + a.ty0, nty, stage, z);
     return flux_launches(ntx, nty);
 }
 
@@ -228,6 +235,27 @@ struct Built {
     int n_heavy = 0;
 };
 
+// Tile shapes of an nx x ny grid before any tuning: the default, unless another
+// shape covers the grid in a tenth fewer tiles (a 1024 x 8 strip: cells in 64
+// tiles of 16 x 16 instead of 128 of 8 x 32).
+Shape default_shape(long nx, long ny) {
+    auto tiles = [](long n, long m, int area, int lg) {
+        const long rows = area >> lg, cols = 1L << lg;
+        return ((n + rows - 1) / rows) * ((m + cols - 1) / cols);
+    };
+    auto pick = [](int lo, int hi, int def, auto cost) {
+        int best = def;
+        for (int lg = lo; lg <= hi; ++lg)
+            if (cost(lg) < cost(best) && 10 * cost(lg) < 9 * cost(def)) best = lg;
+        return best;
+    };
+    Shape s;
+    s.lgx = pick(FX_LG_MIN, FX_LG_MAX, FX_LG_DEF, [&](int lg) { return tiles(nx + 1, ny, FLUX_FACES, lg); });
+    s.lgy = pick(FY_LG_MIN, FY_LG_MAX, FY_LG_DEF, [&](int lg) { return tiles(nx, ny + 1, FLUX_FACES, lg); });
+    s.lgr = pick(RHS_LG_MIN, RHS_LG_MAX, RHS_LG_DEF, [&](int lg) { return tiles(nx, ny, RHS_THREADS, lg); });
+    return s;
+}
+
 // Validates one instance description and resolves its ghost records
 // (ghost.rs:18-46, bc1.rs:50-57 and the static parts of the cheap BCs).
 int build_instance(const rh3t_instance& d, int inst, HostInst& H, Inst& I, Built& B, std::string& err) {
@@ -246,6 +274,7 @@ int build_instance(const rh3t_instance& d, int inst, HostInst& H, Inst& I, Built
     const long long plane = (long long)nxp * nyp;
     H.grid = *grid;
     H.nx = nx; H.ny = ny; H.nyp = nyp; H.plane = plane;
+    H.shape = default_shape(nx, ny);
     H.fluid.assign(d.fluid, d.fluid + (size_t)nx * ny);
     const uint8_t* fluid = H.fluid.data();
     I = Inst{};

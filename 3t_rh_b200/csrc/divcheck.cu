@@ -3,7 +3,9 @@
 // the device: random ones, divisors with all-ones significands, quotients
 // next to a rounding midpoint, operands at and beyond the fast path's
 // exponent range, and special values; and the reciprocals of a face's
-// L-row divisors that roe_div (physics.cuh) forms by scaling 1/(12 c^2).
+// L-row divisors that roe_div (physics.cuh) forms by scaling 1/(12 c^2). The
+// branch-free routines are checked on the same operands wherever their range
+// tests accept them.
 #include <cstdint>
 
 #include <cuda_runtime.h>
@@ -42,6 +44,25 @@ __device__ __forceinline__ bool same_bits(double x, double y) {
 }
 
 constexpr int DIV_CATEGORIES = 7;
+
+// the branch-free quotient of case (a, b), or `want` where its range tests
+// refuse the operands (a / 3 and a / 6: any finite a, subnormals among them)
+__device__ __forceinline__ double near_quotient(int cat, double a, double b, double want) {
+    if (cat == 4 || cat == 5) {
+        if (!isfinite(a)) return want;
+        // the same operand scaled into the subnormal range and its edge
+        const int sh = (int)((unsigned)__double2loint(a) % 120u) - 1070;
+        const double t = scalbn(a, sh - ilogb(a));
+        const double got3 = div3_near(t), got6 = div6_near(t);
+        if (cat == 4 && !same_bits(got3, __ddiv_rn(t, 3.0))) return got3;
+        if (cat == 5 && num6_near(t) && !same_bits(got6, __ddiv_rn(t, 6.0))) return got6;
+        return cat == 4 ? div3_near(a) : (num6_near(a) ? div6_near(a) : want);
+    }
+    if (!den_near(b) || !num_near(a)) return want;
+    const double q = div_near(a, recip_near(b));
+    if (!same_bits(q, want)) return q;
+    return a > 0.0 ? div_once(a, b) : q;
+}
 
 // category of case k: 0 random, 1 all-ones divisors, 2 near-midpoint
 // quotients, 3 range edges and special values, 4 a / 3, 5 a / 6, 6 the
@@ -106,6 +127,7 @@ __global__ void k_div_check(long long n, unsigned long long seed, unsigned long 
         if (cat == 4) got = div3_rn(a);
         else if (cat == 5) got = div6_rn(a);
         else got = div_rn(a, recip(b));
+        if (same_bits(got, want)) got = near_quotient(cat, a, b, want);
         if (!same_bits(got, want)) {
             atomicAdd(&bad[cat], 1ull);
             if (atomicAdd(&bad[DIV_CATEGORIES], 1ull) == 0) {

@@ -106,4 +106,100 @@ __device__ __forceinline__ double div6_rn(double a) {
     return __fma_rn(r, y, q);
 }
 
+// ---------------------------------------------------------------- branch-free form
+// The same quotients without a branch each: the caller tests the operands of
+// a whole group of divisions once (den_near for the divisors, num_near or a
+// bound of its own for the numerators) and takes the routines above, or IEEE
+// divisions, for the group that fails. A branch per quotient made each
+// division a basic block of its own, a chain of five dependent FP64 operations
+// with nothing to overlap it; in this form the scheduler interleaves the
+// chains of a group.
+//
+// recip_near(b): the PTX approximation rcp.approx.ftz.f64 (it reads the upper
+// 32 bits of b; |1 - b y| <= 2^-19.9, measured over all 2^20 leading fractions
+// and both extremes of the lower word) and two Newton steps y <- y + y (1 - b y),
+// each by two FMAs: the error before the last rounding is 2^-79, so y lies
+// within (1/2 + 2^-26) ulp of 1/b. The argument above then holds with
+// |K| <= (1 + 2^-25) B / 2, and with |R| <= (1/2 + 2^-51) B (q1 is that close
+// to z): |R K 2^-104| < B^2 2^-106 (1 + 2^-24) < 1 for every B below
+// 2^53 (1 - 2^-20). den_near refuses the divisors above that (leading 20
+// fraction bits all ones).
+//
+// With yl = (1 - b y) y, the reciprocal y + yl holds 1/b to 2^-100, and
+// q = RN(a y + a yl) is within (1/2 + 2^-50) ulp of z: faithful in two operations,
+// so the one correction that follows rounds correctly (the argument above
+// with this q for q1): four operations a quotient instead of five. The
+// quotient's sign is the numerator's (b > 0), set explicitly because a zero
+// numerator would lose it; den_near refuses b <= 0.
+struct RecipN {
+    double b, y, yl;
+};
+__device__ __forceinline__ RecipN recip_near(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    double e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, e, y);
+    e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, e, y);
+    e = __fma_rn(-b, y, 1.0);
+    return {b, y, __dmul_rn(e, y)};
+}
+
+// b > 0, exponent in [-450, 450], leading 20 fraction bits not all ones
+__device__ __forceinline__ bool den_near(double b) {
+    const unsigned h = (unsigned)__double2hiint(b);
+    return h - 0x23d00000u <= 0x384fffffu && (h & 0xfffffu) != 0xfffffu;
+}
+
+// a is zero, or its exponent is in [-450, 450]
+__device__ __forceinline__ bool num_near(double a) {
+    const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return h - 0x23d00000u <= 0x384fffffu || (h | (unsigned)__double2loint(a)) == 0u;
+}
+
+// a / d.b, correctly rounded
+__device__ __forceinline__ double div_near(double a, const RecipN& d) {
+    const double q = __fma_rn(a, d.y, __dmul_rn(a, d.yl));
+    const double r = __fma_rn(-d.b, q, a);
+    const double z = __fma_rn(r, d.y, q);
+    return __hiloint2double((__double2hiint(z) & 0x7fffffff) | (__double2hiint(a) & 0x80000000), __double2loint(z));
+}
+
+// c / b, correctly rounded, for one quotient by b (c > 0): the reciprocal's
+// low part would serve this quotient alone, so the correction runs twice
+// instead
+__device__ __forceinline__ double div_once(double c, double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    double e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, e, y);
+    e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, e, y);
+    double q = __dmul_rn(c, y);
+    double r = __fma_rn(-b, q, c);
+    q = __fma_rn(r, y, q);
+    r = __fma_rn(-b, q, c);
+    return __fma_rn(r, y, q);
+}
+
+// a / 3 for every finite a (the residual taken as 3 q - a and the correction
+// as -y, so that a zero numerator keeps its sign): the residual is a small
+// multiple of ulp(q), or of 2^-1074, so it is exact down to the subnormals, where a / 3 is
+// never a tie. a / 6 likewise, except that a subnormal quotient can be a
+// tie: for a zero or |a| >= 2^-1000 (num6_near).
+__device__ __forceinline__ double div3_near(double a) {
+    const double y = 0x1.5555555555555p-2;
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(3.0, q, -a), -y, q);
+}
+__device__ __forceinline__ double div6_near(double a) {
+    const double y = 0x1.5555555555555p-3;
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(6.0, q, -a), -y, q);
+}
+__device__ __forceinline__ bool num6_near(double a) {
+    const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return h >= 0x01700000u || (h | (unsigned)__double2loint(a)) == 0u;
+}
+
 } // namespace rh3t

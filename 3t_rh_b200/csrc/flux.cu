@@ -1,25 +1,35 @@
 // Interface fluxes (main.rs:165-246: weno.rs:685-802 reconstruction_fast per
 // x and y face, plus diffusion.rs:27-50 when diffusion is on).
 //
-// A block of 6 warps covers 64 faces (a TI x TJ tile, shape chosen per tile)
-// in three phases:
+// A block of two warps covers 64 faces (a TI x TJ tile, shape chosen per
+// tile), one face per thread:
 //   1. staging: the tile's stencil points (x faces: (TI + 5) x TJ points,
 //      y faces: TI x (TJ + 5)) with their primitives and physical flux go to
 //      shared memory once (the reference evaluates them once per face, six
-//      times per point); then each face's Roe state, from the staged
-//      primitives of its points 3 and 2, and its activity flag;
-//   2. characteristic pass: a warp takes one characteristic field c for
-//      32 faces (one per lane) at a time, two (field, half) pairs per warp,
-//      so the row of L, the projections and the two WENO5 reconstructions
-//      of f+ and f- are warp-uniform code; g_c goes to shared memory;
-//   3. output pass: likewise one component k for 32 faces at a time,
-//      returning (R g)_k = sum_c R[k][c] g_c in the reference's summation
+//      times per point);
+//   2. face: each thread forms its face's Roe state from the staged
+//      primitives of its points 3 and 2;
+//   3. characteristic pass: field by field (warp-uniform code), the row of
+//      L, the projections and the two WENO5 reconstructions of f+ and f-;
+//   4. output pass: (R g)_k = sum_c R[k][c] g_c in the reference's summation
 //      order (weno.rs:793, 834-843), plus the diffusion flux for k >= 3.
-// Point data sit in shared memory as component pairs (double2), so a lane
-// reads a point's state and flux with six 16-byte loads.
+//
+// Bound by the FP64 pipe (72% busy in the no-contraction build; a loop of
+// independent FMAs reaches 92%), at about 2,850 FP64 operations a face. A face
+// per thread instead of a field per warp: nothing but the staged points
+// crosses threads, so the two warps meet one barrier of equal work (with six
+// warps each on other fields the barriers were the top stall, 2.1-2.6 warps per
+// issued instruction), and the quotients a face's rows share are formed once.
+// 8 blocks of 128 registers: 10 blocks of 96 spill (3% slower), 6 blocks of 150
+// 4% slower. Without a branch per quotient (divrn.cuh) and in this form the 24
+// batch instances' fluxes take 1.30 ms a step instead of 2.08 ms, the
+// 961 x 3841 half-cylinder's 4.75 ms instead of 7.44 ms (same bits); FMA build
+// 0.94 ms instead of 1.17 ms.
 //
 // RH3T_EXACT selects the reference's expressions; otherwise the fastm forms
 // (shared reciprocals, one division per WENO5) are used.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "physics.cuh"
@@ -32,20 +42,42 @@ constexpr bool kExact = true;
 constexpr bool kExact = false;
 #endif
 
-// Roe state: u v w2 ee ei er cs2 cs he hi hr b den, then the reciprocals
-// the L rows divide by: FMA build 1/cs2, 1/b; no-contraction build RN(1/d)
-// of d = den, b, 6 cs2, 3 cs2, gt cs2 (their quotients stay the IEEE ones)
-constexpr int NQ = 18;
-
+// Shared memory of a block, sized for the launch's largest tile (npt points):
+//   pt: per point seven double2: the state (rho, mx) (my, ee) (ei, er), the
+//       physical flux, (u, v). 112 bytes: the 16-byte loads of consecutive
+//       points fall in different banks;
+//   E:  per point e_e, e_i, e_r, sqrt(rho), for the Roe averages; then G, the
+//       six g_c of a face;
+//   Q:  per face the Roe state u v w2 ee ei er cs2 cs he hi hr b den, then
+//       the reciprocals the L rows divide by: no-contraction build
+//       (recip_near, both parts) of den, b, gt cs2; FMA build 1/cs2, 1/b;
+//   T:  per point te, ti, tr (launches with a diffusive instance);
+//   gkgt, y6: no-contraction build, gk / gt and the reciprocal of 6 gk (both
+//       parts) for gk = ge, gi, gr.
+constexpr int NQ = kExact ? 19 : 15, PT = 7;
 struct FluxShared {
-    double2 U[3][FLUX_NPT]; // (rho, mx), (my, ee), (ei, er)
-    double2 F[3][FLUX_NPT];
-    double T[3][FLUX_NPT];
-    double PR[5][FLUX_NPT]; // u, v, e_e, e_i, e_r of each point (the face Roe averages reuse them)
-    double Q[NQ][FLUX_FACES];
-    double G[6][FLUX_FACES];
-    int act[FLUX_FACES];
+    double2* pt;
+    double *E, *G, *Q, *T, *gkgt, *y6;
+    int npt;
 };
+__host__ __device__ __forceinline__ int flux_e_doubles(int npt) {
+    return 4 * npt > 6 * FLUX_FACES ? 4 * npt : 6 * FLUX_FACES;
+}
+__host__ __device__ __forceinline__ int flux_smem(int npt, bool diffusion) {
+    return npt * PT * 16 + 8 * (flux_e_doubles(npt) + NQ * FLUX_FACES + 10 + (diffusion ? 3 * npt : 0));
+}
+__device__ __forceinline__ FluxShared flux_shared(unsigned char* smem, int npt) {
+    FluxShared S;
+    S.npt = npt;
+    S.pt = reinterpret_cast<double2*>(smem);
+    S.Q = reinterpret_cast<double*>(S.pt + npt * PT);
+    S.gkgt = S.Q + NQ * FLUX_FACES;
+    S.y6 = S.gkgt + 3;
+    S.E = S.gkgt + 10;
+    S.G = S.E;
+    S.T = S.E + flux_e_doubles(npt);
+    return S;
+}
 
 // face f of the tile -> face (i, j), first stencil point p0 and point stride
 template <int DIR>
@@ -57,42 +89,29 @@ __device__ __forceinline__ void face_index(const Tile& t, int f, int& i, int& j,
     else { p0 = r * ((1 << t.lg) + 5) + cc; ps = 1; }
 }
 
-__device__ __forceinline__ void load_q(const FluxShared& S, int f, Roe& q, double& ics2, double& ib) {
-    q.u = S.Q[0][f]; q.v = S.Q[1][f]; q.w2 = S.Q[2][f]; q.ee = S.Q[3][f]; q.ei = S.Q[4][f];
-    q.er = S.Q[5][f]; q.cs2 = S.Q[6][f]; q.cs = S.Q[7][f]; q.he = S.Q[8][f]; q.hi = S.Q[9][f];
-    q.hr = S.Q[10][f]; q.b = S.Q[11][f]; q.den = S.Q[12][f];
-    ics2 = S.Q[13][f]; ib = S.Q[14][f];
+// Qf: the face's column of Q (stride FLUX_FACES)
+__device__ __forceinline__ void load_q(const double* Qf, Roe& q) {
+    constexpr int F = FLUX_FACES;
+    q.u = Qf[0]; q.v = Qf[F]; q.w2 = Qf[2 * F]; q.ee = Qf[3 * F]; q.ei = Qf[4 * F]; q.er = Qf[5 * F];
+    q.cs2 = Qf[6 * F]; q.cs = Qf[7 * F]; q.he = Qf[8 * F]; q.hi = Qf[9 * F]; q.hr = Qf[10 * F]; q.b = Qf[11 * F];
+    q.den = Qf[12 * F];
 }
 
-template <int DIR>
-__device__ __forceinline__ double char_flux(const FluxShared& S, const DevParams& P, const Recip& rgt, int c, int f,
-                                            int p0, int ps) {
-    Roe q;
-    double ics2, ib;
-    load_q(S, f, q, ics2, ib);
-    double Lc[6];
-    if (kExact) {
-        RoeDiv rd;
-        const double gt = (P.gamma_i - 1.0) + (P.gamma_e - 1.0) + (P.gamma_r - 1.0);
-        rd.den = recip_of(q.den, S.Q[13][f]);
-        rd.b = recip_of(q.b, S.Q[14][f]);
-        rd.c6 = recip_of(6.0 * q.cs2, S.Q[15][f]);
-        rd.c3 = recip_of(3.0 * q.cs2, S.Q[16][f]);
-        rd.cg = recip_of(gt * q.cs2, S.Q[17][f]);
-        rd.gt = rgt;
-        l_row<DIR>(c, q, rd, P, Lc);
-    } else {
-        fastm::l_row<DIR>(c, q, ics2, ib, P, Lc);
-    }
+template <int DIR> __device__ __forceinline__ double char_speed(int c, const Roe& q) {
     const double vel = DIR == 0 ? q.u : q.v;
-    const double lam = c == 0 ? vel - q.cs : (c == 5 ? vel + q.cs : vel);
-    const double a = fabs(lam);
-    double fp[6], fm[6];
+    return fabs(c == 0 ? vel - q.cs : (c == 5 ? vel + q.cs : vel));
+}
+
+// f+ and f- of field c at the six points (weno.rs:760-780): L . f, L . u and
+// the Lax-Friedrichs split with speed a. pf: the face's first point, ps the
+// point stride in double2
+__device__ __forceinline__ void split_fluxes(const double2* pf, int ps, const double Lc[6], double a, double fp[6],
+                                             double fm[6]) {
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-        const int p = p0 + k * ps;
-        const double2 u01 = S.U[0][p], u23 = S.U[1][p], u45 = S.U[2][p];
-        const double2 f01 = S.F[0][p], f23 = S.F[1][p], f45 = S.F[2][p];
+        const double2* p = pf + k * ps;
+        const double2 u01 = p[0], u23 = p[1], u45 = p[2];
+        const double2 f01 = p[3], f23 = p[4], f45 = p[5];
         const double cf = Lc[0] * f01.x + Lc[1] * f01.y + Lc[2] * f23.x + Lc[3] * f23.y + Lc[4] * f45.x +
                           Lc[5] * f45.y;
         const double cs = Lc[0] * u01.x + Lc[1] * u01.y + Lc[2] * u23.x + Lc[3] * u23.y + Lc[4] * u45.x +
@@ -100,12 +119,40 @@ __device__ __forceinline__ double char_flux(const FluxShared& S, const DevParams
         fp[k] = 0.5 * (cf + a * cs);
         fm[k] = 0.5 * (cf - a * cs);
     }
-    if (!kExact)
-        return fastm::weno5(fp[0], fp[1], fp[2], fp[3], fp[4], P.eps) +
-               fastm::weno5(fm[5], fm[4], fm[3], fm[2], fm[1], P.eps);
-    // no-contraction build: the two reconstructions as a two-pass loop over
-    // one inlined WENO5 (one copy of its code, no call: the out-of-line
-    // version spilled registers around each of its calls and ran 3% slower)
+}
+
+// the same for the transverse field, whose row of L is (-w, 0, 1, 0, 0, 0), w
+// the transverse velocity, with the 1 at the transverse momentum
+// (finite data: the four products by 0 add zeros)
+template <int DIR>
+__device__ __forceinline__ void split_transverse(const double2* pf, int ps, double w, double a, double fp[6],
+                                                 double fm[6]) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const double2* p = pf + k * ps;
+        const double cf = DIR == 0 ? -w * p[3].x + p[4].x : -w * p[3].x + p[3].y;
+        const double cs = DIR == 0 ? -w * p[0].x + p[1].x : -w * p[0].x + p[0].y;
+        fp[k] = 0.5 * (cf + a * cs);
+        fm[k] = 0.5 * (cf - a * cs);
+    }
+}
+
+// index of an energy row's gk (0 for the other rows, which do not use it)
+template <int DIR> __device__ __forceinline__ int energy_index(int c) {
+    const int mode = row_mode<DIR>(c);
+    return mode < 2 || mode == 5 ? 0 : mode - 2;
+}
+
+// Quotients with a test and a fallback each (divrn.cuh), out of line: faces
+// with operands outside the branch-free form's range
+template <int DIR>
+static __device__ __noinline__ double char_flux_each(const double2* pf, int ps, const double* Qf, const DevParams& P,
+                                                     int c, double gkgt) {
+    Roe q;
+    double Lc[6], fp[6], fm[6];
+    load_q(Qf, q);
+    l_row<DIR>(c, q, roe_div(q, P), gkgt, P, Lc);
+    split_fluxes(pf, ps, Lc, char_speed<DIR>(c, q), fp, fm);
     double r0 = 0.0, r1 = 0.0;
 #pragma unroll 1
     for (int s = 0; s < 2; ++s) {
@@ -118,15 +165,46 @@ __device__ __forceinline__ double char_flux(const FluxShared& S, const DevParams
     return r0 + r1;
 }
 
+// g_c; near: the face's quotients are within the branch-free form's range
+template <int DIR>
+__device__ __forceinline__ double char_flux(const double2* pf, int ps, const double* Qf, const DevParams& P, int c,
+                                            const double* gkgt, bool near) {
+    Roe q;
+    load_q(Qf, q);
+    double Lc[6], fp[6], fm[6];
+    const double a = char_speed<DIR>(c, q);
+    if (row_mode<DIR>(c) == 1) {
+        split_transverse<DIR>(pf, ps, DIR == 0 ? q.v : q.u, a, fp, fm);
+    } else if (kExact) {
+        RoeDivN rd;
+        const double gt = (P.gamma_i - 1.0) + (P.gamma_e - 1.0) + (P.gamma_r - 1.0);
+        rd.den = {q.den, Qf[13 * FLUX_FACES], Qf[14 * FLUX_FACES]};
+        rd.b = {q.b, Qf[15 * FLUX_FACES], Qf[16 * FLUX_FACES]};
+        rd.cg = {gt * q.cs2, Qf[17 * FLUX_FACES], Qf[18 * FLUX_FACES]};
+        rd.scale();
+        l_row<DIR>(c, q, rd, gkgt[energy_index<DIR>(c)], P, Lc);
+        split_fluxes(pf, ps, Lc, a, fp, fm);
+    } else {
+        fastm::l_row<DIR>(c, q, Qf[13 * FLUX_FACES], Qf[14 * FLUX_FACES], P, Lc);
+        split_fluxes(pf, ps, Lc, a, fp, fm);
+    }
+    if (!kExact)
+        return fastm::weno5(fp[0], fp[1], fp[2], fp[3], fp[4], P.eps) +
+               fastm::weno5(fm[5], fm[4], fm[3], fm[2], fm[1], P.eps);
+    const double r0 = weno5_near(fp[0], fp[1], fp[2], fp[3], fp[4], P.eps, near);
+    const double r1 = weno5_near(fm[5], fm[4], fm[3], fm[2], fm[1], P.eps, near);
+    return near ? r0 + r1 : char_flux_each<DIR>(pf, ps, Qf, P, c, gkgt[energy_index<DIR>(c)]);
+}
+
 // The diffusion terms (off in most runs) are out of line: their code stays
 // out of the instruction cache of runs without diffusion.
-// diffusion.rs:27-50: component 3 <- Te, 4 <- Ti, 5 <- Tr^4 (m3 = 0, 1, 2)
-static __device__ __noinline__ void diffusion_out(const FluxShared& S, const DevParams& P, int m3, int p0, int ps,
-                                                  double* out) {
+// diffusion.rs:27-50: component 3 <- Te, 4 <- Ti, 5 <- Tr^4 (m3 = 0, 1, 2); T:
+// the temperature at the face's first point, ps the point stride
+static __device__ __noinline__ void diffusion_out(const double* T, int ps, const DevParams& P, int m3, double* out) {
     double v[6];
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-        const double x = S.T[m3][p0 + m * ps];
+        const double x = T[m * ps];
         v[m] = m3 == 2 ? pow4d(x) : x;
     }
     const double kap = m3 == 0 ? P.kappa_e : (m3 == 1 ? P.kappa_i : P.kappa_r);
@@ -134,159 +212,169 @@ static __device__ __noinline__ void diffusion_out(const FluxShared& S, const Dev
     *out = term / 180.0;
 }
 
-// temperatures of staged point p (its state was written to S.U by this thread)
-static __device__ __noinline__ void stage_temps(FluxShared& S, int p, const DevParams& P) {
-    const double s[6] = {S.U[0][p].x, S.U[0][p].y, S.U[1][p].x, S.U[1][p].y, S.U[2][p].x, S.U[2][p].y};
-    double te, ti, tr;
-    temps_from_state(s, P, te, ti, tr);
-    S.T[0][p] = te; S.T[1][p] = ti; S.T[2][p] = tr;
+// temperatures of a staged point
+static __device__ __noinline__ void stage_temps(const double2* p, const DevParams& P, double* T, int npt) {
+    const double s[6] = {p[0].x, p[0].y, p[1].x, p[1].y, p[2].x, p[2].y};
+    temps_from_state(s, P, T[0], T[npt], T[2 * npt]);
 }
 
+// (R g)_k in the reference's summation order (weno.rs:793, 834-843); Gf: the
+// face's column of G
+template <int DIR, bool NEAR>
+__device__ __forceinline__ double r_dot(const Roe& q, const double* Gf, const double* y6, const DevParams& P, int k) {
+    double Rr[6];
+    RecipN r6k = {1.0, 1.0, 0.0};
+    if (NEAR && k >= 3) {
+        const double gk = (k == 3 ? P.gamma_e : (k == 4 ? P.gamma_i : P.gamma_r)) - 1.0;
+        r6k = {6.0 * gk, y6[k - 3], y6[k]};
+    }
+    r_row<DIR, NEAR>(k, q, r6k, P, Rr);
+    constexpr int F = FLUX_FACES;
+    return Rr[0] * Gf[0] + Rr[1] * Gf[F] + Rr[2] * Gf[2 * F] + Rr[3] * Gf[3 * F] + Rr[4] * Gf[4 * F] +
+           Rr[5] * Gf[5 * F];
+}
 template <int DIR>
-__device__ __forceinline__ void face_out(const Inst& I, const FluxShared& S, const Tile& t, int k, int f) {
-    const DevParams& P = I.P;
-    const int nx = I.nx, ny = I.ny;
-    int i, j, p0, ps;
-    face_index<DIR>(t, f, i, j, p0, ps);
+static __device__ __noinline__ double r_dot_each(const double* Qf, const double* Gf, const DevParams& P, int k) {
     Roe q;
-    double ics2, ib;
-    load_q(S, f, q, ics2, ib);
-    double Rr[6], lam_unused;
-    r_row<DIR>(k, q, P, Rr, lam_unused);
-    const double out = Rr[0] * S.G[0][f] + Rr[1] * S.G[1][f] + Rr[2] * S.G[2][f] + Rr[3] * S.G[3][f] +
-                       Rr[4] * S.G[4][f] + Rr[5] * S.G[5][f];
-    long long fplane, fidx;
-    double *fo, *dfo;
-    if (DIR == 0) { fplane = (long long)(nx + 1) * ny; fidx = (long long)i * ny + j; fo = I.fx; dfo = I.dfx; }
-    else { fplane = (long long)nx * (ny + 1); fidx = (long long)i * (ny + 1) + j; fo = I.fy; dfo = I.dfy; }
-    fo[k * fplane + fidx] = out;
-    if (I.diffusion && k >= 3) diffusion_out(S, P, k - 3, p0, ps, dfo + (k - 3) * fplane + fidx);
+    load_q(Qf, q);
+    return r_dot<DIR, false>(q, Gf, nullptr, P, k);
 }
 
 template <int DIR>
-__device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stage, FluxShared& S) {
+__device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stage, const FluxShared& S) {
     const DevParams& P = I.P;
     const double* __restrict__ buf = stage_src(I, stage);
     const long long plane = I.plane;
-    const int nx = I.nx, ny = I.ny;
+    const int nx = I.nx, ny = I.ny, npt = S.npt;
     const int cols = 1 << t.lg, rows = FLUX_FACES >> t.lg;
     const int np = DIR == 0 ? (rows + 5) * cols : rows * (cols + 5);
     const bool diff = I.diffusion != 0;
-    // ---- 1. staging: points (state, primitives, physical flux), then faces
-    for (int p = threadIdx.x; p < np; p += blockDim.x) {
+    if (kExact && threadIdx.x < 3) {
+        const int k = threadIdx.x;
+        const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
+        const double gk = k == 0 ? ge : (k == 1 ? gi : gr);
+        S.gkgt[k] = __ddiv_rn(gk, gi + ge + gr);
+        const RecipN r = recip_near(6.0 * gk);
+        S.y6[k] = r.y;
+        S.y6[3 + k] = r.yl;
+    }
+    // ---- 1. staging: state, primitives and physical flux of every point
+    for (int p = threadIdx.x; p < np; p += FLUX_THREADS) {
         int pi, pj;
         if (DIR == 0) { pi = t.i - 3 + (p >> t.lg); pj = t.j0 + (p & (cols - 1)); }
         else { const int r = p / (cols + 5); pi = t.i + r; pj = t.j0 - 3 + (p - r * (cols + 5)); }
         double s[6] = {1.0, 0.0, 0.0, 1.0, 1.0, 1.0};
         if (pi >= -RH3T_PAD && pi < nx + RH3T_PAD && pj >= -RH3T_PAD && pj < ny + RH3T_PAD)
             load6(buf, plane, node_of(I, pi, pj), s);
-        Prim d = kExact ? prim_from_state(s, P) : fastm::prim(s, P);
+        const Prim d = kExact ? prim_from_state(s, P) : fastm::prim(s, P);
         double f[6];
         phys_flux<DIR>(s, d, f);
+        double2* q = S.pt + PT * p;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            S.U[k][p] = make_double2(s[2 * k], s[2 * k + 1]);
-            S.F[k][p] = make_double2(f[2 * k], f[2 * k + 1]);
+            q[k] = make_double2(s[2 * k], s[2 * k + 1]);
+            q[3 + k] = make_double2(f[2 * k], f[2 * k + 1]);
         }
-        S.PR[0][p] = d.u; S.PR[1][p] = d.v; S.PR[2][p] = d.e_e; S.PR[3][p] = d.e_i; S.PR[4][p] = d.e_r;
-        if (diff) stage_temps(S, p, P);
+        q[6] = make_double2(d.u, d.v);
+        S.E[p] = d.e_e; S.E[npt + p] = d.e_i; S.E[2 * npt + p] = d.e_r; S.E[3 * npt + p] = sqrt(s[0]);
+        if (diff) stage_temps(q, P, S.T + p, npt);
+    }
+    // ---- 2. this thread's face
+    const int f = threadIdx.x;
+    int i, j, p0, ps;
+    face_index<DIR>(t, f, i, j, p0, ps);
+    bool valid = DIR == 0 ? (i <= nx && j < ny) : (i < nx && j <= ny);
+    if (valid) {
+        const uint8_t m0 = I.mask[node_of(I, i, j)];
+        const uint8_t m1 = DIR == 0 ? I.mask[node_of(I, i - 1, j)] : I.mask[node_of(I, i, j - 1)];
+        valid = (m0 | m1) != 0;
     }
     __syncthreads();
-    for (int f = threadIdx.x; f < FLUX_FACES; f += blockDim.x) {
-        int i, j, p0, ps;
-        face_index<DIR>(t, f, i, j, p0, ps);
-        bool valid = DIR == 0 ? (i <= nx && j < ny) : (i < nx && j <= ny);
-        if (valid) {
-            const uint8_t m0 = I.mask[node_of(I, i, j)];
-            const uint8_t m1 = DIR == 0 ? I.mask[node_of(I, i - 1, j)] : I.mask[node_of(I, i, j - 1)];
-            valid = (m0 | m1) != 0;
-        }
-        S.act[f] = valid ? 1 : 0;
-        if (!valid) continue;
-        // points[3] and points[2] of the face: the staged states and primitives
-        // (the same functions of the same states as a fresh evaluation)
+    double* Qf = S.Q + f;
+    bool near = true;
+    if (valid) {
+        // points[3] and points[2] of the face: the staged primitives (the
+        // same functions of the same states as a fresh evaluation)
         const int p3 = p0 + 3 * ps, p2 = p0 + 2 * ps;
+        const double2 v3 = S.pt[PT * p3 + 6], v2 = S.pt[PT * p2 + 6];
         Prim d3, d2;
-        d3.u = S.PR[0][p3]; d3.v = S.PR[1][p3]; d3.e_e = S.PR[2][p3]; d3.e_i = S.PR[3][p3]; d3.e_r = S.PR[4][p3];
-        d2.u = S.PR[0][p2]; d2.v = S.PR[1][p2]; d2.e_e = S.PR[2][p2]; d2.e_i = S.PR[3][p2]; d2.e_r = S.PR[4][p2];
-        const double rho3 = S.U[0][p3].x, rho2 = S.U[0][p2].x;
+        d3.u = v3.x; d3.v = v3.y; d3.e_e = S.E[p3]; d3.e_i = S.E[npt + p3]; d3.e_r = S.E[2 * npt + p3];
+        d2.u = v2.x; d2.v = v2.y; d2.e_e = S.E[p2]; d2.e_i = S.E[npt + p2]; d2.e_r = S.E[2 * npt + p2];
+        const double rho3 = S.E[3 * npt + p3], rho2 = S.E[3 * npt + p2];
         Roe q;
+        double y[6];
         if (kExact) {
-            q = roe_average(rho3, d3, rho2, d2, P);
+            q = roe_average_sqrt(rho3, d3, rho2, d2, P);
+            RoeDivN rd;
+            const double gt = (P.gamma_i - 1.0) + (P.gamma_e - 1.0) + (P.gamma_r - 1.0);
+            near = near_face(q, gt, rd) & near_params(P);
+            y[0] = rd.den.y; y[1] = rd.den.yl; y[2] = rd.b.y; y[3] = rd.b.yl; y[4] = rd.cg.y; y[5] = rd.cg.yl;
         } else {
-            const double a6[6] = {sqrt(rho3), d3.u, d3.v, d3.e_e, d3.e_i, d3.e_r};
-            const double b6[6] = {sqrt(rho2), d2.u, d2.v, d2.e_e, d2.e_i, d2.e_r};
+            const double a6[6] = {rho3, d3.u, d3.v, d3.e_e, d3.e_i, d3.e_r};
+            const double b6[6] = {rho2, d2.u, d2.v, d2.e_e, d2.e_i, d2.e_r};
             q = fastm::roe(a6, b6, P);
+            y[0] = 1.0 / q.cs2;
+            y[1] = 1.0 / q.b;
         }
-        double qv[NQ] = {q.u, q.v, q.w2, q.ee, q.ei, q.er, q.cs2, q.cs, q.he, q.hi, q.hr, q.b, q.den,
-                         0.0, 0.0, 0.0, 0.0, 0.0};
-        if (kExact) {
-            const RoeDiv rd = roe_div(q, P);
-            qv[13] = rd.den.y; qv[14] = rd.b.y; qv[15] = rd.c6.y; qv[16] = rd.c3.y; qv[17] = rd.cg.y;
-        } else {
-            qv[13] = 1.0 / q.cs2;
-            qv[14] = 1.0 / q.b;
-        }
+        const double qv[13] = {q.u, q.v, q.w2, q.ee, q.ei, q.er, q.cs2, q.cs, q.he, q.hi, q.hr, q.b, q.den};
 #pragma unroll
-        for (int k = 0; k < NQ; ++k) S.Q[k][f] = qv[k];
+        for (int k = 0; k < 13; ++k) Qf[k * FLUX_FACES] = qv[k];
+#pragma unroll
+        for (int k = 13; k < NQ; ++k) Qf[k * FLUX_FACES] = y[k - 13];
     }
-    __syncthreads();
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // Each warp takes one heavy and one light half in both passes, so the
-    // six warps reach the barrier (and the block's end) together: the energy
-    // fields' L rows hold most of a face's divisions (x faces: fields 1-3,
-    // 0 and 5 acoustic, 4 transverse; y faces: 2-4, 0 and 5, 1), and so do
-    // the energy components' R rows (3-5). Field of warp w for faces 0..31
-    // and 32..63, one hex digit per warp:
-    constexpr unsigned kC0 = DIR == 0 ? 0x450321u : 0x150432u;
-    constexpr unsigned kC1 = DIR == 0 ? 0x321450u : 0x432150u;
-    Recip rgt = {1.0, 1.0, false};
-    if (kExact) rgt = recip((P.gamma_i - 1.0) + (P.gamma_e - 1.0) + (P.gamma_r - 1.0));
-    // ---- 2. characteristic pass: field c of faces lane and lane + 32 (a
-    // loop, not unrolled: one copy of the pass's code keeps the kernel
-    // within the instruction cache)
+    __syncthreads(); // E is read; G takes its place
+    if (!valid) return;
+    // ---- 3. characteristic pass (a loop, not unrolled: one copy of its code
+    // stays within the instruction cache)
+    double* Gf = S.G + f;
+    const double2* pf = S.pt + PT * p0;
 #pragma unroll 1
-    for (int h = 0; h < FLUX_FACES / 32; ++h) {
-        const int f = lane + 32 * h;
-        const int c = (int)(((h ? kC1 : kC0) >> (4 * w)) & 15u); // warp-uniform
-        if (S.act[f]) {
-            int i, j, p0, ps;
-            face_index<DIR>(t, f, i, j, p0, ps);
-            S.G[c][f] = char_flux<DIR>(S, P, rgt, c, f, p0, ps);
-        }
-    }
-    __syncthreads();
-    // ---- 3. output pass: component k of faces lane and lane + 32
+    for (int c = 0; c < 6; ++c) Gf[c * FLUX_FACES] = char_flux<DIR>(pf, PT * ps, Qf, P, c, S.gkgt, near);
+    // ---- 4. output pass
+    long long fplane, fidx;
+    double *fo, *dfo;
+    if (DIR == 0) { fplane = (long long)(nx + 1) * ny; fidx = (long long)i * ny + j; fo = I.fx; dfo = I.dfx; }
+    else { fplane = (long long)nx * (ny + 1); fidx = (long long)i * (ny + 1) + j; fo = I.fy; dfo = I.dfy; }
+    if (!kExact || near) {
+        Roe q;
+        load_q(Qf, q);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) fo[k * fplane + fidx] = r_dot<DIR, kExact>(q, Gf, S.y6, P, k);
+    } else {
 #pragma unroll 1
-    for (int h = 0; h < FLUX_FACES / 32; ++h) {
-        const int f = lane + 32 * h;
-        const int k = h ? (w + 3) % 6 : w;
-        if (S.act[f]) face_out<DIR>(I, S, t, k, f);
+        for (int k = 0; k < 6; ++k) fo[k * fplane + fidx] = r_dot_each<DIR>(Qf, Gf, P, k);
     }
+    if (diff)
+#pragma unroll 1
+        for (int m = 0; m < 3; ++m) diffusion_out(S.T + m * npt + p0, ps, P, m, dfo + m * fplane + fidx);
 }
 
-// FMA build: 64 registers, 5 blocks (30 warps) per SM instead of 4 at the
-// uncapped 76. No-contraction build: 80 registers, 4 blocks (its divisions
-// by shared reciprocals keep more values live; at 64 it spills).
-#ifndef FLUX_MIN_BLOCKS_EXACT
-#define FLUX_MIN_BLOCKS_EXACT 4
+// blocks per SM (FMA build: 12 blocks of 80 registers 2% faster than 8)
+#ifndef FLUX_MIN_BLOCKS
+#define FLUX_MIN_BLOCKS (kExact ? 8 : 12)
 #endif
-constexpr int FLUX_MIN_BLOCKS = kExact ? FLUX_MIN_BLOCKS_EXACT : 5;
 // x faces and y faces in two launches: each kernel holds one direction's
 // code, half of what an instruction cache shared by both would need
 template <int DIR>
 __global__ void __launch_bounds__(FLUX_THREADS, FLUX_MIN_BLOCKS) k_flux(const Inst* __restrict__ insts,
-                                                                     const Tile* __restrict__ tiles, int stage) {
-    __shared__ FluxShared S;
+                                                                     const Tile* __restrict__ tiles, int stage,
+                                                                     int npt) {
+    extern __shared__ __align__(16) unsigned char flux_mem[];
     const Tile t = tiles[blockIdx.x];
     const Inst& I = insts[t.inst];
     if (has_error(I)) return;
-    flux_tile<DIR>(I, t, stage, S);
+    flux_tile<DIR>(I, t, stage, flux_shared(flux_mem, npt));
 }
 
-void launch_flux(cudaStream_t s, const Inst* insts, const Tile* tx, int ntx, const Tile* ty, int nty, int stage) {
-    if (ntx > 0) k_flux<0><<<ntx, FLUX_THREADS, 0, s>>>(insts, tx, stage);
-    if (nty > 0) k_flux<1><<<nty, FLUX_THREADS, 0, s>>>(insts, ty, stage);
+int flux_points(int dir, int lg) {
+    const int cols = 1 << lg, rows = FLUX_FACES >> lg;
+    return dir == 0 ? (rows + 5) * cols : rows * (cols + 5);
+}
+
+void launch_flux(cudaStream_t s, const Inst* insts, const Tile* tx, int ntx, const Tile* ty, int nty, int stage,
+                 const FluxSize& z) {
+    if (ntx > 0) k_flux<0><<<ntx, FLUX_THREADS, flux_smem(z.npx, z.diffusion), s>>>(insts, tx, stage, z.npx);
+    if (nty > 0) k_flux<1><<<nty, FLUX_THREADS, flux_smem(z.npy, z.diffusion), s>>>(insts, ty, stage, z.npy);
 }
 
 int flux_launches(int ntx, int nty) { return (ntx > 0 ? 1 : 0) + (nty > 0 ? 1 : 0); }

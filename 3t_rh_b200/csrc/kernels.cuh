@@ -10,8 +10,16 @@ namespace rh3t {
 void launch_ghosts(cudaStream_t s, const Inst* insts, const GhostRec* heavy, int nh, const GhostRec* cheap, int nc,
                    double* hrec, int stage);
 int ghost_launches(int nh, int nc);
+// Shared memory of a flux launch: stencil points of its largest x and y tile
+// (flux_points of direction and shape), and whether an instance has diffusion on
+struct FluxSize {
+    int npx, npy;
+    bool diffusion;
+};
+int flux_points(int dir, int lg);
 // x faces, then y faces: flux_launches() kernels
-void launch_flux(cudaStream_t s, const Inst* insts, const Tile* tx, int ntx, const Tile* ty, int nty, int stage);
+void launch_flux(cudaStream_t s, const Inst* insts, const Tile* tx, int ntx, const Tile* ty, int nty, int stage,
+                 const FluxSize& z);
 int flux_launches(int ntx, int nty);
 void launch_rhs_stage(cudaStream_t s, const Inst* insts, const Tile* tc, int nt, int stage, int mode, double* rhs);
 void launch_dt(cudaStream_t s, const Inst* insts, const Tile* tc, int nt, int mode);

@@ -85,50 +85,110 @@ struct Prim {
     double u, v, e_e, e_i, e_r, pe, pi, pr;
 };
 
-// Every quotient is the IEEE one (divrn.cuh): the five by rho share one
-// reciprocal, w2 / 6 and rho w2 / 6 are each formed once.
-__device__ __forceinline__ Prim prim_from_state(const double s[6], const DevParams& P) {
+// How the quotients of one routine are formed: IEEE divisions by a shared
+// reciprocal with a test (and fallback) each, or the branch-free form whose
+// operands the routine tests as a group (divrn.cuh). The quotients are the
+// same wherever the group's tests hold.
+struct DivEach {
+    bool ok = true;
+    __device__ __forceinline__ Recip den(double b) { return recip(b); }
+    __device__ __forceinline__ double div(double a, const Recip& d) { return div_rn(a, d); }
+    __device__ __forceinline__ double div6(double a) { return div6_rn(a); }
+};
+struct DivGroup {
+    bool ok = true; // every operand so far is within the branch-free form's range
+    __device__ __forceinline__ RecipN den(double b) {
+        ok = ok & den_near(b);
+        return recip_near(b);
+    }
+    __device__ __forceinline__ double div(double a, const RecipN& d) {
+        ok = ok & num_near(a);
+        return div_near(a, d);
+    }
+    __device__ __forceinline__ double div6(double a) {
+        ok = ok & num_near(a);
+        return div6_near(a);
+    }
+};
+
+// The five quotients by rho share one reciprocal, w2 / 6 and rho w2 / 6 are
+// each formed once.
+template <class DV> __device__ __forceinline__ Prim prim_by(const double s[6], const DevParams& P, DV& dv) {
     Prim d;
-    const Recip r0 = recip(s[0]);
-    d.u = div_rn(s[1], r0);
-    d.v = div_rn(s[2], r0);
+    const auto r0 = dv.den(s[0]);
+    d.u = dv.div(s[1], r0);
+    d.v = dv.div(s[2], r0);
     double w2 = sqd(d.u) + sqd(d.v);
-    const double w6 = div6_rn(w2), rw6 = div6_rn(s[0] * w2);
-    d.e_e = div_rn(s[3], r0) - w6;
-    d.e_i = div_rn(s[4], r0) - w6;
-    d.e_r = div_rn(s[5], r0) - w6;
+    const double w6 = dv.div6(w2), rw6 = dv.div6(s[0] * w2);
+    d.e_e = dv.div(s[3], r0) - w6;
+    d.e_i = dv.div(s[4], r0) - w6;
+    d.e_r = dv.div(s[5], r0) - w6;
     d.pe = (P.gamma_e - 1.0) * (s[3] - rw6);
     d.pi = (P.gamma_i - 1.0) * (s[4] - rw6);
     d.pr = (P.gamma_r - 1.0) * (s[5] - rw6);
     return d;
 }
 
-// state.rs:245-276 te, ti, tr (diffusion and source only). r6e, r6i, ra:
-// the instance's divisors 6 cve, 6 cvi and a_rad with their reciprocals
-// (every quotient stays the IEEE one, divrn.cuh)
-__device__ __forceinline__ void temps_from_state(const double s[6], const DevParams& P, const Recip& r6e,
-                                                 const Recip& r6i, const Recip& ra, double& te, double& ti,
-                                                 double& tr) {
-    const Recip r0 = recip(s[0]);
-    double u = div_rn(s[1], r0), v = div_rn(s[2], r0);
-    double w2 = sqd(u) + sqd(v);
-    te = s[3] / (s[0] * P.cve) - div_rn(w2, r6e);
-    ti = s[4] / (s[0] * P.cvi) - div_rn(w2, r6i);
-    double er_term = div_rn(s[5], r0) - div6_rn(w2);
-    tr = cr_pow_quarter(div_rn(er_term * s[0], ra));
+// out of line, in and out by memory: the rare states outside the group range
+static __device__ __noinline__ void prim_each(const double* s, const DevParams& P, Prim* d) {
+    DivEach dv;
+    *d = prim_by(s, P, dv);
 }
 
-// the same values with plain IEEE divisions (callers without the instance's
-// reciprocals at hand)
+__device__ __forceinline__ Prim prim_from_state(const double s[6], const DevParams& P) {
+    DivGroup dv;
+    Prim d = prim_by(s, P, dv);
+    if (!dv.ok) {
+        // an all-zero state (a node no stencil of a fluid cell reaches; the
+        // tiles along a boundary stage many): 0 / 0 in every quotient
+        if (s[0] == 0.0 && s[1] == 0.0 && s[2] == 0.0 && s[3] == 0.0 && s[4] == 0.0 && s[5] == 0.0)
+            return {NAN, NAN, NAN, NAN, NAN, NAN, NAN, NAN};
+        const double t[6] = {s[0], s[1], s[2], s[3], s[4], s[5]};
+        Prim e;
+        prim_each(t, P, &e);
+        d = e;
+    }
+    return d;
+}
+
+// state.rs:245-276 te, ti, tr (diffusion and source only). r6e, r6i, ra: the
+// divisors 6 cve, 6 cvi and a_rad
+template <class DV, class R>
+__device__ __forceinline__ void temps_by(const double s[6], const DevParams& P, const R& r6e, const R& r6i,
+                                         const R& ra, DV& dv, double& te, double& ti, double& er) {
+    const auto r0 = dv.den(s[0]);
+    const double u = dv.div(s[1], r0), v = dv.div(s[2], r0);
+    const double w2 = sqd(u) + sqd(v);
+    te = dv.div(s[3], dv.den(s[0] * P.cve)) - dv.div(w2, r6e);
+    ti = dv.div(s[4], dv.den(s[0] * P.cvi)) - dv.div(w2, r6i);
+    const double er_term = dv.div(s[5], r0) - dv.div6(w2);
+    er = dv.div(er_term * s[0], ra);
+}
+static __device__ __noinline__ void temps_each(const double* s, const DevParams& P, double* t) {
+    DivEach dv;
+    temps_by(s, P, dv.den(6.0 * P.cve), dv.den(6.0 * P.cvi), dv.den(P.a_rad), dv, t[0], t[1], t[2]);
+}
+// r6e, r6i, ra with their reciprocals by recip_near, ok: den_near of the three
+__device__ __forceinline__ void temps_from_state(const double s[6], const DevParams& P, const RecipN& r6e,
+                                                 const RecipN& r6i, const RecipN& ra, bool ok, double& te,
+                                                 double& ti, double& tr) {
+    DivGroup dv;
+    double er;
+    temps_by(s, P, r6e, r6i, ra, dv, te, ti, er);
+    if (!(dv.ok & ok)) {
+        const double t[6] = {s[0], s[1], s[2], s[3], s[4], s[5]};
+        double o[3];
+        temps_each(t, P, o);
+        te = o[0]; ti = o[1]; er = o[2];
+    }
+    tr = cr_pow_quarter(er);
+}
+// the same values for callers without the instance's reciprocals at hand
 __device__ __forceinline__ void temps_from_state(const double s[6], const DevParams& P, double& te, double& ti,
                                                  double& tr) {
-    const Recip r0 = recip(s[0]);
-    double u = div_rn(s[1], r0), v = div_rn(s[2], r0);
-    double w2 = sqd(u) + sqd(v);
-    te = s[3] / (s[0] * P.cve) - w2 / (6.0 * P.cve);
-    ti = s[4] / (s[0] * P.cvi) - w2 / (6.0 * P.cvi);
-    double er_term = div_rn(s[5], r0) - div6_rn(w2);
-    tr = cr_pow_quarter(er_term * s[0] / P.a_rad);
+    DivGroup dv;
+    const RecipN r6e = dv.den(6.0 * P.cve), r6i = dv.den(6.0 * P.cvi), ra = dv.den(P.a_rad);
+    temps_from_state(s, P, r6e, r6i, ra, dv.ok, te, ti, tr);
 }
 
 // state.rs:56-85 flux_from_derived
@@ -153,18 +213,18 @@ template <class T> struct RoeT {
 };
 using Roe = RoeT<double>;
 
-__device__ __forceinline__ Roe roe_average(double rho_s1, const Prim& d3, double rho_s2, const Prim& d2,
-                                           const DevParams& P) {
+template <class DV>
+__device__ __forceinline__ Roe roe_by(double rho1, const Prim& d3, double rho2, const Prim& d2, const DevParams& P,
+                                      DV& dv) {
     Roe q;
-    double rho1 = sqrt(rho_s1), rho2 = sqrt(rho_s2);
     double rho_sum = rho1 + rho2;
-    const Recip rs = recip(rho_sum);
-    q.u = div_rn(d3.u * rho1 + d2.u * rho2, rs);
-    q.v = div_rn(d3.v * rho1 + d2.v * rho2, rs);
+    const auto rs = dv.den(rho_sum);
+    q.u = dv.div(d3.u * rho1 + d2.u * rho2, rs);
+    q.v = dv.div(d3.v * rho1 + d2.v * rho2, rs);
     q.w2 = sqd(q.u) + sqd(q.v);
-    q.ee = div_rn(d3.e_e * rho1 + d2.e_e * rho2, rs);
-    q.ei = div_rn(d3.e_i * rho1 + d2.e_i * rho2, rs);
-    q.er = div_rn(d3.e_r * rho1 + d2.e_r * rho2, rs);
+    q.ee = dv.div(d3.e_e * rho1 + d2.e_e * rho2, rs);
+    q.ei = dv.div(d3.e_i * rho1 + d2.e_i * rho2, rs);
+    q.er = dv.div(d3.e_r * rho1 + d2.e_r * rho2, rs);
     const double GE = P.gamma_e, GI = P.gamma_i, GR = P.gamma_r;
     const double gi = GI - 1.0, ge = GE - 1.0, gr = GR - 1.0;
     const double gt = gi + ge + gr;
@@ -176,6 +236,30 @@ __device__ __forceinline__ Roe roe_average(double rho_s1, const Prim& d3, double
     q.b = gt * (36.0 * ge * gi * gr + gt * sqd(q.w2)) * q.cs2;
     q.den = 12.0 * q.cs2;
     return q;
+}
+
+static __device__ __noinline__ void roe_each(double rho1, const Prim* d3, double rho2, const Prim* d2,
+                                             const DevParams& P, Roe* q) {
+    DivEach dv;
+    *q = roe_by(rho1, *d3, rho2, *d2, P, dv);
+}
+
+// rho1, rho2: the square roots of the two densities
+__device__ __forceinline__ Roe roe_average_sqrt(double rho1, const Prim& d3, double rho2, const Prim& d2,
+                                                const DevParams& P) {
+    DivGroup dv;
+    Roe q = roe_by(rho1, d3, rho2, d2, P, dv);
+    if (!dv.ok) {
+        const Prim a = d3, b = d2;
+        Roe e;
+        roe_each(rho1, &a, rho2, &b, P, &e);
+        q = e;
+    }
+    return q;
+}
+__device__ __forceinline__ Roe roe_average(double rho_s1, const Prim& d3, double rho_s2, const Prim& d2,
+                                           const DevParams& P) {
+    return roe_average_sqrt(sqrt(rho_s1), d3, sqrt(rho_s2), d2, P);
 }
 
 // Mode of left eigenvector row `row`: 0 acoustic-, 1 transverse, 2 electron,
@@ -291,16 +375,16 @@ __device__ __forceinline__ void r_col(int col, const RoeT<T>& q, const DevParams
     }
 }
 
-// Row `row` of the right eigenvector matrix (weno.rs:518-545) and the
-// eigenvalue of characteristic field `row`.
-template <int DIR>
-__device__ __forceinline__ void r_row(int row, const Roe& q, const DevParams& P, double R[6], double& lam) {
+// Row `row` of the right eigenvector matrix (weno.rs:518-545). NEAR: the
+// quotients in the branch-free form, for a face that near_face accepts
+// (r6k: 6 gk with its reciprocal, k = row - 3).
+template <int DIR, bool NEAR>
+__device__ __forceinline__ void r_row(int row, const Roe& q, const RecipN& r6k, const DevParams& P, double R[6]) {
     const double GE = P.gamma_e, GI = P.gamma_i, GR = P.gamma_r;
     const double gi = GI - 1.0, ge = GE - 1.0, gr = GR - 1.0;
     const double gt = gi + ge + gr;
     const double u = q.u, v = q.v, w2 = q.w2, cs = q.cs;
     const double vel = DIR == 0 ? u : v;
-    lam = row == 0 ? vel - cs : (row == 5 ? vel + cs : vel);
     if (row >= 3) {
         // energy components k = 0, 1, 2 (e, i, r): one code path with the
         // component's operands. Entries 0 and 5: Gk ek + w2/6 -+ vel cs / 3;
@@ -312,11 +396,11 @@ __device__ __forceinline__ void r_row(int row, const Roe& q, const DevParams& P,
         const double Gk = k == 0 ? GE : (k == 1 ? GI : GR);
         const double ek = k == 0 ? q.ee : (k == 1 ? q.ei : q.er);
         const double gk = k == 0 ? ge : (k == 1 ? gi : gr);
-        const double base = Gk * ek + div6_rn(w2);
-        const double vc = div3_rn(vel * cs);
+        const double base = Gk * ek + (NEAR ? div6_near(w2) : div6_rn(w2));
+        const double vc = NEAR ? div3_near(vel * cs) : div3_rn(vel * cs);
         R[0] = base - vc;
         R[5] = base + vc;
-        const double dk = gt * w2 / (6.0 * gk);
+        const double dk = NEAR ? div_near(gt * w2, r6k) : gt * w2 / (6.0 * gk);
         const int o = DIR == 0 ? 1 : 2;
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
@@ -324,7 +408,8 @@ __device__ __forceinline__ void r_row(int row, const Roe& q, const DevParams& P,
             const double gl = l == 0 ? ge : (l == 1 ? gi : gr);
             R[o + m] = m == k ? dk : (m == (k + 2) % 3 ? gl : -gl);
         }
-        R[DIR == 0 ? 4 : 1] = div3_rn(DIR == 0 ? v : u);
+        const double vt = DIR == 0 ? v : u;
+        R[DIR == 0 ? 4 : 1] = NEAR ? div3_near(vt) : div3_rn(vt);
     } else if (DIR == 0) {
         switch (row) {
         case 0: R[0] = 1.0; R[1] = 1.0; R[2] = 1.0; R[3] = 1.0; R[4] = 0.0; R[5] = 1.0; break;
@@ -369,10 +454,53 @@ __device__ __forceinline__ RoeDiv roe_div(const Roe& q, const DevParams& P) {
     return r;
 }
 
+// The branch-free form for a whole face: reciprocals of the five divisors
+// (rd), and whether every quotient of its rows of L and R is covered by the
+// argument in divrn.cuh. The divisors are within 2^-100..2^101 and u, v are
+// zero or within 2^-430..2^101, so with the gammas' factors gk, gt within
+// 2^-20..2^21 (near_params) the numerators u, v, w2, vel cs and their
+// multiples by gk, gt, cs are zero or at least 2^-904 and the quotients at least
+// 2^-1005: residuals are multiples of 2^-1008, so nothing underflows.
+__device__ __forceinline__ bool near_params(const DevParams& P) {
+    const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
+    const double lo = 0x1p-20, hi = 0x1p20;
+    return ge >= lo && ge <= hi && gi >= lo && gi <= hi && gr >= lo && gr <= hi && P.eps >= 0x1p-100 &&
+           P.eps <= 0x1p100 && den_near(6.0 * ge) && den_near(6.0 * gi) && den_near(6.0 * gr);
+}
+__device__ __forceinline__ bool near_divisor(double b) {
+    const unsigned h = (unsigned)__double2hiint(b);
+    return h - 0x39b00000u <= 0x0c8fffffu && (h & 0xfffffu) != 0xfffffu;
+}
+__device__ __forceinline__ bool near_velocity(double a) {
+    const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return h - 0x25100000u <= 0x212fffffu || (h | (unsigned)__double2loint(a)) == 0u;
+}
+struct RoeDivN {
+    RecipN den, b, c6, c3, cg;
+    // 6 cs2 and 3 cs2 are den / 2 and den / 4 exactly
+    __device__ __forceinline__ void scale() {
+        c6 = {0.5 * den.b, 2.0 * den.y, 2.0 * den.yl};
+        c3 = {0.25 * den.b, 4.0 * den.y, 4.0 * den.yl};
+    }
+};
+__device__ __forceinline__ bool near_face(const Roe& q, double gt, RoeDivN& rd) {
+    const double cg = gt * q.cs2;
+    rd.den = recip_near(q.den);
+    rd.b = recip_near(q.b);
+    rd.cg = recip_near(cg);
+    return near_divisor(q.den) & near_divisor(q.b) & near_divisor(cg) & near_velocity(q.u) & near_velocity(q.v);
+}
+
+__device__ __forceinline__ double quot(double a, const Recip& d) { return div_rn(a, d); }
+__device__ __forceinline__ double quot(double a, const RecipN& d) { return div_near(a, d); }
+
 // l_row over double with the face's shared divisors: the same expressions
-// as l_row<DIR, T> (weno.rs:79-458), the same roundings.
-template <int DIR>
-__device__ __forceinline__ void l_row(int row, const Roe& q, const RoeDiv& rd, const DevParams& P, double L[6]) {
+// as l_row<DIR, T> (weno.rs:79-458), the same roundings. gkgt: the quotient
+// gk / gt of an energy row. RD: RoeDiv, or RoeDivN for a face that near_face
+// accepts.
+template <int DIR, class RD>
+__device__ __forceinline__ void l_row(int row, const Roe& q, const RD& rd, double gkgt, const DevParams& P,
+                                      double L[6]) {
     const double GE = P.gamma_e, GI = P.gamma_i, GR = P.gamma_r;
     const double gi = GI - 1.0, ge = GE - 1.0, gr = GR - 1.0;
     const double gt = gi + ge + gr;
@@ -383,17 +511,17 @@ __device__ __forceinline__ void l_row(int row, const Roe& q, const RoeDiv& rd, c
         // entries: x + s y with s = +-1 is x + y or x - y exactly
         const double s = mode == 0 ? 1.0 : -1.0;
         if (DIR == 0) {
-            L[0] = div_rn(gt * w2 + s * (6.0 * u * cs), rd.den);
-            L[1] = div_rn(-2.0 * gt * u + -s * (6.0 * cs), rd.den);
-            L[2] = div_rn(-2.0 * gt * v, rd.den);
+            L[0] = quot(gt * w2 + s * (6.0 * u * cs), rd.den);
+            L[1] = quot(-2.0 * gt * u + -s * (6.0 * cs), rd.den);
+            L[2] = quot(-2.0 * gt * v, rd.den);
         } else {
-            L[0] = div_rn(gt * w2 + s * (6.0 * v * cs), rd.den);
-            L[1] = div_rn(-2.0 * gt * u, rd.den);
-            L[2] = div_rn(-2.0 * gt * v + -s * (6.0 * cs), rd.den);
+            L[0] = quot(gt * w2 + s * (6.0 * v * cs), rd.den);
+            L[1] = quot(-2.0 * gt * u, rd.den);
+            L[2] = quot(-2.0 * gt * v + -s * (6.0 * cs), rd.den);
         }
-        L[3] = div_rn(6.0 * ge, rd.den);
-        L[4] = div_rn(6.0 * gi, rd.den);
-        L[5] = div_rn(6.0 * gr, rd.den);
+        L[3] = quot(6.0 * ge, rd.den);
+        L[4] = quot(6.0 * gi, rd.den);
+        L[5] = quot(6.0 * gr, rd.den);
     } else if (mode == 1) {
         if (DIR == 0) { L[0] = -v; L[1] = 0.0; L[2] = 1.0; }
         else { L[0] = -u; L[1] = 1.0; L[2] = 0.0; }
@@ -408,9 +536,9 @@ __device__ __forceinline__ void l_row(int row, const Roe& q, const RoeDiv& rd, c
         const int k = mode - 2;
         const double gk = k == 0 ? ge : (k == 1 ? gi : gr);
         const double hk = k == 0 ? q.he : (k == 1 ? q.hi : q.hr);
-        L[0] = div_rn(gk, rd.gt) - div_rn(gk * w2, rd.c6) - div_rn(gk * gt * w2, rd.b) * (hk - cs2 * w2);
-        L[1] = div_rn(gk * u, rd.c3) + div_rn(2.0 * gk * gt * u, rd.b) * (hk - cs2 * w2);
-        L[2] = div_rn(gk * v, rd.c3) + div_rn(2.0 * gk * gt * v, rd.b) * (hk - cs2 * w2);
+        L[0] = gkgt - quot(gk * w2, rd.c6) - quot(gk * gt * w2, rd.b) * (hk - cs2 * w2);
+        L[1] = quot(gk * u, rd.c3) + quot(2.0 * gk * gt * u, rd.b) * (hk - cs2 * w2);
+        L[2] = quot(gk * v, rd.c3) + quot(2.0 * gk * gt * v, rd.b) * (hk - cs2 * w2);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             const bool diag = j == k;
@@ -420,7 +548,7 @@ __device__ __forceinline__ void l_row(int row, const Roe& q, const RoeDiv& rd, c
             const double t = 6.0 * gl * cs2;
             const double n2 = diag ? 6.0 * gk : 6.0 * gk * gj;
             const double f = diag ? gk * hk - gt * cs2 * w2 : hk + (j == (k + 2) % 3 ? t : -t);
-            L[3 + j] = div_rn(-gk * gj, rd.cg) - div_rn(n2, rd.b) * f;
+            L[3 + j] = quot(-gk * gj, rd.cg) - quot(n2, rd.b) * f;
         }
     }
 }
@@ -558,6 +686,33 @@ __device__ __forceinline__ double weno5(double u0, double u1, double u2, double 
     double p0 = div3_rn(u0) - 7.0 / 6.0 * u1 + 11.0 / 6.0 * u2;
     double p1 = div6_rn(-u1) + 5.0 / 6.0 * u2 + div3_rn(u3);
     double p2 = div3_rn(u2) + 5.0 / 6.0 * u3 - div6_rn(u4);
+    return w0 * p0 + w1 * p1 + w2 * p2;
+}
+
+// weno5 in the branch-free form (divrn.cuh); ok is cleared when an operand is
+// outside its range (then the value is not used). Numerators need no test: the
+// 0.1, 0.6, 0.3 and the alphas they give are bounded by the divisors' range;
+// u / 3 holds for every finite u, and a u that is not finite makes one of the
+// three divisors infinite or NaN.
+__device__ __forceinline__ double weno5_near(double u0, double u1, double u2, double u3, double u4, double eps,
+                                             bool& ok) {
+    // products by 2, 4 and 1/4 are exact, so their sums are one FMA each
+    const double c1312 = 13.0 / 12.0, u23 = __dmul_rn(3.0, u2);
+    const double t2 = __dadd_rn(__fma_rn(-2.0, u3, u2), u4), r2 = __dadd_rn(__fma_rn(-4.0, u3, u23), u4);
+    const double t1 = __dadd_rn(__fma_rn(-2.0, u2, u1), u3), r1 = __dadd_rn(u1, -u3);
+    const double t0 = __dadd_rn(__fma_rn(-2.0, u1, u0), u2), r0 = __dadd_rn(__fma_rn(-4.0, u1, u0), u23);
+    const double beta2 = __fma_rn(0.25, sqd(r2), c1312 * sqd(t2));
+    const double beta1 = __fma_rn(0.25, sqd(r1), c1312 * sqd(t1));
+    const double beta0 = __fma_rn(0.25, sqd(r0), c1312 * sqd(t0));
+    const double s0 = sqd(eps + beta0), s1 = sqd(eps + beta1), s2 = sqd(eps + beta2);
+    const double a0 = div_once(0.1, s0), a1 = div_once(0.6, s1), a2 = div_once(0.3, s2);
+    const double sum_o = a0 + a1 + a2;
+    const RecipN rs = recip_near(sum_o);
+    const double w0 = div_near(a0, rs), w1 = div_near(a1, rs), w2 = div_near(a2, rs);
+    const double p0 = div3_near(u0) - 7.0 / 6.0 * u1 + 11.0 / 6.0 * u2;
+    const double p1 = div6_near(-u1) + 5.0 / 6.0 * u2 + div3_near(u3);
+    const double p2 = div3_near(u2) + 5.0 / 6.0 * u3 - div6_near(u4);
+    ok = ok & den_near(s0) & den_near(s1) & den_near(s2) & den_near(sum_o) & num6_near(u1) & num6_near(u4);
     return w0 * p0 + w1 * p1 + w2 * p2;
 }
 

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(RHS_THREADS, 2) k_rhs_stage(const Inst* __rest
         double s[6];
         load6(src, plane, n, s);
         double te, ti_, tr;
-        temps_from_state(s, P, rhs_recip(I, sR, 4), rhs_recip(I, sR, 5), rhs_recip(I, sR, 6), te, ti_, tr);
+        temps_from_state(s, P, te, ti_, tr);
         const double so[3] = {-P.omega_ei * (te - ti_) - P.omega_er * (pow4d(te) - pow4d(tr)),
                               P.omega_ei * (te - ti_), P.omega_er * (pow4d(te) - pow4d(tr))};
 #pragma unroll

@@ -57,7 +57,8 @@ bool save_cache(const char* path) {
 enum Kind { KX = 0, KY = 1, KR = 2 };
 
 // minimum over `reps` launches of one tile kind over the class's tiles (ms)
-int time_kind(rh3t_ctx* c, Kind kind, const std::vector<Tile>& tiles, int reps, double* ms_out) {
+int time_kind(rh3t_ctx* c, Kind kind, const std::vector<Tile>& tiles, const Shape& sh, bool diffusion, int reps,
+              double* ms_out) {
     *ms_out = 0.0;
     if (tiles.empty()) return RH3T_OK;
     cudaStream_t s = c->stream;
@@ -68,9 +69,10 @@ int time_kind(rh3t_ctx* c, Kind kind, const std::vector<Tile>& tiles, int reps, 
     if (e == cudaSuccess) e = cudaEventCreate(&a);
     if (e == cudaSuccess) e = cudaEventCreate(&b);
     const int n = (int)tiles.size();
+    const FluxSize z{flux_points(0, sh.lgx), flux_points(1, sh.lgy), diffusion};
     auto launch = [&]() {
-        if (kind == KX) launch_flux(s, c->d_inst, d, n, nullptr, 0, 0);
-        else if (kind == KY) launch_flux(s, c->d_inst, nullptr, 0, d, n, 0);
+        if (kind == KX) launch_flux(s, c->d_inst, d, n, nullptr, 0, 0, z);
+        else if (kind == KY) launch_flux(s, c->d_inst, nullptr, 0, d, n, 0, z);
         else launch_rhs_stage(s, c->d_inst, d, n, 0, 0, c->d_io2);
         c->launches += 1;
     };
@@ -156,7 +158,7 @@ extern "C" int rh3t_autotune(rh3t_ctx* c, const char* cache_path, int32_t reps, 
                         instance_tiles(c->hi[k], sh, k, kind == KX ? &tiles : nullptr,
                                        kind == KY ? &tiles : nullptr, kind == KR ? &tiles : nullptr);
                     double t = 0.0;
-                    int rc = time_kind(c, (Kind)kind, tiles, reps, &t);
+                    int rc = time_kind(c, (Kind)kind, tiles, sh, kv.first.diffusion != 0, reps, &t);
                     if (rc) return rc;
                     ms[kind][lg - lo[kind]] = t;
                     if (t < tbest) { tbest = t; pick[kind] = lg; }
