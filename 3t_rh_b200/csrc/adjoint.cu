@@ -906,7 +906,6 @@ constexpr int AG_WARPS = 3;
 constexpr int AG_LR_THREADS = 128;
 constexpr int AG_RB = 80;
 __constant__ int kAStOff[6] = {0, 1, 5, 14, 30, 55};
-__constant__ int kASOff[6] = {0, 1, 17, 98, 354, 979};
 __constant__ int kAWOff[6] = {0, 1, 9, 36, 100, 225};
 
 
@@ -921,7 +920,10 @@ struct AdjGhostWarp {
     double vb[5][6];
     double Z[6][6];
     double omm[6][5]; // omega_r * omega-bar_r per field
+    double w[226];    // w_{r,k}, term b at kAWOff[r] + k m + b (kept from the dot products)
 };
+static_assert(sizeof(AdjGhostWarp) % 16 == 0, "rows of D stay 16-byte aligned");
+constexpr int AG_SMEM = AG_WARPS * (int)sizeof(AdjGhostWarp); // four blocks per SM
 
 __device__ __forceinline__ int aorder(int a) { return a < 1 ? 0 : (a < 5 ? 1 : (a < 14 ? 2 : (a < 30 ? 3 : 4))); }
 
@@ -1130,51 +1132,51 @@ __device__ __noinline__ bool wall_outflow_vjp(const Inst& I, const GhostRec& Rg,
     return true;
 }
 
-// two rows of one order of the record (S_r transposed, stride m, or w_{r,k},
-// stride 1; read from global memory, prefetched to L2) with the stencil
-// data d, all six fields: an S row stores (S_r d_c)_a, a w row V^(k)_{c,r}
-__device__ __forceinline__ void adj_dot_pair(AdjGhostWarp& G, const double* __restrict__ rec, unsigned codes) {
-    if (codes == kPairNone) return;
-    const unsigned c1 = codes & 0xffffu, c2 = codes >> 16;
-    const int r = (int)((c1 >> 5) & 7u), m = (r + 1) * (r + 1);
-    const int i1 = (int)(c1 & 31u), i2 = (int)(c2 & 31u);
-    const bool w1 = (c1 >> 8) != 0, w2 = (c2 >> 8) != 0;
-    const double* __restrict__ p1 = w1 ? rec + GH_W + kAWOff[r] + i1 * m : rec + GH_S + kASOff[r] + i1;
-    const double* __restrict__ p2 = w2 ? rec + GH_W + kAWOff[r] + i2 * m : rec + GH_S + kASOff[r] + i2;
-    const int s1 = w1 ? 1 : m, s2 = w2 ? 1 : m;
+// a pair of rows of one order of the record (read from global memory,
+// prefetched to L2) with the stencil data d, all six fields: an S row stores
+// (S_r d_c)_a, a w row V^(k)_{c,r}
+__device__ __forceinline__ void adj_dot_pair(AdjGhostWarp& G, const double* __restrict__ rec, unsigned code) {
+    if (code == kPairNone) return;
+    const int r = (int)(code >> 8), quad = (int)(code >> 4) & 15, h = (int)code & 15, m = (r + 1) * (r + 1);
+    const int R1 = r < 2 ? 2 * quad : quad_row(r, quad, 2 * h), R2 = r < 2 ? R1 + 1 : quad_row(r, quad, 2 * h + 1);
+    const bool w1 = R1 >= m, w2 = R2 >= m;
+    const int i1 = w1 ? R1 - m : R1, i2 = w2 ? R2 - m : R2;
+    const double2* __restrict__ rows = reinterpret_cast<const double2*>(rec + GH_ROWS);
+    // places of the pair's chunks: three runs of terms (orders 1 and 0 in the first)
+    const int s0 = r == 1 ? 3 : 31, o0 = r == 0 ? GR_ORDER0 : (r == 1 ? GR_ORDER1 + quad : quad_chunk(r, quad, h, 0));
+    const int o1 = quad_chunk(r, quad, h, 9) - 25 * 9, o2 = quad_chunk(r, quad, h, 16) - 15 * 16;
+    auto chunk = [&](int b) { return __ldg(rows + (b < 9 ? o0 + s0 * b : (b < 16 ? o1 + 25 * b : o2 + 15 * b))); };
     const double(*__restrict__ D)[6] = G.D + kDOff[r];
     double a1[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, a2[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     // the record is read from L2: the loads of the next four terms are in
     // flight while four terms are summed (in order)
     constexpr int PF = 4;
-    double x1[PF], x2[PF];
+    double2 x[PF];
 #pragma unroll
-    for (int j = 0; j < PF; ++j) {
-        x1[j] = j < m ? __ldg(p1 + j * s1) : 0.0;
-        x2[j] = j < m ? __ldg(p2 + j * s2) : 0.0;
-    }
+    for (int j = 0; j < PF; ++j) x[j] = j < m ? chunk(j) : make_double2(0.0, 0.0);
     for (int b0 = 0; b0 < m; b0 += PF) {
-        double y1[PF], y2[PF];
+        double2 y[PF];
 #pragma unroll
         for (int j = 0; j < PF; ++j) {
             const int bn = b0 + PF + j;
-            y1[j] = bn < m ? __ldg(p1 + bn * s1) : 0.0;
-            y2[j] = bn < m ? __ldg(p2 + bn * s2) : 0.0;
+            y[j] = bn < m ? chunk(bn) : make_double2(0.0, 0.0);
         }
 #pragma unroll
         for (int j = 0; j < PF; ++j) {
             if (b0 + j < m) {
                 double d[6];
                 load_d6(D[b0 + j], d);
+                if (w1) G.w[kAWOff[r] + i1 * m + b0 + j] = x[j].x;
+                if (w2) G.w[kAWOff[r] + i2 * m + b0 + j] = x[j].y;
 #pragma unroll
                 for (int c = 0; c < 6; ++c) {
-                    a1[c] += x1[j] * d[c];
-                    a2[c] += x2[j] * d[c];
+                    a1[c] += x[j].x * d[c];
+                    a2[c] += x[j].y * d[c];
                 }
             }
         }
 #pragma unroll
-        for (int j = 0; j < PF; ++j) { x1[j] = y1[j]; x2[j] = y2[j]; }
+        for (int j = 0; j < PF; ++j) x[j] = y[j];
     }
     const int off = kAStOff[r];
 #pragma unroll
@@ -1366,16 +1368,15 @@ __device__ void ghost_vjp_warp(const Inst& I, const GhostRec& Rg, const double* 
         for (int k = 0; k < 5; ++k) G.V[oc][orr][k] = om * G.vb[k][oc];                 // now V-bar
     }
     __syncwarp();
-    // D-bar over the 55 nodes: beta = d^T S d, V = w . d (the w columns of
-    // both of a lane's nodes are loaded together)
+    // D-bar over the 55 nodes: beta = d^T S d, V = w . d
     {
         const int r0 = aorder(lane), m0 = (r0 + 1) * (r0 + 1), ar0 = lane - kAStOff[r0];
         const int ar1 = lane + 32 - kAStOff[4]; // the second node is of order 4
         double wv0[5], wv1[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
-            wv0[k] = k <= r0 ? __ldg(&rec[GH_W + kAWOff[r0] + k * m0 + ar0]) : 0.0;
-            wv1[k] = lane + 32 < 55 ? __ldg(&rec[GH_W + kAWOff[4] + k * 25 + ar1]) : 0.0;
+            wv0[k] = k <= r0 ? G.w[kAWOff[r0] + k * m0 + ar0] : 0.0;
+            wv1[k] = lane + 32 < 55 ? G.w[kAWOff[4] + k * 25 + ar1] : 0.0;
         }
         for (int c = 0; c < 6; ++c) {
             double acc = G.beta[c][r0] * (2.0 * G.ACC[c][lane]);
@@ -1485,7 +1486,8 @@ __global__ void __launch_bounds__(AG_WARPS * 32, 5) k_adj_ghosts(const Inst* __r
                                                              const double* __restrict__ Wb,
                                                              double* __restrict__ Ubb, double* __restrict__ pbar,
                                                              double* __restrict__ slots, int nbh) {
-    __shared__ AdjGhostWarp G[AG_WARPS];
+    extern __shared__ __align__(16) unsigned char ag_smem[];
+    AdjGhostWarp* G = reinterpret_cast<AdjGhostWarp*>(ag_smem);
     const int lane = threadIdx.x & 31;
     if ((int)blockIdx.x < nbh) {
         const int g = blockIdx.x * AG_WARPS + (threadIdx.x >> 5);
@@ -1543,6 +1545,8 @@ void launch_adj_l(cudaStream_t s, const Inst* insts, int k0, int n, long long ma
         cudaFuncSetAttribute(k_adj_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_CELL_SMEM);
         cudaFuncSetAttribute(k_adj_flux, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjFluxShared));
         cudaFuncSetAttribute(k_adj_ghost_lr, cudaFuncAttributeMaxDynamicSharedMemorySize, AG_LR_SMEM);
+        cudaFuncSetAttribute(k_adj_ghosts<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AG_SMEM);
+        cudaFuncSetAttribute(k_adj_ghosts<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AG_SMEM);
         attr = true;
     }
     if (nh > 0)
@@ -1554,10 +1558,10 @@ void launch_adj_l(cudaStream_t s, const Inst* insts, int k0, int n, long long ma
     if (ntr > 0) k_adj_cells<<<ntr, RHS_THREADS, ADJ_CELL_SMEM, s>>>(insts, tr, ntr, X, rbar, W, pbar);
     const int nbh = (nh + AG_WARPS - 1) / AG_WARPS, nbc = (nc + AG_WARPS * 32 - 1) / (AG_WARPS * 32);
     if (nbh + nbc > 0)
-        k_adj_ghosts<false><<<nbh + nbc, AG_WARPS * 32, 0, s>>>(insts, heavy, nh, cheap, nc, hrec, X, W, Ub, pbar,
+        k_adj_ghosts<false><<<nbh + nbc, AG_WARPS * 32, AG_SMEM, s>>>(insts, heavy, nh, cheap, nc, hrec, X, W, Ub, pbar,
                                                                  slots, nbh);
     if (wall_outflow && nbh > 0)
-        k_adj_ghosts<true><<<nbh, AG_WARPS * 32, 0, s>>>(insts, heavy, nh, cheap, 0, hrec, X, W, Ub, pbar, slots, nbh);
+        k_adj_ghosts<true><<<nbh, AG_WARPS * 32, AG_SMEM, s>>>(insts, heavy, nh, cheap, 0, hrec, X, W, Ub, pbar, slots, nbh);
     if (nh > 0) k_adj_ghost_tail<<<(nh + 127) / 128, 128, 0, s>>>(insts, heavy, nh, X, slots, Ub);
     k_adj_fluid<<<dim3(cb, n), 128, 0, s>>>(insts, k0, W, Ub);
 }

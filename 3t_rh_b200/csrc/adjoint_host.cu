@@ -119,7 +119,7 @@ void enqueue_recorded_step(rh3t_ctx* c, double* rec) {
     int nh, nc;
     ghost_ranges(c, nh, nc);
     for (int st = 0; st < 3; ++st) {
-        launch_ghosts(s, c->d_inst, c->d_gpart, nh, c->d_gpart + c->n_gheavy, nc, c->d_hrec, st);
+        launch_ghosts(s, c->d_inst, c->d_gpart, nh, c->d_gpart + c->n_gheavy, nc, c->d_hrec, c->d_lr, st);
         launch_adj_copy(s, c->d_inst, 0, c->n_inst, mp, st, rec + st * np, 0);
         const int nf = enqueue_flux(c, s, st, r);
         enqueue_rhs(c, s, st, 2, rec + (3 + st) * np, r);
@@ -147,7 +147,7 @@ extern "C" int rh3t_l_vjp(rh3t_ctx* c, int32_t k, const double* rbar, double* ub
     CK(c, cudaMemcpyAsync(&sc->t_stage[0], &sc->t_after, sizeof(double), cudaMemcpyDeviceToDevice, s));
     int nh, nc;
     ghost_ranges(c, nh, nc);
-    launch_ghosts(s, c->d_inst, c->d_gpart, nh, c->d_gpart + c->n_gheavy, nc, c->d_hrec, 0);
+    launch_ghosts(s, c->d_inst, c->d_gpart, nh, c->d_gpart + c->n_gheavy, nc, c->d_hrec, c->d_lr, 0);
     launch_adj_copy(s, c->d_inst, 0, c->n_inst, max_plane(c), 0, a->U2, 0); // X = U2 as scratch
     CK(c, cudaMemsetAsync(a->rbar, 0, np * sizeof(double), s));
     CK(c, cudaMemsetAsync(a->U0, 0, np * sizeof(double), s));

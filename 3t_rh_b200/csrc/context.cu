@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "context.h"
+#include "ghost_rows.cuh"
 #include "kernels.cuh"
 
 using namespace rh3t;
@@ -163,7 +164,7 @@ int enqueue_ghosts(rh3t_ctx* c, cudaStream_t s, int stage, Span r) {
     const HostInst& a = c->hi[r.k0];
     int nh, nc;
     ghost_counts(c, r, nh, nc);
-    launch_ghosts(s, c->d_inst, c->d_gpart + a.gh0, nh, c->d_gpart + c->n_gheavy + a.gc0, nc, c->d_hrec, stage);
+    launch_ghosts(s, c->d_inst, c->d_gpart + a.gh0, nh, c->d_gpart + c->n_gheavy + a.gc0, nc, c->d_hrec, c->d_lr, stage);
     return ghost_launches(nh, nc);
 }
 
@@ -367,19 +368,23 @@ int build_instance(const rh3t_instance& d, int inst, HostInst& H, Inst& I, Built
             R.src = R.node;
         }
     }
-    // heavy records: S | w | d | pad | stencil nodes
+    // heavy records: rows of S and w | d | pad | stencil nodes
     B.hrec.assign((size_t)nh * GH_REC, 0.0);
+    std::vector<int> place; // of S (979 values), then w (225), in the record's rows
+    if (nh) {
+        place.reserve(1204);
+        for (int q = 0; q < 5; ++q) // S_q row-major
+            for (int a = 0; a < (q + 1) * (q + 1); ++a)
+                for (int b = 0; b < (q + 1) * (q + 1); ++b) place.push_back(row_place(q, a, b));
+        for (int q = 0; q < 5; ++q) // w_{q,k}
+            for (int k = 0; k <= q; ++k)
+                for (int b = 0; b < (q + 1) * (q + 1); ++b) place.push_back(row_place(q, (q + 1) * (q + 1) + k, b));
+    }
     for (int k = 0; k < nh; ++k) {
         double* r = B.hrec.data() + (size_t)k * GH_REC;
-        // S_r transposed per order (the kernel reads column b of all rows a)
-        static const int soff[5] = {0, 1, 17, 98, 354};
-        const double* S = gt->s + (size_t)k * 979;
-        for (int q = 0; q < 5; ++q) {
-            const int m = (q + 1) * (q + 1);
-            for (int a = 0; a < m; ++a)
-                for (int b = 0; b < m; ++b) r[GH_S + soff[q] + b * m + a] = S[soff[q] + a * m + b];
-        }
-        std::memcpy(r + GH_W, gt->w + (size_t)k * 225, 225 * sizeof(double));
+        const double *S = gt->s + (size_t)k * 979, *w = gt->w + (size_t)k * 225;
+        for (int e = 0; e < 979; ++e) r[GH_ROWS + place[e]] = S[e];
+        for (int e = 0; e < 225; ++e) r[GH_ROWS + place[979 + e]] = w[e];
         std::memcpy(r + GH_D, gt->d + (size_t)k * 5, 5 * sizeof(double));
         int32_t st[56] = {0};
         for (int a = 0; a < 55; ++a) {
@@ -684,6 +689,7 @@ extern "C" int rh3t_batch_create(int32_t n, const rh3t_instance* desc, int32_t d
     DA(c->d_ghosts, std::max(c->n_ghosts, 1));
     DA(c->d_gpart, std::max(c->n_ghosts, 1));
     DA(c->d_hrec, std::max((long long)c->n_heavy * GH_REC, 1LL));
+    DA(c->d_lr, std::max((long long)c->n_heavy * GH_LR, 1LL));
     DA(c->d_io, c->total_cells * 6);
     DA(c->d_io2, (c->total_cells + c->max_ghosts) * 6); // rhs planes, then ghost values
 #undef DA
@@ -765,7 +771,7 @@ extern "C" void rh3t_destroy(rh3t_ctx* c) {
         if (x) cudaStreamDestroy(x);
     if (c->h_sc) cudaFreeHost(c->h_sc);
     dfree(c->d_state); dfree(c->d_mask); dfree(c->d_faces); dfree(c->d_bcs); dfree(c->d_sc); dfree(c->d_err);
-    dfree(c->d_times); dfree(c->d_inst); dfree(c->d_ghosts); dfree(c->d_gpart); dfree(c->d_hrec);
+    dfree(c->d_times); dfree(c->d_inst); dfree(c->d_ghosts); dfree(c->d_gpart); dfree(c->d_hrec); dfree(c->d_lr);
     dfree(c->d_tx); dfree(c->d_ty); dfree(c->d_tc); dfree(c->d_tr); dfree(c->d_io); dfree(c->d_io2);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;

@@ -54,6 +54,7 @@ struct rh3t_ctx {
     rh3t::GhostRec* d_ghosts = nullptr; // table order (instance-major, gid within)
     rh3t::GhostRec* d_gpart = nullptr;  // heavy ghosts by heavy slot, then the cheap ones
     double* d_hrec = nullptr;           // heavy records (GH_REC doubles each)
+    double* d_lr = nullptr;             // ghost update's scratch (GH_LR doubles per heavy record)
     rh3t::Tile* d_tx = nullptr;
     rh3t::Tile* d_ty = nullptr;
     rh3t::Tile* d_tc = nullptr;

@@ -1,12 +1,46 @@
 // The 70 dot products of a heavy ghost's WENO extrapolation (bc1.rs:221-244)
-// with its stencil data d (rows of S_0..S_4 and w_{r,k}), scheduled over the
-// 32 lanes of a warp as pairs of rows of one order, and the row layout of d
-// that keeps the loads of different orders in different shared-memory banks.
-// Used by the ghost update (ghosts.cu) and its vector-Jacobian product
-// (adjoint.cu).
+// with its stencil data d (rows of S_0..S_4 and w_{r,k}): how the rows lie in
+// the ghost's record, and the row layout of d that keeps the loads of different
+// orders in different shared-memory banks. Used by the ghost update
+// (ghosts.cu), its vector-Jacobian product (adjoint.cu) and the packing of
+// the records (context.cu).
+//
+// The rows of order r are S_r's (r+1)^2 rows, then w_{r,0..r}. The ghost update
+// gives a ghost 16 lanes, four rows of one order (a quad) each: lanes 0-6 and 15
+// order 4 (lane 15 its last two rows), 7-11 order 3, 12-14 order 2; quad_row
+// orders a quad's rows so that the rows of D which the lanes touch together lie
+// in different shared-memory banks. Term by term a quad is stored as two
+// 16-byte chunks of two rows; at term b the lanes' first chunks lie side by
+// side, then their second ones, so each load of a half-warp is one contiguous
+// run: terms 0-8 hold 16 + 15 chunks (all lanes), 9-15 13 + 12 (orders 4, 3),
+// 16-24 8 + 7 (order 4). Orders 1 (3 pairs x 4 terms) and 0 (1 pair) follow.
 #pragma once
 
 namespace rh3t {
+
+constexpr int GR_SEG1 = 9 * 31, GR_SEG2 = GR_SEG1 + 7 * 25, GR_ORDER1 = GR_SEG2 + 9 * 15;
+constexpr int GR_ORDER0 = GR_ORDER1 + 12, GR_CHUNKS = GR_ORDER0 + 1; // 602 chunks of 16 bytes
+
+// row i (0-3) of a quad: rotated by quad / 2, so that D rows 4 quad + (i + quad
+// / 2) mod 4 of eight consecutive quads differ mod 8 (the last quad of order 4
+// holds two rows, both in its first chunk)
+__host__ __device__ constexpr int quad_row(int r, int quad, int i) {
+    return 4 * quad + ((i + (r == 4 && quad == 7 ? 0 : quad >> 1)) & 3);
+}
+// chunk h (0, 1) of a quad of order 2, 3 or 4 at term b
+__host__ __device__ __forceinline__ int quad_chunk(int r, int quad, int h, int b) {
+    const int lane = r == 4 ? (quad < 7 ? quad : 15) : (r == 3 ? 7 + quad : 12 + quad);
+    if (b < 9) return 31 * b + (h ? 16 + lane : lane);
+    if (b < 16) return GR_SEG1 + 25 * (b - 9) + (h ? 13 + lane : (lane == 15 ? 12 : lane));
+    return GR_SEG2 + 15 * (b - 16) + (h ? 8 + lane : (lane == 15 ? 7 : lane));
+}
+// place of term b of row R of order r in the record's rows
+__host__ __device__ __forceinline__ int row_place(int r, int R, int b) {
+    if (r == 0) return 2 * GR_ORDER0 + R;
+    if (r == 1) return 2 * (GR_ORDER1 + 3 * b + (R >> 1)) + (R & 1);
+    const int quad = R >> 2, i = ((R & 3) - (r == 4 && quad == 7 ? 0 : quad >> 1)) & 3;
+    return 2 * quad_chunk(r, quad, i >> 1, b) + (i & 1);
+}
 
 // Row of D holding stencil node a of order r: the order blocks start at
 // kDOff[r], whose residues mod 8 differ, so the 16-byte loads of D rows of
@@ -14,31 +48,21 @@ namespace rh3t {
 static __constant__ int kDOff[5] = {0, 1, 5, 14, 31};
 __host__ __device__ constexpr int d_row(int a) { return a + (a >= 30 ? 1 : 0); }
 
-// Schedule of the 70 dot products with the stencil data d (55 rows of
-// S_0..S_4 and the 15 rows w_{r,k}), all six fields at once, as 35 pairs of
-// rows of one order (one load of a D row serves both), in two slots a warp
-// runs one after the other (25 and 4 terms at most). Row code:
-// w-row flag << 8 | r << 5 | a (S row) or k (w row); 0xffff = none.
-constexpr unsigned short kRowNone = 0xffff;
-__host__ __device__ constexpr unsigned short srow(int r, int a) { return (unsigned short)((r << 5) | a); }
-__host__ __device__ constexpr unsigned short wrow(int r, int k) { return (unsigned short)(0x100 | (r << 5) | k); }
-__host__ __device__ constexpr unsigned pair(unsigned short x, unsigned short y) { return (unsigned)x | ((unsigned)y << 16); }
+// Schedule of the 70 dot products of the vector-Jacobian product, all six
+// fields at once, as the 35 chunks' pairs of rows, in two slots a warp runs one
+// after the other (25 and 4 terms at most): order << 8 | quad << 4 | chunk (orders
+// 1 and 0: the pair for the quad); kPairNone = none
 constexpr unsigned kPairNone = 0xffffffffu;
+__host__ __device__ constexpr unsigned pair(int r, int quad, int h) { return (unsigned)(r << 8 | quad << 4 | h); }
 static __constant__ unsigned kSlotA[32] = {  // orders 4 (lanes 0-14), 3 (15-24), 2 (25-30), 1 (31)
-    pair(srow(4, 0), srow(4, 1)), pair(srow(4, 2), srow(4, 3)), pair(srow(4, 4), srow(4, 5)),
-    pair(srow(4, 6), srow(4, 7)), pair(srow(4, 8), srow(4, 9)), pair(srow(4, 10), srow(4, 11)),
-    pair(srow(4, 12), srow(4, 13)), pair(srow(4, 14), srow(4, 15)), pair(srow(4, 16), srow(4, 17)),
-    pair(srow(4, 18), srow(4, 19)), pair(srow(4, 20), srow(4, 21)), pair(srow(4, 22), srow(4, 23)),
-    pair(srow(4, 24), wrow(4, 0)), pair(wrow(4, 1), wrow(4, 2)), pair(wrow(4, 3), wrow(4, 4)),
-    pair(srow(3, 0), srow(3, 1)), pair(srow(3, 2), srow(3, 3)), pair(srow(3, 4), srow(3, 5)),
-    pair(srow(3, 6), srow(3, 7)), pair(srow(3, 8), srow(3, 9)), pair(srow(3, 10), srow(3, 11)),
-    pair(srow(3, 12), srow(3, 13)), pair(srow(3, 14), srow(3, 15)), pair(wrow(3, 0), wrow(3, 1)),
-    pair(wrow(3, 2), wrow(3, 3)),
-    pair(srow(2, 0), srow(2, 1)), pair(srow(2, 2), srow(2, 3)), pair(srow(2, 4), srow(2, 5)),
-    pair(srow(2, 6), srow(2, 7)), pair(srow(2, 8), wrow(2, 0)), pair(wrow(2, 1), wrow(2, 2)),
-    pair(srow(1, 0), srow(1, 1))};
+    pair(4, 0, 0), pair(4, 0, 1), pair(4, 1, 0), pair(4, 1, 1), pair(4, 2, 0), pair(4, 2, 1), pair(4, 3, 0),
+    pair(4, 3, 1), pair(4, 4, 0), pair(4, 4, 1), pair(4, 5, 0), pair(4, 5, 1), pair(4, 6, 0), pair(4, 6, 1),
+    pair(4, 7, 0),
+    pair(3, 0, 0), pair(3, 0, 1), pair(3, 1, 0), pair(3, 1, 1), pair(3, 2, 0), pair(3, 2, 1), pair(3, 3, 0),
+    pair(3, 3, 1), pair(3, 4, 0), pair(3, 4, 1),
+    pair(2, 0, 0), pair(2, 0, 1), pair(2, 1, 0), pair(2, 1, 1), pair(2, 2, 0), pair(2, 2, 1), pair(1, 0, 0)};
 static __constant__ unsigned kSlotB[32] = {  // the rest of order 1, order 0
-    pair(srow(1, 2), srow(1, 3)), pair(wrow(1, 0), wrow(1, 1)), pair(srow(0, 0), wrow(0, 0)),
+    pair(1, 1, 0), pair(1, 2, 0), pair(0, 0, 0),
     kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone,
     kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone,
     kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone, kPairNone,

@@ -1,39 +1,35 @@
 // Ghost-node update of one RK stage (ghost.rs:199-268 update_values_parallel,
-// bc1.rs:609-928 set_ghost_point_value with precomputed GhostBC data), in
-// two launches.
-//
-// k_ghost_prep, one thread per ghost:
-//   - heavy ghosts (Wall / Outflow / FarField): L, R and lambda at the
-//     nearest fluid node, rotated to the (normal, tangential) frame
-//     (bc1.rs:294-312); every thread runs the same six rows, so no lane waits
-//     on another's branch. The 80 doubles of a ghost go through shared
-//     memory and are stored into its record by whole warps (coalesced);
-//   - cheap ghosts (ReflectiveWall, ZerothOrder, Periodic, Constant,
-//     TimeDependent), six threads each, complete.
-// k_ghosts, heavy ghosts on persistent warps, one ghost at a time per warp.
-// A ghost's record (S_r, w, d, the E_r stencil and this stage's L, R,
-// lambda; 10.5 KB) arrives in shared memory by one bulk copy (cp.async.bulk,
-// completion on an mbarrier). One record buffer per warp: L, R and lambda
-// are copied out of it first, and once step 3 has read S_r and w (and d is
-// in registers) the next ghost's copy is issued into the same buffer, so the
-// table stream overlaps steps 4-6, and 12 warps fit on an SM.
+// bc1.rs:609-928 set_ghost_point_value with precomputed GhostBC data), in one
+// launch. Cheap ghosts (ReflectiveWall, ZerothOrder, Periodic, Constant,
+// TimeDependent) take six threads each at its start.
+// k_ghosts, heavy ghosts on persistent warps, two ghosts at a time per warp, one
+// on each half-warp. A ghost's tables (the rows of S_r and w, d; 9.7 KB)
+// arrive in shared memory by a bulk copy (cp.async.bulk, completion on an
+// mbarrier). One table buffer per half-warp: once step 3 has read the rows
+// (and d is in registers) the next pair's copies are issued into the same
+// buffers, so the table stream overlaps steps 4-6.
 // Per ghost:
-//   1. the E_r stencil states (E_0..E_4, 55 nodes, two per lane) were
-//      gathered while the ghost before was processed; the fetches for the
-//      next ghost are spread over the steps so that none waits on another;
+//   1. L, R and lambda at the nearest fluid node, rotated to the (normal,
+//      tangential) frame (bc1.rs:294-312): for the warp's next 30 ghosts at
+//      once, one per lane (on the lanes of one ghost its six rows, three kinds
+//      of code, took a quarter of the pair's time), staged in the table buffers
+//      and kept in global scratch until the ghost's turn; they and the E_r
+//      stencil states (E_0..E_4, 55 nodes, four per lane) are loaded while the
+//      pair before is processed, the fetches spread over the steps so that none
+//      waits on another;
 //   2. lanes spread over the 55 stencil nodes: rotate the momentum and
 //      project on the six characteristic fields (bc1.rs:209-219);
-//   3. the 70 dot products with the stencil data, all six fields at once,
-//      in three slots of 25, 16 and 4 terms (a fixed per-lane schedule):
-//      the 55 rows of S_0..S_4, each stored as its beta term
-//      d_c,a (S_r d_c)_a, and the 15 rows w_{r,k}, V^(k)_{c,r} = w_{r,k} . d_c
-//      (bc1.rs:221-244); S_r is stored transposed so the lanes of one order
-//      read consecutive words;
+//   3. the 70 dot products with the stencil data, all six fields at once, four
+//      rows of one order per lane (ghost_rows.cuh): the 55 rows of S_0..S_4,
+//      each then stored over the data as its beta term d_c,a (S_r d_c)_a, and
+//      the 15 rows w_{r,k}, V^(k)_{c,r} = w_{r,k} . d_c (bc1.rs:221-244);
+//      orders 1 and 0 by (row, field);
 //   4. lanes (c, r): beta_{c,r} = the sum of its row terms in order and
 //      alpha = d_r / (eps + beta)^q;
-//   5. lanes (k, c): V^(k)_c = sum_r alpha_r / sum(alpha) V_r (bc1.rs:247-252);
-//   6. FarField rows, R products and the Taylor sum on lanes (bc1.rs:829-923);
-//      Wall (two 6x6 LU solves) and Outflow (LODI) on lane 0 (bc1.rs:691-828).
+//   5. lanes (c, r): the weight alpha_r / sum(alpha); lanes (k, c): V^(k)_c =
+//      the weighted sum of V_r (bc1.rs:247-252);
+//   6. FarField rows, R products, the Wall's two 6x6 LU solves (a column per
+//      lane), Outflow's LODI row and the Taylor sum on lanes (bc1.rs:691-923).
 // The per-k loop of the reference (bc1.rs:673-675) recomputes steps 2-4
 // unchanged; they are done once. Every sum keeps the reference's order, so
 // the no-contraction build reproduces the reference's values.
@@ -53,138 +49,159 @@ constexpr bool kExactG = true;
 constexpr bool kExactG = false;
 #endif
 
-constexpr int GH_WARPS = 4;
-constexpr int GH_BLOCKS_PER_SM = 3;
-constexpr int GH_PREP_THREADS = 64; // 41.6 KB of staging per block: 5 blocks per SM
-__constant__ int kStOff[6] = {0, 1, 5, 14, 30, 55};
-__constant__ int kSOff[6] = {0, 1, 17, 98, 354, 979};
-__constant__ int kWOff[6] = {0, 1, 9, 36, 100, 225};
+constexpr int GH_WARPS = 8; // one block per SM
 
-struct GhostWarp {
-    double rec[1][GH_REC]; // the heavy record (the next one is copied in during step 5)
-    double LR[80];         // this ghost's L, R, lambda (copied out of the record)
-    double D[56][6];       // characteristic data d_c at stencil node a, row d_row(a)
-    double ACC[56][6];     // d_c,a (S_r d_c)_a at stencil row a; later u[5][6] and vinf[6]
-    double alpha[6][5];
+struct GhostSlot { // one ghost: half a warp
+    double rec[GH_COPY];   // the tables (the next ones are copied in during step 4)
+    double LR[GH_LR];      // this ghost's L, R, lambda
+    double D[56][6];       // characteristic data d_c at stencil node a, row d_row(a); then d_c,a (S_r d_c)_a; then u
+    double alpha[6][5];    // alpha, then the weights
     double V[6][15];       // [c][r (r + 1) / 2 + k], k <= r
     double v[5][6];        // V^(k)_c
-    GhostRec cur;          // this ghost's GhostRec (copied in while the ghost before it ran)
+    double ui[6], vinf[6]; // FarField state, and L of it
+    GhostRec cur;          // this ghost's GhostRec (copied in while the pair before it ran)
+};
+struct GhostWarp {
+    GhostSlot g[2];
     unsigned long long bar[2];
 };
-static_assert(sizeof(GhostWarp) % 16 == 0, "records stay 16-byte aligned");
+static_assert(sizeof(GhostSlot) % 16 == 0 && sizeof(GhostWarp) % 16 == 0, "tables stay 16-byte aligned");
+static_assert(GH_COPY * 8 % 16 == 0 && GH_REC * 8 % 16 == 0 && 2 * GR_CHUNKS == GH_D, "record layout");
 constexpr int GH_SMEM = GH_WARPS * (int)sizeof(GhostWarp);
-constexpr int GH_LR_R = GH_R - GH_L, GH_LR_LAM = GH_LAM - GH_L;
+static_assert(GH_SMEM <= 232448, "one block per SM");
+constexpr int GH_LR_R = 36, GH_LR_LAM = 72; // of a slot's LR
+constexpr int CHUNK = 15; // pairs whose L, R and lambda are formed together: 78 x 15 values in a slot's rec
+static_assert(78 * CHUNK <= GH_COPY, "a chunk's L, R, lambda fit in the table buffer");
 
 // ---------------------------------------------------------------- bulk copy
-// one thread: expect `bytes` on bar, then copy global -> shared (16-byte
-// aligned addresses, bytes a multiple of 16). The buffer is reused: the
-// proxy fence orders the warp's earlier reads of it (generic proxy, made
-// visible to this thread by the __syncwarp before every call) before the
-// copy's writes (async proxy).
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, unsigned long long* bar) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
+// one thread: expect the tables of two ghosts on bar, then copy them global ->
+// shared (16-byte aligned addresses, sizes a multiple of 16). The buffers are
+// reused: the proxy fence orders the warp's earlier reads of them (generic
+// proxy, made visible to this thread by the __syncwarp before every call)
+// before the copies' writes (async proxy).
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, unsigned long long* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                      smem_u32(dst)),
                  "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
+__device__ __forceinline__ void load_tables(GhostWarp& W, const double* __restrict__ hrec, int heavy0, int heavy1) {
+    constexpr uint32_t bytes = GH_COPY * 8;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&W.bar[0])), "r"(2 * bytes)
+                 : "memory");
+    bulk_copy(W.g[0].rec, hrec + (size_t)heavy0 * GH_REC, bytes, &W.bar[0]);
+    bulk_copy(W.g[1].rec, hrec + (size_t)heavy1 * GH_REC, bytes, &W.bar[0]);
+}
 
-// bc1.rs:467-469 solve6 with LAPACK getrf/getrs semantics
-__device__ bool solve6(double A[6][6], double b[6]) {
-    int piv[6];
+// a / b for operands of any sign, correctly rounded (divrn.cuh: |b| > 0 there)
+__device__ __forceinline__ double quot_any(double a, double b) {
+    const double m = fabs(b);
+    if (den_near(m) && num_near(a)) return div_near(b < 0.0 ? -a : a, recip_near(m));
+    return div_ieee(a, b);
+}
+
+// bc1.rs:467-469 solve6 with LAPACK getrf/getrs semantics (first-maximum
+// pivots, multipliers by the pivot's reciprocal), on one half-warp: lane k < 6
+// holds column k of A in a, lane 6 the right-hand side, which is eliminated with
+// the columns (the same products in the same order as a forward substitution
+// after the factorisation). The solution is left in lane 6's a; returns false on
+// every lane if a pivot is zero. m: the half's lanes, h: its first lane
+__device__ __forceinline__ bool solve6(double a[6], int l, unsigned m, int h) {
+#pragma unroll
     for (int j = 0; j < 6; ++j) {
         int p = j;
-        double mx = fabs(A[j][j]);
+        double mx = fabs(a[j]), pv = a[j];
+#pragma unroll
         for (int i = j + 1; i < 6; ++i)
-            if (fabs(A[i][j]) > mx) { mx = fabs(A[i][j]); p = i; }
-        piv[j] = p;
-        if (A[p][j] == 0.0) return false;
-        if (p != j)
-            for (int k = 0; k < 6; ++k) { double t = A[j][k]; A[j][k] = A[p][k]; A[p][k] = t; }
-        double rcp = 1.0 / A[j][j];
-        for (int i = j + 1; i < 6; ++i) A[i][j] *= rcp;
-        for (int k = j + 1; k < 6; ++k)
-            for (int i = j + 1; i < 6; ++i) A[i][k] -= A[i][j] * A[j][k];
+            if (fabs(a[i]) > mx) { mx = fabs(a[i]); pv = a[i]; p = i; }
+        p = __shfl_sync(m, p, h + j);
+        pv = __shfl_sync(m, pv, h + j);
+        if (pv == 0.0) return false;
+#pragma unroll
+        for (int i = j + 1; i < 6; ++i)
+            if (p == i) { const double t = a[j]; a[j] = a[i]; a[i] = t; }
+        if (j == 5) break;
+        const double rcp = quot_any(1.0, pv);
+#pragma unroll
+        for (int i = j + 1; i < 6; ++i) {
+            const double f = __shfl_sync(m, a[i], h + j) * rcp;
+            if (l == j) a[i] = f;
+            else if (l > j) a[i] -= f * a[j];
+        }
     }
-    for (int j = 0; j < 6; ++j)
-        if (piv[j] != j) { double t = b[j]; b[j] = b[piv[j]]; b[piv[j]] = t; }
-    for (int k = 0; k < 6; ++k)
-        for (int i = k + 1; i < 6; ++i) b[i] -= b[k] * A[i][k];
+#pragma unroll
     for (int k = 5; k >= 0; --k) {
-        b[k] /= A[k][k];
-        for (int i = 0; i < k; ++i) b[i] -= b[k] * A[i][k];
+        const double d = __shfl_sync(m, a[k], h + k);
+        const double x = quot_any(a[k], d);
+#pragma unroll
+        for (int i = 0; i < k; ++i) {
+            const double f = __shfl_sync(m, a[i], h + k);
+            if (l == 6) a[i] -= x * f;
+        }
+        if (l == 6) a[k] = x;
     }
     return true;
 }
 
-// out[i] = sum_j R[i][j] x[j] with R stored by column (Rc[6 j + i])
-__device__ __forceinline__ void r_times(const double* Rc, const double x[6], double* out) {
-    for (int i = 0; i < 6; ++i) {
-        double acc = 0.0;
-        for (int j = 0; j < 6; ++j) acc += Rc[6 * j + i] * x[j];
-        out[i] = acc;
-    }
-}
-
-// Wall (bc1.rs:691-756) and Outflow (bc1.rs:760-828) rows on one lane;
-// fills u[5][6]. Returns false when an ILW system is singular.
-__device__ __noinline__ bool serial_tail(const Inst& I, const GhostRec& Rg, const double* LR,
-                                         const double (*v)[6], double (*u)[6]) {
+// Wall (bc1.rs:691-756): u_0 and u_1 from the two ILW systems; Outflow
+// (bc1.rs:760-828): u_1 with the LODI row. On the half-warp (m, h as above) of
+// a ghost whose u_k = R v_k are in u. Returns false when an ILW system is
+// singular. (On one lane, with the systems in local memory, it took most of a
+// Wall ghost's time: 47 us for the 1,344 Wall ghosts of a double Mach stage.)
+__device__ __noinline__ bool wall_outflow_rows(const Inst& I, const GhostRec& Rg, const double* LR,
+                                               const double (*v)[6], double (*u)[6], int l, unsigned m, int h) {
     const DevParams& P = I.P;
-    const double* L = LR;
-    const double* Rc = LR + GH_LR_R;
+    const double ge = P.gamma_e - 1.0, gi = P.gamma_i - 1.0, gr = P.gamma_r - 1.0;
     if (Rg.kind == BC_WALL) {
-        double A0[6][6], rhs0[6];
-        for (int i = 0; i < 6; ++i)
-            for (int k = 0; k < 6; ++k) A0[i][k] = L[6 * i + k];
-        for (int k = 0; k < 6; ++k) A0[0][k] = k == 1 ? 1.0 : 0.0;
-        for (int k = 0; k < 6; ++k) rhs0[k] = v[0][k];
-        rhs0[0] = 0.0;
-        if (!solve6(A0, rhs0)) return false;
-        for (int k = 0; k < 6; ++k) u[0][k] = rhs0[k];
-        const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
         const double gt = gi + ge + gr;
-        const double u1 = u[0][0], u3 = u[0][2];
-        double row1[6] = {-gt * sqd(u3) / (6.0 * sqd(u1)), 0.0, gt * u3 / (6.0 * u1), -ge, -gi, -gr};
-        double A1[6][6], rhs1[6];
-        for (int i = 0; i < 6; ++i)
-            for (int k = 0; k < 6; ++k) A1[i][k] = L[6 * i + k];
-        for (int k = 0; k < 6; ++k) A1[0][k] = row1[k];
-        for (int k = 0; k < 6; ++k) rhs1[k] = v[1][k];
-        rhs1[0] = 0.0;
-        if (!solve6(A1, rhs1)) return false;
-        for (int k = 0; k < 6; ++k) u[1][k] = rhs1[k];
-        for (int k = 2; k <= 4; ++k) r_times(Rc, v[k], u[k]);
+        double a[6];
+        a[0] = l == 1 ? 1.0 : 0.0;
+#pragma unroll
+        for (int i = 1; i < 6; ++i) a[i] = l < 6 ? LR[6 * i + l] : (l == 6 ? v[0][i] : 0.0);
+        if (!solve6(a, l, m, h)) return false;
+        const double u1 = __shfl_sync(m, a[0], h + 6), u3 = __shfl_sync(m, a[2], h + 6);
+        if (l == 6)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) u[0][k] = a[k];
+        const double q0 = -gt * sqd(u3) / (6.0 * sqd(u1)), q2 = gt * u3 / (6.0 * u1);
+        a[0] = l == 0 ? q0 : (l == 2 ? q2 : (l == 3 ? -ge : (l == 4 ? -gi : (l == 5 ? -gr : 0.0))));
+#pragma unroll
+        for (int i = 1; i < 6; ++i) a[i] = l < 6 ? LR[6 * i + l] : (l == 6 ? v[1][i] : 0.0);
+        if (!solve6(a, l, m, h)) return false;
+        if (l == 6)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) u[1][k] = a[k];
         return true;
     }
     // Outflow
     const DevBC& bc = I.bcs[Rg.bc];
-    r_times(Rc, v[0], u[0]);
     const double rho0 = u[0][0];
     const double un0 = u[0][1] / rho0, ut0 = u[0][2] / rho0;
     const double w2 = un0 * un0 + ut0 * ut0;
     const double ee1 = u[0][3] / rho0 - w2 / 6.0, ei1 = u[0][4] / rho0 - w2 / 6.0, er1 = u[0][5] / rho0 - w2 / 6.0;
-    const double ge = P.gamma_e - 1.0, gi = P.gamma_i - 1.0, gr = P.gamma_r - 1.0;
     const double p0 = rho0 * (ge * ee1 + gi * ei1 + gr * er1);
     const double a2 = P.gamma_e * ge * ee1 + P.gamma_i * gi * ei1 + P.gamma_r * gr * er1;
     const double a = sqrt(a2);
     const double lambda1 = un0 - a;
-    double rhs1[6];
-    for (int k = 0; k < 6; ++k) rhs1[k] = v[1][k];
+    double r0 = v[1][0];
     if (lambda1 < 0.0) {
         const double m_local = fabs(un0 / a);
         const double l1 = bc.sigma * (1.0 - sqd(m_local)) * a / bc.l_domain * (p0 - bc.p_inf);
-        rhs1[0] = l1 / lambda1;
+        r0 = l1 / lambda1;
     }
-    r_times(Rc, rhs1, u[1]);
-    for (int k = 2; k <= 4; ++k) r_times(Rc, v[k], u[k]);
+    if (l < 6) {
+        const double* Rc = LR + GH_LR_R;
+        double acc = 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) acc += Rc[6 * j + l] * (j == 0 ? r0 : v[1][j]);
+        u[1][l] = acc;
+    }
     return true;
 }
 
-// ---------------------------------------------------------------- preparation
-__device__ void cheap_ghost(const Inst& I, const GhostRec& Rg, int c, int stage) {
+// ---------------------------------------------------------------- cheap ghosts
+__device__ __forceinline__ void cheap_ghost(const Inst& I, const GhostRec& Rg, int c, int stage) {
     double* buf = const_cast<double*>(stage_src(I, stage));
     const long long plane = I.plane;
     const DevBC& bc = I.bcs[Rg.bc];
@@ -207,346 +224,470 @@ __device__ void cheap_ghost(const Inst& I, const GhostRec& Rg, int c, int stage)
 }
 
 // ---------------------------------------------------------------- heavy ghosts
-// L, R and lambda at the nearest fluid node of heavy ghost Rg in its
-// (normal, tangential) frame (bc1.rs:294-312): LR[6c + k] = L[c][k],
-// LR[36 + 6c + i] = R[i][c], LR[72 + c] = lambda_c
-__device__ __forceinline__ void local_lr(const Inst& I, const GhostRec& Rg, const double* __restrict__ buf,
-                                         double* LR, int stride) {
+// L, R and lambda of a Roe state: LR[6c + k] = L[c][k], LR[36 + 6c + i] =
+// R[i][c], LR[72 + c] = lambda_c, value e at LR[e * CHUNK]
+__device__ __forceinline__ void store_lr(double* LR, int row, const double Lr[6], const double Rr[6], const Roe& q) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        LR[(6 * row + k) * CHUNK] = Lr[k];
+        LR[(GH_LR_R + 6 * k + row) * CHUNK] = Rr[k];
+    }
+    LR[(GH_LR_LAM + row) * CHUNK] = row == 0 ? q.u - q.cs : (row == 5 ? q.u + q.cs : q.u);
+}
+// states outside the branch-free quotients' range (divrn.cuh)
+static __device__ __noinline__ void lr_each(const Roe* q, const DevParams& P, double* LR) {
+#pragma unroll 1
+    for (int row = 0; row < 6; ++row) {
+        double Lr[6], Rr[6];
+        l_row<0>(row, *q, P, Lr);
+        r_row<0, false>(row, *q, RecipN{1.0, 1.0, 0.0}, P, Rr);
+        store_lr(LR, row, Lr, Rr, *q);
+    }
+}
+
+// A double whose quotients take the branch-free form: the FMA build forms the
+// rows by the templates of physics.cuh over it, which contract as over double
+struct NearD {
+    double v;
+    __device__ __forceinline__ NearD() {}
+    __device__ __forceinline__ NearD(double x) : v(x) {}
+};
+__device__ __forceinline__ NearD operator-(NearD a) { return -a.v; }
+__device__ __forceinline__ NearD operator+(NearD a, NearD b) { return a.v + b.v; }
+__device__ __forceinline__ NearD operator-(NearD a, NearD b) { return a.v - b.v; }
+__device__ __forceinline__ NearD operator*(NearD a, NearD b) { return a.v * b.v; }
+__device__ __forceinline__ NearD operator/(NearD a, NearD b) { return div_near(a.v, recip_near(b.v)); }
+__device__ __forceinline__ NearD quot3(NearD x) { return div3_near(x.v); }
+__device__ __forceinline__ NearD quot6(NearD x) { return div6_near(x.v); }
+// L, R and lambda at the nearest fluid node of heavy ghost Rg in its (normal,
+// tangential) frame (bc1.rs:294-312)
+__device__ __forceinline__ void local_lr(const Inst& I, const GhostRec& Rg, int stage, double* LR) {
     const DevParams& P = I.P;
     double s[6];
-    load6(buf, I.plane, Rg.src, s);
+    load6(stage_src(I, stage), I.plane, Rg.src, s);
     const double mom_n = s[1] * Rg.nx + s[2] * Rg.ny;
     const double mom_t = -s[1] * Rg.ny + s[2] * Rg.nx;
     const double q6[6] = {s[0], mom_n, mom_t, s[3], s[4], s[5]};
     const Prim d1 = prim_from_state(q6, P);
-    const Roe q = roe_average(q6[0], d1, q6[0], d1, P);
-    for (int row = 0; row < 6; ++row) {
-        double Lr[6], Rc[6], lam;
-        l_row<0>(row, q, P, Lr);
-        r_col<0>(row, q, P, Rc, lam);
+    const double rt = sqrt(q6[0]);
+    const Roe q = roe_average_sqrt(rt, d1, rt, d1, P);
+    const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
+    const double gt = gi + ge + gr;
+    RoeDivN rd;
+    if (near_face(q, gt, rd) & near_params(P) & near_divisor(gt)) {
+        if (!kExactG) {
+            const RoeT<NearD> n = {q.u, q.v, q.w2, q.ee, q.ei, q.er, q.cs2, q.cs, q.he, q.hi, q.hr, q.b, q.den};
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            LR[(6 * row + k) * stride] = Lr[k];
-            LR[(GH_LR_R + 6 * row + k) * stride] = Rc[k];
+            for (int row = 0; row < 6; ++row) {
+                NearD Lr[6], Rc[6], lam;
+                l_row<0>(row, n, P, Lr);
+                r_col<0>(row, n, P, Rc, lam);
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    LR[(6 * row + k) * CHUNK] = Lr[k].v;
+                    LR[(GH_LR_R + 6 * row + k) * CHUNK] = Rc[k].v;
+                }
+                LR[(GH_LR_LAM + row) * CHUNK] = lam.v;
+            }
+            return;
         }
-        LR[(GH_LR_LAM + row) * stride] = lam;
-    }
-}
-
-// blocks [0, nbp): L, R, lambda of one heavy ghost per thread, staged in
-// shared memory ([value][thread], stride GH_PREP_THREADS + 1) and stored by
-// whole warps into the records; blocks [nbp, ...): cheap ghosts
-constexpr int GH_PREP_SMEM = GH_LR * (GH_PREP_THREADS + 1) * (int)sizeof(double);
-__global__ void __launch_bounds__(GH_PREP_THREADS) k_ghost_prep(const Inst* __restrict__ insts,
-                                                               const GhostRec* __restrict__ heavy, int nh,
-                                                               const GhostRec* __restrict__ cheap, int nc,
-                                                               double* __restrict__ hrec, int stage, int nbp) {
-    extern __shared__ __align__(16) double prep_smem[];
-    if ((int)blockIdx.x < nbp) {
-        constexpr int ST = GH_PREP_THREADS + 1;
-        const int g0 = blockIdx.x * GH_PREP_THREADS, g = g0 + threadIdx.x;
-        if (g < nh) {
-            const GhostRec Rg = heavy[g];
-            const Inst& I = insts[Rg.inst];
-            if (!has_error(I)) local_lr(I, Rg, stage_src(I, stage), prep_smem + threadIdx.x, ST);
-        }
-        __syncthreads();
-        // warp w stores the 80 values of ghosts g0 + 32 w .. g0 + 32 w + 31
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        for (int j = 0; j < 32; ++j) {
-            const int t = 32 * w + j, gj = g0 + t;
-            if (gj >= nh) break;
-            double* r = hrec + (size_t)__ldg(&heavy[gj].heavy) * GH_REC + GH_L;
-            for (int e = lane; e < GH_LR; e += 32) r[e] = prep_smem[e * ST + t];
+        rd.scale();
+        const RecipN rgt = recip_near(gt);
+#pragma unroll
+        for (int row = 0; row < 6; ++row) {
+            double Lr[6], Rr[6];
+            const double gl = row == 1 ? ge : (row == 2 ? gi : gr); // of an energy row of L (1-3)
+            const double gk = row == 3 ? ge : (row == 4 ? gi : gr); // of an energy row of R (3-5)
+            l_row<0>(row, q, rd, row >= 1 && row <= 3 ? div_near(gl, rgt) : 0.0, P, Lr);
+            r_row<0, true>(row, q, row >= 3 ? recip_near(6.0 * gk) : rgt, P, Rr);
+            store_lr(LR, row, Lr, Rr, q);
         }
     } else {
-        const int t = (blockIdx.x - nbp) * GH_PREP_THREADS + threadIdx.x;
-        const int g = t / 6, c = t - 6 * (t / 6);
-        if (g >= nc) return;
-        const GhostRec Rg = cheap[g];
-        const Inst& I = insts[Rg.inst];
-        if (has_error(I)) return;
-        cheap_ghost(I, Rg, c, stage);
+        const Roe t = q;
+        lr_each(&t, P, LR);
     }
 }
 
-// characteristic data of stencil node a from its state (bc1.rs:209-219)
-__device__ __forceinline__ void project_node(GhostWarp& G, const double* __restrict__ L, const double s[6],
-                                             double nx, double ny, int a) {
-    const double mn = s[1] * nx + s[2] * ny;
-    const double mt = -s[1] * ny + s[2] * nx;
-    const double u6[6] = {s[0], mn, mt, s[3], s[4], s[5]};
+// x + y . (d of one stencil node): one term of four rows for all six fields
+__device__ __forceinline__ void four_rows(double acc[4][6], const double2 x01, const double2 x23, const double* D) {
     double d[6];
+    load_d6(D, d);
+    const double x[4] = {x01.x, x01.y, x23.x, x23.y};
 #pragma unroll
-    for (int c = 0; c < 6; ++c)
-        d[c] = L[6 * c + 0] * u6[0] + L[6 * c + 1] * u6[1] + L[6 * c + 2] * u6[2] + L[6 * c + 3] * u6[3] +
-               L[6 * c + 4] * u6[4] + L[6 * c + 5] * u6[5];
-    store_d6(G.D[d_row(a)], d);
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) acc[i][c] += x[i] * d[c];
 }
 
-// source of a step-3 row: S_r transposed in the record (stride m, so the
-// lanes of one order read consecutive words), or w_{r,k} (stride 1)
-__device__ __forceinline__ const double* row_src(const double* __restrict__ rec, unsigned code, int m, int& stride) {
-    const bool wr = (code >> 8) != 0;
-    const int r = (int)((code >> 5) & 7u), ix = (int)(code & 31u);
-    stride = wr ? 1 : m;
-    return wr ? rec + GH_W + kWOff[r] + ix * m : rec + GH_S + kSOff[r] + ix;
+// a / b: IEEE quotients of positive operands, branch-free where they are in range
+__device__ __forceinline__ double quot_pos(double a, double b) {
+    if (a > 0.0 && num_near(a) && den_near(b)) return div_once(a, b);
+    return div_ieee(a, b);
 }
 
-// an S row stores d_c,a (S_r d_c)_a, the term of beta_{c,r}; a w row stores
-// V^(k)_{c,r} = w_{r,k} . d_c
-__device__ __forceinline__ void row_out(GhostWarp& G, unsigned code, const double acc[6]) {
-    const int r = (int)((code >> 5) & 7u), ix = (int)(code & 31u);
-    if ((code >> 8) != 0) {
-#pragma unroll
-        for (int c = 0; c < 6; ++c) G.V[c][r * (r + 1) / 2 + ix] = acc[c];
+// alpha = d_r / x^q, x = eps + beta (bc1.rs:241)
+__device__ __forceinline__ double alpha_of(double dr, double x, double weno_q) {
+    double xq;
+    if (!kExactG && weno_q == 10.0) { // four products (within a few ulp) in the FMA build
+        const double x2 = x * x, x4 = x2 * x2, x8 = x4 * x4;
+        xq = x8 * x2;
     } else {
-        double d[6], p[6];
-        load_d6(G.D[kDOff[r] + ix], d);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) p[c] = d[c] * acc[c];
-        store_d6(G.ACC[kStOff[r] + ix], p);
+        xq = pow_q(x, weno_q); // correctly rounded, as the reference's powf
     }
+    return quot_pos(dr, xq);
 }
 
-// two rows of one order for all six fields c, each summed over b in order
-// (bc1.rs:224-236)
-__device__ __forceinline__ void dot_pair(GhostWarp& G, const double* __restrict__ rec, unsigned codes) {
-    if (codes == kPairNone) return;
-    const unsigned c1 = codes & 0xffffu, c2 = codes >> 16;
-    const int r = (int)((c1 >> 5) & 7u);
-    const int m = (r + 1) * (r + 1);
-    const double(*__restrict__ D)[6] = G.D + kDOff[r];
-    int st1, st2;
-    const double* __restrict__ p1 = row_src(rec, c1, m, st1);
-    const double* __restrict__ p2 = row_src(rec, c2, m, st2);
-    double a1[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, a2[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-#pragma unroll 4
-    for (int b = 0; b < m; ++b) {
-        const double x1 = p1[b * st1], x2 = p2[b * st2];
-        double d[6];
-        load_d6(D[b], d);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            a1[c] += x1 * d[c];
-            a2[c] += x2 * d[c];
-        }
-    }
-    row_out(G, c1, a1);
-    row_out(G, c2, a2);
-}
+// the 30 (c, r) tasks of steps 4 and 5 on 16 lanes in two rounds, the long
+// sums (orders 4 and 3) in the first: a hex digit per lane; lanes 14 and 15
+// have one task
+constexpr unsigned long long kTaskC[2] = {0x3210543210543210ull, 0x0054321054321054ull};
+constexpr unsigned long long kTaskR[2] = {0x2222333333444444ull, 0x0000000011111122ull};
+__device__ __forceinline__ int task_digit(unsigned long long k, int l) { return (int)(k >> (4 * l)) & 15; }
 
-// Fetches for the warp's next ghost (record slot n_heavy, -1 for none, and
-// instance n_inst, loaded before this ghost's wait) are spread over the steps
-// so that no load waits on the one before it: its stencil indices and state
-// buffer after step 3, its stencil states (n0, n1) and its instance's error
-// flag (n_skip) after step 4, its record once step 3 has read this one.
-__device__ __forceinline__ void heavy_ghost(const Inst* __restrict__ insts, const Inst& I, const GhostRec& Rg,
-                                            GhostWarp& G, const double* __restrict__ rec,
-                                            const double* __restrict__ hrec, int lane, int stage,
-                                            unsigned slot_a, unsigned slot_b, double dr, const double s0[6],
-                                            const double s1[6], int n_heavy, int n_inst, double n0[6],
-                                            double n1[6], bool& n_skip) {
-    const DevParams& P = I.P;
-    double* buf = const_cast<double*>(stage_src(I, stage));
-    const long long plane = I.plane;
-    const double nx = Rg.nx, ny = Rg.ny;
-    const double* L = G.LR;
-    const double* Rc = G.LR + GH_LR_R;
-    const double* lam = G.LR + GH_LR_LAM;
-    // 2. characteristic data of the 55 stencil nodes
-    project_node(G, L, s0, nx, ny, lane);
-    if (lane + 32 < 55) project_node(G, L, s1, nx, ny, lane + 32);
-    __syncwarp();
-    // 3. the 70 rows: d_c,a (S_r d_c)_a and V^(k)_{c,r}
-    dot_pair(G, rec, slot_a);
-    dot_pair(G, rec, slot_b);
-    // the next ghost's stencil indices, state buffer and error flag address
-    int st0 = 0, st1 = 0;
-    const double* nbuf = nullptr;
-    long long nplane = 0;
-    const DevError* nerr = nullptr;
-    if (n_heavy >= 0) {
-        const int32_t* st = reinterpret_cast<const int32_t*>(hrec + (size_t)n_heavy * GH_REC + GH_ST);
-        st0 = __ldg(&st[lane]);
-        if (lane + 32 < 55) st1 = __ldg(&st[lane + 32]);
-        nbuf = stage_src(insts[n_inst], stage);
-        nplane = insts[n_inst].plane;
-        nerr = insts[n_inst].err;
-    }
-    __syncwarp();
-    // the record is not read below: bring in the next ghost's
-    if (lane == 0 && n_heavy >= 0) bulk_load(G.rec[0], hrec + (size_t)n_heavy * GH_REC, GH_REC * 8, &G.bar[0]);
-    // 4. lanes (c, r): beta_{c,r} = sum_a d_a (S d)_a in order, alpha = d_r / (eps + beta)^q
-    if (lane < 30) {
-        const int c = lane / 5, r = lane - 5 * (lane / 5);
-        const int m = (r + 1) * (r + 1), off = kStOff[r];
-        double beta = 0.0;
-#pragma unroll 5
-        for (int a = 0; a < m; ++a) beta += G.ACC[off + a][c];
-        const double x = P.eps + beta;
-        double xq;
-        if (!kExactG && P.weno_q == 10.0) { // four products (within a few ulp) in the FMA build
-            const double x2 = x * x, x4 = x2 * x2, x8 = x4 * x4;
-            xq = x8 * x2;
-        } else {
-            xq = pow_q(x, P.weno_q); // correctly rounded, as the reference's powf
-        }
-        G.alpha[c][r] = dr / xq;
-    }
-    // the next ghost's stencil states (used in its step 2) and error flag
-    if (n_heavy >= 0) {
-        load6(nbuf, nplane, st0, n0);
-        if (lane + 32 < 55) load6(nbuf, nplane, st1, n1);
-        n_skip = nerr->key != ~0ull;
-    }
-    __syncwarp();
-    // 5. nonlinear weights (bc1.rs:247-252); V^(k)_r = 0 for k > r
-    if (lane < 30) {
-        const int k = lane / 6, c = lane - 6 * (lane / 6);
-        double asum = 0.0;
-        for (int r = 0; r < 5; ++r) asum += G.alpha[c][r];
-        const Recip ra = recip(asum); // five quotients by one divisor (IEEE results, divrn.cuh)
-        double res = 0.0;
-        for (int r = 0; r < 5; ++r)
-            res += div_rn(G.alpha[c][r], ra) * (k <= r ? G.V[c][r * (r + 1) / 2 + k] : 0.0);
-        G.v[k][c] = res;
-    }
-    __syncwarp();
-    // 6. BC rows, R products, Taylor expansion (bc1.rs:690-924)
-    double (*u)[6] = reinterpret_cast<double (*)[6]>(&G.ACC[0][0]); // ACC is dead here
-    double* vinf = &G.ACC[5][0];
-    bool ok = true;
-    if (Rg.kind == BC_FAR_FIELD) {
-        const DevBC& bc = I.bcs[Rg.bc];
-        if (lane < 6) {
-            const double* ui = bc.state;
-            const double uinf[6] = {ui[0], ui[1] * nx + ui[2] * ny, -ui[1] * ny + ui[2] * nx, ui[3], ui[4], ui[5]};
-            double acc = 0.0;
-            for (int j = 0; j < 6; ++j) acc += L[6 * lane + j] * uinf[j];
-            vinf[lane] = acc;
-        }
-        __syncwarp();
-        if (lane < 30) {
-            const int k = lane / 6, i = lane - 6 * (lane / 6);
-            double acc = 0.0;
-            for (int m2 = 0; m2 < 6; ++m2) {
-                const double x = lam[m2] < 0.0 ? (k == 0 ? vinf[m2] : 0.0) : G.v[k][m2];
-                acc += Rc[6 * m2 + i] * x;
-            }
-            u[k][i] = acc;
-        }
-    } else if (lane == 0) {
-        ok = serial_tail(I, Rg, G.LR, G.v, u);
-    }
-    __syncwarp();
-    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-    if (!ok) {
-        if (lane == 0) report(I, 1 + 2 * stage, 3, (unsigned)Rg.gid);
-        return;
-    }
-    double g = 0.0;
-    if (lane < 6) {
-        g = u[0][lane];
-        double coef = 1.0;
-        for (int k = 1; k <= 4; ++k) {
-            coef *= Rg.dist / (double)k;
-            g = g + coef * u[k][lane];
-        }
-    }
-    const double mn = __shfl_sync(0xffffffffu, g, 1), mt = __shfl_sync(0xffffffffu, g, 2);
-    if (lane < 6) {
-        const double out = lane == 1 ? mn * nx - mt * ny : (lane == 2 ? mn * ny + mt * nx : g);
-        buf[lane * plane + Rg.node] = out;
-        if (!isfinite(out)) report(I, 1 + 2 * stage, 2, (unsigned)Rg.gid);
-    }
-}
-
-// stencil states of ghost g (lane a and a + 32), from the record in global memory
-__device__ __forceinline__ void gather_stencil(const Inst& I, const double* __restrict__ grec, int lane, int stage,
-                                               double s0[6], double s1[6]) {
-    const int32_t* st = reinterpret_cast<const int32_t*>(grec + GH_ST);
-    const double* buf = stage_src(I, stage);
-    load6(buf, I.plane, st[lane], s0);
-    if (lane + 32 < 55) load6(buf, I.plane, st[lane + 32], s1);
-}
-
-// warps take the heavy ghosts in turn (record of the next one in flight; the
-// next ghost's GhostRec is loaded at the start of a ghost and kept in shared
-// memory, so a ghost starts without a dependent global load: 4.5% faster)
-__global__ void __launch_bounds__(GH_WARPS * 32, GH_BLOCKS_PER_SM) k_ghosts(const Inst* __restrict__ insts,
-                                                         const GhostRec* __restrict__ heavy, int nh,
-                                                         const double* __restrict__ hrec, int stage) {
+// Warps take the heavy ghosts in turn, two at a time (half-warps 0 and 1; an
+// odd last ghost runs on both halves and is written by the first). What the
+// next pair needs is fetched in four places, so that no load waits on the one
+// before it: its GhostRecs (slot, instance) at the top, its stencil
+// indices after step 3, its stencil states, L, R, lambda and error flags after
+// step 4, its tables once step 3 has read this pair's.
+//
+// Bound by latency and by the L1 / shared-memory data pipe (55% busy; FP64 pipe
+// 40%). Four rows a lane halve the loads of the data against two rows a lane and
+// one ghost a warp, two ghosts a warp give every serial step (4-6) two chains
+// to interleave, and nothing on a pair's path waits for a global load. 24 batch
+// instances (84,000 ghosts), a stage: 348 us against 425 us for a preparation
+// kernel and one ghost a warp on 12 warps a SM (FMA build 293 us against 426);
+// 1024 x 8 planar shock, where one pass is all latency: 18 us against 34 us.
+// Tables read from L2 by the lanes instead of bulk copies: 1.32 ms a step of the
+// 24 instances against 1.23 ms at that point, with 12 warps (168 registers,
+// spills) 1.73 ms; stencil indices fetched before step 3: 1.15 against 1.06 ms.
+__global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restrict__ insts,
+                                                             const GhostRec* __restrict__ heavy, int nh,
+                                                             const GhostRec* __restrict__ cheap, int nc,
+                                                             const double* __restrict__ hrec, double* lrbuf, int stage) {
     extern __shared__ __align__(128) unsigned char gh_smem[];
-    const int lane = threadIdx.x & 31;
-    GhostWarp& G = reinterpret_cast<GhostWarp*>(gh_smem)[threadIdx.x >> 5];
-    const int stride = gridDim.x * GH_WARPS;
-    int g = blockIdx.x * GH_WARPS + (threadIdx.x >> 5);
-    if (g < nh) { // warp-uniform
-        const unsigned slot_a = kSlotA[lane], slot_b = kSlotB[lane];
-        if (lane == 0) {
-            mbar_init(&G.bar[0], 1);
-            mbar_fence_init();
-            bulk_load(G.rec[0], hrec + (size_t)heavy[g].heavy * GH_REC, GH_REC * 8, &G.bar[0]);
+    const int lane = threadIdx.x & 31, half = lane >> 4, l = lane & 15, warp = threadIdx.x >> 5;
+    GhostWarp& W = reinterpret_cast<GhostWarp*>(gh_smem)[warp];
+    GhostSlot& G = W.g[half];
+    const int npair = (nh + 1) >> 1, stride = gridDim.x * GH_WARPS;
+    // cheap ghosts, six threads each, on the warps that come last in the order of the pairs first
+    for (int t = ((GH_WARPS - 1 - warp) * gridDim.x + blockIdx.x) * 32 + lane; t < 6 * nc;
+         t += gridDim.x * GH_WARPS * 32) {
+        const int c = t % 6;
+        const GhostRec Rg = cheap[t / 6];
+        const Inst& I = insts[Rg.inst];
+        if (!has_error(I)) cheap_ghost(I, Rg, c, stage);
+    }
+    const int first = blockIdx.x + gridDim.x * warp; // pairs spread over the SMs first
+    if (first >= npair) return;                      // warp-uniform
+    // this lane's four rows of step 3
+    const int ord = l < 7 || l == 15 ? 4 : (l < 12 ? 3 : 2);
+    const int quad = l < 7 ? l : (l == 15 ? 7 : (l < 12 ? l - 7 : l - 12));
+    const int ord_m = (ord + 1) * (ord + 1);
+    // tasks (c, r) of steps 4 and 5
+    const int c0 = task_digit(kTaskC[0], l), r0 = task_digit(kTaskR[0], l);
+    const int c1 = task_digit(kTaskC[1], l), r1 = task_digit(kTaskR[1], l);
+    // task (row, three fields) of orders 1 (rows 0-3 of S, 4-5 w) and 0 (row 6 S, 7 w)
+    const int lrow = l >> 1, lc = 3 * (l & 1);
+    constexpr int kRecWords = (int)(sizeof(GhostRec) / 8);
+    static_assert(sizeof(GhostRec) % 8 == 0 && kRecWords <= 16, "GhostRec copied as words by half a warp");
+
+    if (lane == 0) {
+        mbar_init(&W.bar[0], 1);
+        mbar_fence_init();
+    }
+    // per pair, loaded while the pair before it runs
+    double s[4][6], lr[5], ui_l, eps, weno_q;
+    double* out_p; // component l (< 6) of the ghost node
+    bool skip, n_skip = false;
+    int it = 0;
+    for (int i0 = first; i0 < npair; i0 += CHUNK * stride) {
+    // ---- 1. L, R, lambda of the chunk's ghosts, one per lane, staged in the
+    // table buffer and stored by half-warps
+    {
+        const bool mine = l < CHUNK && i0 + l * stride < npair;
+        int slot = 0;
+        if (mine) {
+            const GhostRec Rg = heavy[min(2 * (i0 + l * stride) + half, nh - 1)];
+            slot = Rg.heavy;
+            local_lr(insts[Rg.inst], Rg, stage, G.rec + l);
         }
         __syncwarp();
-        // stencil states of the warp's first ghost; later ones are gathered
-        // while the ghost before them is processed
-        constexpr int kRecWords = (int)(sizeof(GhostRec) / 8);
-        static_assert(sizeof(GhostRec) % 8 == 0 && kRecWords <= 32, "GhostRec copied as words by one warp");
-        double s0[6], s1[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        bool skip;
-        {
-            const GhostRec& R0 = heavy[g];
-            gather_stencil(insts[R0.inst], hrec + (size_t)R0.heavy * GH_REC, lane, stage, s0, s1);
-            skip = has_error(insts[R0.inst]);
-            if (lane < kRecWords)
-                reinterpret_cast<unsigned long long*>(&G.cur)[lane] =
-                    __ldg(reinterpret_cast<const unsigned long long*>(&heavy[g]) + lane);
-        }
-        for (int it = 0; g < nh; ++it, g += stride) {
-            const int gn = g + stride;
-            int n_heavy = -1, n_inst = 0;
-            unsigned long long nword = 0;
-            if (gn < nh) {
-                n_heavy = __ldg(&heavy[gn].heavy);
-                n_inst = __ldg(&heavy[gn].inst);
-                if (lane < kRecWords) nword = __ldg(reinterpret_cast<const unsigned long long*>(&heavy[gn]) + lane);
-            }
-            __syncwarp();
-            const GhostRec Rg = G.cur; // loaded while the ghost before ran (no dependent global load here)
-            const Inst& I = insts[Rg.inst];
-            bool n_skip = false;
-            double n0[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, n1[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-            const bool ok = __all_sync(0xffffffffu, mbar_wait(&G.bar[0], (uint32_t)(it & 1)));
-            if (!ok) {
-                if (lane == 0) report(I, 1 + 2 * stage, MBAR_TIMEOUT_CODE, (unsigned)Rg.gid);
-                return;
-            }
-            for (int e = lane; e < GH_LR; e += 32) G.LR[e] = G.rec[0][GH_L + e];
-            // d_r of lane (c, r), read here with L/R: every read of the record
-            // is then long complete when the next ghost's copy overwrites it
-            const double dr = lane < 30 ? G.rec[0][GH_D + lane - 5 * (lane / 5)] : 0.0;
-            __syncwarp();
-            if (!skip) {
-                heavy_ghost(insts, I, Rg, G, G.rec[0], hrec, lane, stage, slot_a, slot_b, dr, s0, s1, n_heavy,
-                            n_inst, n0, n1, n_skip);
-            } else if (n_heavy >= 0) {
-                if (lane == 0) bulk_load(G.rec[0], hrec + (size_t)n_heavy * GH_REC, GH_REC * 8, &G.bar[0]);
-                gather_stencil(insts[n_inst], hrec + (size_t)n_heavy * GH_REC, lane, stage, n0, n1);
-                n_skip = has_error(insts[n_inst]);
-            }
-            __syncwarp();
-            if (lane < kRecWords) reinterpret_cast<unsigned long long*>(&G.cur)[lane] = nword;
-            skip = n_skip;
+        for (int t = 0; t < CHUNK && i0 + t * stride < npair; ++t) {
+            double* o = lrbuf + (size_t)__shfl_sync(0xffffffffu, slot, (lane & 16) + t) * GH_LR;
 #pragma unroll
-            for (int q = 0; q < 6; ++q) { s0[q] = n0[q]; s1[q] = n1[q]; }
+            for (int j = 0; j < 5; ++j)
+                if (l + 16 * j < 78) o[l + 16 * j] = G.rec[(l + 16 * j) * CHUNK + t];
         }
+        __syncwarp();
+    }
+    // the chunk's first pair
+    {
+        const GhostRec& R0 = heavy[min(2 * i0 + half, nh - 1)];
+        const int slot = __ldg(&R0.heavy);
+        const int slot1 = __shfl_sync(0xffffffffu, slot, 16);
+        if (lane == 0) load_tables(W, hrec, slot, slot1);
+        const Inst& I = insts[__ldg(&R0.inst)];
+        const int32_t* st = reinterpret_cast<const int32_t*>(hrec + (size_t)slot * GH_REC + GH_ST);
+        const double* buf = stage_src(I, stage);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (l + 16 * j < 55) load6(buf, I.plane, __ldg(&st[l + 16 * j]), s[j]);
+#pragma unroll
+        for (int j = 0; j < 5; ++j) lr[j] = __ldcg(lrbuf + (size_t)slot * GH_LR + l + 16 * j);
+        ui_l = l < 6 ? I.bcs[__ldg(&R0.bc)].state[l] : 0.0;
+        eps = I.P.eps;
+        weno_q = I.P.weno_q;
+        out_p = const_cast<double*>(buf) + (l < 6 ? l : 0) * I.plane + __ldg(&R0.node);
+        skip = has_error(I);
+        if (l < kRecWords)
+            reinterpret_cast<unsigned long long*>(&G.cur)[l] =
+                __ldg(reinterpret_cast<const unsigned long long*>(&R0) + l);
+        __syncwarp();
+    }
+    for (int t = 0, i = i0; t < CHUNK && i < npair; ++t, ++it, i += stride) {
+        const bool more = t + 1 < CHUNK && i + stride < npair; // warp-uniform
+        int n_heavy = 0, n_inst = 0, n_bc = 0, n_node = 0;
+        unsigned long long nword = 0;
+        if (more) {
+            const GhostRec* R = heavy + min(2 * (i + stride) + half, nh - 1);
+            n_heavy = __ldg(&R->heavy);
+            n_inst = __ldg(&R->inst);
+            n_bc = __ldg(&R->bc);
+            n_node = __ldg(&R->node);
+            if (l < kRecWords) nword = __ldg(reinterpret_cast<const unsigned long long*>(R) + l);
+        }
+#pragma unroll
+        for (int j = 0; j < 5; ++j) G.LR[l + 16 * j] = lr[j];
+        if (l < 6) G.ui[l] = ui_l;
+        const double nx = G.cur.nx, ny = G.cur.ny;
+        const int kind = G.cur.kind;
+        const Inst& I = insts[G.cur.inst];
+        const bool write = !skip && 2 * i + half < nh;
+        const double* L = G.LR;
+        const double* Rc = G.LR + GH_LR_R;
+        const double* lam = G.LR + GH_LR_LAM;
+        __syncwarp();
+        // ---- 2. characteristic data of the 55 stencil nodes
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const double mn = s[j][1] * nx + s[j][2] * ny, mt = -s[j][1] * ny + s[j][2] * nx;
+            s[j][1] = mn;
+            s[j][2] = mt;
+        }
+#pragma unroll
+        for (int c = 0; c < 6; c += 2) {
+            const double2* q = reinterpret_cast<const double2*>(L + 6 * c);
+            const double2 a0 = q[0], a1 = q[1], a2 = q[2], b0 = q[3], b1 = q[4], b2 = q[5];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double* u = s[j];
+                const double d0 = a0.x * u[0] + a0.y * u[1] + a1.x * u[2] + a1.y * u[3] + a2.x * u[4] + a2.y * u[5];
+                const double d1 = b0.x * u[0] + b0.y * u[1] + b1.x * u[2] + b1.y * u[3] + b2.x * u[4] + b2.y * u[5];
+                if (l + 16 * j < 55) *reinterpret_cast<double2*>(&G.D[d_row(l + 16 * j)][c]) = make_double2(d0, d1);
+            }
+        }
+        if (l < 6) { // the FarField state in characteristic variables (bc1.rs:839-846)
+            const double uinf[6] = {G.ui[0], G.ui[1] * nx + G.ui[2] * ny, -G.ui[1] * ny + G.ui[2] * nx,
+                                    G.ui[3], G.ui[4], G.ui[5]};
+            double a = 0.0;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) a += L[6 * l + j] * uinf[j];
+            G.vinf[l] = a;
+        }
+        const bool ok_copy = __all_sync(0xffffffffu, mbar_wait(&W.bar[0], (uint32_t)(it & 1)));
+        if (!ok_copy) {
+            if (l == 0 && write) report(I, 1 + 2 * stage, MBAR_TIMEOUT_CODE, (unsigned)G.cur.gid);
+            return;
+        }
+        __syncwarp();
+        // ---- 3. the 70 rows: orders 4, 3 and 2
+        double acc[4][6];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) acc[q][c] = 0.0;
+        {
+            const double2* rows = reinterpret_cast<const double2*>(G.rec);
+            const double* D = &G.D[kDOff[ord]][0];
+            // (lane 15 has one pair: its second chunk is a neighbour's and goes unused)
+#pragma unroll 3
+            for (int b = 0; b < 9; ++b) four_rows(acc, rows[31 * b + l], rows[31 * b + 16 + l], D + 6 * b);
+            if (ord >= 3) {
+                const double2* p = rows + GR_SEG1 + (l == 15 ? 12 : l);
+                const double2* p2 = rows + GR_SEG1 + 13 + l;
+#pragma unroll
+                for (int b = 0; b < 7; ++b) four_rows(acc, p[25 * b], p2[25 * b], D + 54 + 6 * b);
+            }
+            if (ord == 4) {
+                const double2* p = rows + GR_SEG2 + (l == 15 ? 7 : l);
+                const double2* p2 = rows + GR_SEG2 + 8 + l;
+#pragma unroll 3
+                for (int b = 0; b < 9; ++b) four_rows(acc, p[15 * b], p2[15 * b], D + 96 + 6 * b);
+            }
+        }
+        double low[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const double* d = &G.D[lrow < 6 ? 1 + b : 0][lc];
+            if (lrow < 6 || b == 0)
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    low[c] += G.rec[lrow < 6 ? row_place(1, lrow, b) : 2 * GR_ORDER0 + lrow - 6] * d[c];
+        }
+        const double dr0 = G.rec[GH_D + r0], dr1 = G.rec[GH_D + r1];
+        // the next pair's stencil indices, state buffer, error flag and BC table
+        int st[4] = {0, 0, 0, 0};
+        if (more) {
+            const int32_t* q = reinterpret_cast<const int32_t*>(hrec + (size_t)n_heavy * GH_REC + GH_ST);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (l + 16 * j < 55) st[j] = __ldg(&q[l + 16 * j]);
+        }
+        const Inst& In = insts[n_inst];
+        const double* nbuf = stage_src(In, stage);
+        const long long nplane = In.plane;
+        const DevError* nerr = In.err;
+        const DevBC* nbcs = In.bcs;
+        const double n_eps = In.P.eps, n_weno_q = In.P.weno_q;
+        const int n_heavy1 = __shfl_sync(0xffffffffu, n_heavy, 16);
+        __syncwarp();
+        // the tables are not read below: bring in the next pair's
+        if (lane == 0 && more) load_tables(W, hrec, n_heavy, n_heavy1);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int R = quad_row(ord, quad, q);
+            if (R < ord_m) {
+                double* Dr = &G.D[kDOff[ord] + R][0];
+                double d[6], p[6];
+                load_d6(Dr, d);
+#pragma unroll
+                for (int c = 0; c < 6; ++c) p[c] = d[c] * acc[q][c];
+                store_d6(Dr, p);
+            } else if (R - ord_m <= ord) {
+#pragma unroll
+                for (int c = 0; c < 6; ++c) G.V[c][ord * (ord + 1) / 2 + R - ord_m] = acc[q][c];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int row = lrow == 6 ? 0 : 1 + lrow;
+            if (lrow < 4 || lrow == 6) G.D[row][lc + c] = G.D[row][lc + c] * low[c];
+            else G.V[lc + c][lrow == 7 ? 0 : lrow - 3] = low[c];
+        }
+        __syncwarp();
+        // ---- 4. beta_{c,r} = sum_a d_a (S d)_a in order, alpha = d_r / (eps + beta)^q
+        {
+            double b0 = 0.0, b1 = 0.0;
+            const int m0 = (r0 + 1) * (r0 + 1), m1 = (r1 + 1) * (r1 + 1);
+            const double *q0 = &G.D[kDOff[r0]][c0], *q1 = &G.D[kDOff[r1]][c1];
+#pragma unroll
+            for (int a = 0; a < 9; ++a) {
+                b0 += q0[6 * a];
+                if (a < m1) b1 += q1[6 * a];
+            }
+#pragma unroll 8
+            for (int a = 9; a < m0; ++a) b0 += q0[6 * a];
+            const double al0 = alpha_of(dr0, eps + b0, weno_q), al1 = alpha_of(dr1, eps + b1, weno_q);
+            G.alpha[c0][r0] = al0;
+            if (l < 14) G.alpha[c1][r1] = al1;
+        }
+        // the next pair's stencil states, L, R, lambda (used in its step 2), FarField states and error flags
+        if (more) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (l + 16 * j < 55) load6(nbuf, nplane, st[j], s[j]);
+#pragma unroll
+            for (int j = 0; j < 5; ++j) lr[j] = __ldcg(lrbuf + (size_t)n_heavy * GH_LR + l + 16 * j);
+            if (l < 6) ui_l = nbcs[n_bc].state[l];
+            n_skip = nerr->key != ~0ull;
+        }
+        __syncwarp();
+        // ---- 5. nonlinear weights (bc1.rs:247-252); V^(k)_r = 0 for k > r
+        {
+            auto weight = [&](int c, int r) {
+                double asum = 0.0;
+#pragma unroll
+                for (int q = 0; q < 5; ++q) asum += G.alpha[c][q];
+                return quot_pos(G.alpha[c][r], asum);
+            };
+            const double w0 = weight(c0, r0), w1 = weight(c1, r1);
+            __syncwarp();
+            G.alpha[c0][r0] = w0;
+            if (l < 14) G.alpha[c1][r1] = w1;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int t = l + 16 * j, k = t / 6, c = t - 6 * (t / 6);
+            if (t < 30) {
+                double res = 0.0;
+#pragma unroll
+                for (int r = 0; r < 5; ++r) res += G.alpha[c][r] * (k <= r ? G.V[c][r * (r + 1) / 2 + k] : 0.0);
+                G.v[k][c] = res;
+            }
+        }
+        __syncwarp();
+        // ---- 6. BC rows, R products, Taylor expansion (bc1.rs:690-924)
+        double(*u)[6] = reinterpret_cast<double(*)[6]>(&G.D[0][0]); // D is dead here
+        const bool far = kind == BC_FAR_FIELD;
+        {
+            double a[2] = {0.0, 0.0};
+#pragma unroll
+            for (int m = 0; m < 6; ++m) {
+                const bool in = far && lam[m] < 0.0;
+                const double vi = G.vinf[m];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int t = l + 16 * j < 30 ? l + 16 * j : 29, k = t / 6, q = t - 6 * (t / 6);
+                    const double x = in ? (k == 0 ? vi : 0.0) : G.v[k][m];
+                    a[j] += Rc[6 * m + q] * x;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int t = l + 16 * j;
+                if (t < 30) u[t / 6][t - 6 * (t / 6)] = a[j];
+            }
+        }
+        __syncwarp();
+        bool ok = true;
+        if (!far) ok = wall_outflow_rows(I, G.cur, G.LR, G.v, u, l, 0xffffu << (16 * half), 16 * half);
+        __syncwarp();
+        double g = 0.0;
+        if (l < 6) {
+            g = u[0][l];
+            double coef = 1.0;
+            const double dist = G.cur.dist;
+#pragma unroll
+            for (int k = 1; k <= 4; ++k) {
+                coef *= k == 3 ? div3_rn(dist) : dist / (double)k;
+                g = g + coef * u[k][l];
+            }
+        }
+        const double mn = __shfl_sync(0xffffffffu, g, (lane & 16) + 1), mt = __shfl_sync(0xffffffffu, g, (lane & 16) + 2);
+        if (write) {
+            if (!ok) {
+                if (l == 0) report(I, 1 + 2 * stage, 3, (unsigned)G.cur.gid);
+            } else if (l < 6) {
+                const double out = l == 1 ? mn * nx - mt * ny : (l == 2 ? mn * ny + mt * nx : g);
+                *out_p = out;
+                if (!isfinite(out)) report(I, 1 + 2 * stage, 2, (unsigned)G.cur.gid);
+            }
+        }
+        __syncwarp();
+        if (l < kRecWords) reinterpret_cast<unsigned long long*>(&G.cur)[l] = nword;
+        skip = n_skip;
+        eps = n_eps;
+        weno_q = n_weno_q;
+        out_p = const_cast<double*>(nbuf) + (l < 6 ? l : 0) * nplane + n_node;
+        __syncwarp();
+    }
     }
 }
 
 void launch_ghosts(cudaStream_t s, const Inst* insts, const GhostRec* heavy, int nh, const GhostRec* cheap, int nc,
-                   double* hrec, int stage) {
+                   const double* hrec, double* lrbuf, int stage) {
     if (nh + nc <= 0) return;
     static int sm_count[64] = {0};
     int dev = 0;
@@ -556,19 +697,14 @@ void launch_ghosts(cudaStream_t s, const Inst* insts, const GhostRec* heavy, int
         int n = 0;
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         cudaFuncSetAttribute(k_ghosts, cudaFuncAttributeMaxDynamicSharedMemorySize, GH_SMEM);
-        cudaFuncSetAttribute(k_ghost_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, GH_PREP_SMEM);
         sm_count[dev] = n > 0 ? n : 1;
     }
-    const int nbp = (nh + GH_PREP_THREADS - 1) / GH_PREP_THREADS;
-    const int nbc = (nc * 6 + GH_PREP_THREADS - 1) / GH_PREP_THREADS;
-    k_ghost_prep<<<nbp + nbc, GH_PREP_THREADS, GH_PREP_SMEM, s>>>(insts, heavy, nh, cheap, nc, hrec, stage, nbp);
-    if (nh > 0) {
-        const int nbh = std::min((nh + GH_WARPS - 1) / GH_WARPS, GH_BLOCKS_PER_SM * sm_count[dev]);
-        k_ghosts<<<nbh, GH_WARPS * 32, GH_SMEM, s>>>(insts, heavy, nh, hrec, stage);
-    }
+    const int n = std::max((nh + 1) / 2, (6 * nc + GH_WARPS * 32 - 1) / (GH_WARPS * 32));
+    k_ghosts<<<std::min(n, sm_count[dev]), GH_WARPS * 32, GH_SMEM, s>>>(insts, heavy, nh, cheap, nc, hrec, lrbuf,
+                                                                         stage);
 }
 
-int ghost_launches(int nh, int nc) { return (nh + nc > 0 ? 1 : 0) + (nh > 0 ? 1 : 0); }
+int ghost_launches(int nh, int nc) { return nh + nc > 0 ? 1 : 0; }
 
 // one warp: the ghost update's bounded wait on a fresh mbarrier whose phase
 // completes (arrive: one arrival, no bytes expected) or never does; out[0] =

@@ -5,10 +5,10 @@
 
 namespace rh3t {
 // heavy: Wall / Outflow / FarField records; cheap: all other kinds (ghosts.cu)
-// hrec: heavy records (GH_REC doubles per GhostBC slot; the per-stage L, R,
-// lambda part is written by the launch). Two kernels: ghost_launches() of them.
+// hrec: heavy records (GH_REC doubles per GhostBC slot); lrbuf: scratch, GH_LR
+// doubles per slot. One kernel: ghost_launches().
 void launch_ghosts(cudaStream_t s, const Inst* insts, const GhostRec* heavy, int nh, const GhostRec* cheap, int nc,
-                   double* hrec, int stage);
+                   const double* hrec, double* lrbuf, int stage);
 int ghost_launches(int nh, int nc);
 // Shared memory of a flux launch: stencil points of its largest x and y tile
 // (flux_points of direction and shape), and whether an instance has diffusion on

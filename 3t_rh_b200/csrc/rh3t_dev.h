@@ -113,15 +113,13 @@ struct Tile {
 };
 
 // Heavy-ghost record (one per GhostBC slot, bc1.rs:50-57), repacked at set-up
-// so one 16-byte-aligned bulk copy brings a ghost's data to shared memory:
-// S (979 doubles, offsets of bc1.rs:45-47, each S_r stored transposed) |
-// w (225) | d (5) | pad (1) | E_r stencil as 55 padded node indices (int32,
-// + 1 pad) | per stage: L (6x6, row-major), R (6x6, by column), lambda (6),
-// pad (2), written by the ghost preparation kernel.
-constexpr int GH_S = 0, GH_W = 979, GH_D = 1204, GH_ST = 1210;
-constexpr int GH_L = 1238, GH_R = 1274, GH_LAM = 1310;
-constexpr int GH_LR = 80;                        // doubles of the per-stage part at GH_L
-constexpr int GH_REC = 1318;                     // doubles per record (10544 bytes)
+// so one 16-byte-aligned bulk copy of its first GH_COPY doubles brings a ghost's
+// tables to shared memory: the rows of S and w (1204 doubles in the order of
+// ghost_rows.cuh) | d (5) | pad (1) | E_r stencil as 55 padded node indices
+// (int32, + 1 pad).
+constexpr int GH_ROWS = 0, GH_D = 1204, GH_COPY = 1210, GH_ST = 1210;
+constexpr int GH_REC = 1238;                     // doubles per record (9904 bytes)
+constexpr int GH_LR = 80;                        // per GhostBC slot and stage: L, R, lambda (78), pad (ghost update's scratch)
 
 constexpr int CELL_TILE = 128;
 constexpr int FLUX_FACES = 64;                   // faces per flux block
