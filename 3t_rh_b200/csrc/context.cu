@@ -145,7 +145,9 @@ int enqueue_flux(rh3t_ctx* c, cudaStream_t s, int stage, Span r) {
 
 void enqueue_rhs(rh3t_ctx* c, cudaStream_t s, int stage, int mode, double* rhs, Span r) {
     const HostInst &a = c->hi[r.k0], &b = c->hi[r.k1 - 1];
-    launch_rhs_stage(s, c->d_inst, c->d_tr + a.tr0, b.tr0 + b.ntr - a.tr0, stage, mode, rhs);
+    int smem = 0;
+    for (int k = r.k0; k < r.k1; ++k) smem = std::max(smem, rhs_smem(c->hi[k].shape.lgr));
+    launch_rhs_stage(s, c->d_inst, c->d_tr + a.tr0, b.tr0 + b.ntr - a.tr0, stage, mode, rhs, smem);
 }
 
 } // namespace rh3t

@@ -21,7 +21,10 @@ int flux_points(int dir, int lg);
 void launch_flux(cudaStream_t s, const Inst* insts, const Tile* tx, int ntx, const Tile* ty, int nty, int stage,
                  const FluxSize& z);
 int flux_launches(int ntx, int nty);
-void launch_rhs_stage(cudaStream_t s, const Inst* insts, const Tile* tc, int nt, int stage, int mode, double* rhs);
+// smem: rhs_smem of the launch's largest tile
+int rhs_smem(int lg);
+void launch_rhs_stage(cudaStream_t s, const Inst* insts, const Tile* tc, int nt, int stage, int mode, double* rhs,
+                      int smem);
 void launch_dt(cudaStream_t s, const Inst* insts, const Tile* tc, int nt, int mode);
 void launch_set_dt(cudaStream_t s, const Inst* insts, int n_inst, double dt);
 void launch_scatter(cudaStream_t s, const Inst* insts, int k0, int n, long long max_cells, const double* aos,

@@ -93,6 +93,7 @@ struct DivEach {
     bool ok = true;
     __device__ __forceinline__ Recip den(double b) { return recip(b); }
     __device__ __forceinline__ double div(double a, const Recip& d) { return div_rn(a, d); }
+    __device__ __forceinline__ double div3(double a) { return div3_rn(a); }
     __device__ __forceinline__ double div6(double a) { return div6_rn(a); }
 };
 struct DivGroup {
@@ -105,6 +106,7 @@ struct DivGroup {
         ok = ok & num_near(a);
         return div_near(a, d);
     }
+    __device__ __forceinline__ double div3(double a) { return div3_near(a); } // any finite a
     __device__ __forceinline__ double div6(double a) {
         ok = ok & num_near(a);
         return div6_near(a);
@@ -762,33 +764,31 @@ __device__ __forceinline__ void noncon9(const double pe[9], const double pi[9], 
     out[2] = v / 3.0 * der_er + (coef_left * jm_er + coef_right * jp_er) / ds;
 }
 
-// noncon9 with the divisors 60 ds and ds given with their reciprocals (the
-// same quotients, divrn.cuh), for callers that hold them for many cells
-__device__ __forceinline__ void noncon9(const double pe[9], const double pi[9], const double pr[9],
-                                        const double vel[9], const Recip& r60ds, const Recip& rds, double out[3]) {
-    double v = vel[4];
+// noncon9 from the jumps at the cell's two interfaces (jm, jp; each interface's
+// are formed once and shared by its two cells) and from the pressures and
+// the transport velocity in memory at centre p, stride st. r60ds, rds: the
+// divisors 60 ds and ds.
+template <class DV, class R>
+__device__ __forceinline__ void noncon_by(const double* pe, const double* pi, const double* pr, const double* vel,
+                                          int st, const double jm[3], const double jp[3], const R& r60ds,
+                                          const R& rds, DV& dv, double out[3]) {
+    const double v = vel[0];
     auto d6r = [&](const double* q) {
-        return div_rn(q[7] - 9.0 * q[6] + 45.0 * q[5] - 45.0 * q[3] + 9.0 * q[2] - q[1], r60ds);
+        return dv.div(q[3 * st] - 9.0 * q[2 * st] + 45.0 * q[st] - 45.0 * q[-st] + 9.0 * q[-2 * st] - q[-3 * st], r60ds);
     };
-    double dpe = d6r(pe), dpi = d6r(pi), dpr = d6r(pr);
-    double der_ee = 2.0 * dpe - dpi - dpr;
-    double der_ei = 2.0 * dpi - dpe - dpr;
-    double der_er = 2.0 * dpr - dpe - dpi;
-    double nee[9], nei[9], ner[9];
+    const double dpe = d6r(pe), dpi = d6r(pi), dpr = d6r(pr);
+    const double der[3] = {2.0 * dpe - dpi - dpr, 2.0 * dpi - dpe - dpr, 2.0 * dpr - dpe - dpi};
+    const double coef_left = dv.div3(fmax(fmax(v, vel[-st]), 0.0));
+    const double coef_right = dv.div3(fmin(fmin(v, vel[st]), 0.0));
+    const double v3 = dv.div3(v);
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        nee[k] = 2.0 * pe[k] - pi[k] - pr[k];
-        nei[k] = 2.0 * pi[k] - pe[k] - pr[k];
-        ner[k] = 2.0 * pr[k] - pe[k] - pi[k];
-    }
-    double jm_ee = jump8(nee), jm_ei = jump8(nei), jm_er = jump8(ner);
-    double jp_ee = jump8(nee + 1), jp_ei = jump8(nei + 1), jp_er = jump8(ner + 1);
-    double coef_left = div3_rn(fmax(fmax(v, vel[3]), 0.0));
-    double coef_right = div3_rn(fmin(fmin(v, vel[5]), 0.0));
-    const double v3 = div3_rn(v);
-    out[0] = v3 * der_ee + div_rn(coef_left * jm_ee + coef_right * jp_ee, rds);
-    out[1] = v3 * der_ei + div_rn(coef_left * jm_ei + coef_right * jp_ei, rds);
-    out[2] = v3 * der_er + div_rn(coef_left * jm_er + coef_right * jp_er, rds);
+    for (int c = 0; c < 3; ++c) out[c] = v3 * der[c] + dv.div(coef_left * jm[c] + coef_right * jp[c], rds);
+}
+static __device__ __noinline__ void noncon_each(const double* pe, const double* pi, const double* pr,
+                                                const double* vel, int st, const double* jm, const double* jp,
+                                                double ds, double* out) {
+    DivEach dv;
+    noncon_by(pe, pi, pr, vel, st, jm, jp, dv.den(60.0 * ds), dv.den(ds), dv, out);
 }
 
 // dt.rs:5-34 get_local_dt (same association order; CVE^3 = CVE*(CVE*CVE)),
@@ -817,33 +817,60 @@ __device__ __forceinline__ T local_dt_t(const T s[6], double dx, double dy, cons
     return P.lambda / vj;
 }
 
+// local_dt_t over double by either form of quotients, the five by rho through
+// one reciprocal and w2 / 6 formed once
+template <class DV>
+__device__ __forceinline__ double local_dt_by(const double s[6], double dx, double dy, const DevParams& P, DV& dv) {
+    const double OEI = P.omega_ei, OER = P.omega_er;
+    const auto r0 = dv.den(s[0]);
+    const double u = dv.div(s[1], r0), v = dv.div(s[2], r0);
+    const double w6 = dv.div6(sqd(u) + sqd(v));
+    const double ee = dv.div(s[3], r0) - w6, ei = dv.div(s[4], r0) - w6, er = dv.div(s[5], r0) - w6;
+    const double GE = P.gamma_e, GI = P.gamma_i, GR = P.gamma_r, A = P.a_rad, CVE = P.cve, CVI = P.cvi;
+    const double gi = GI - 1.0, ge = GE - 1.0, gr = GR - 1.0;
+    const double cs = sqrt(GE * ge * ee + GI * gi * ei + GR * gr * er);
+    const double c4 = (CVE * CVE) * (CVE * CVE), c3 = CVE * (CVE * CVE);
+    const double ee3 = ee * (ee * ee);
+    const double t1 = A * OEI * c4 + A * OEI * c3 * CVI + 4.0 * A * OER * CVI * ee3 + OER * c4 * CVI * s[0];
+    const double s1 = sqrt(sqd(t1) - 4.0 * A * OEI * OER * c4 * CVI * (4.0 * A * ee3 + c4 * s[0] + c3 * CVI * s[0]));
+    const double s2 = -(A * OEI * c4 + A * OEI * c3 * CVI + 4.0 * A * OER * CVI * ee3 + OER * c4 * CVI * s[0]);
+    const auto sden = dv.den(2.0 * A * c4 * CVI * s[0]);
+    const double sj = fmax(fabs(dv.div(-s1 + s2, sden)), fabs(dv.div(s1 + s2, sden)));
+    const double dj = fmax(fmax(dv.div(P.kappa_e, dv.den(CVE * s[0])), dv.div(P.kappa_i, dv.den(CVI * s[0]))),
+                           dv.div(P.kappa_r, dv.den(A)));
+    const double vj = dv.div(fabs(u) + cs, dv.den(dx)) + dv.div(2.0 * dj, dv.den(sqd(dx) + sqd(dy))) + sj +
+                      dv.div(fabs(v) + cs, dv.den(dy));
+    return dv.div(P.lambda, dv.den(vj));
+}
+static __device__ __noinline__ double local_dt_each(const double* s, double dx, double dy, const DevParams& P) {
+    DivEach dv;
+    return local_dt_by(s, dx, dy, P, dv);
+}
 __device__ __forceinline__ double local_dt(const double s[6], double dx, double dy, const DevParams& P) {
-    return local_dt_t<double>(s, dx, dy, P, P.omega_ei, P.omega_er);
+    DivGroup dv;
+    const double d = local_dt_by(s, dx, dy, P, dv);
+    if (dv.ok) return d;
+    const double t[6] = {s[0], s[1], s[2], s[3], s[4], s[5]};
+    return local_dt_each(t, dx, dy, P);
 }
 
 namespace fastm {
 
-// noncon.rs:288-332 with the divisions by 60 ds, 3 and ds as multiplications
-__device__ __forceinline__ void noncon9(const double pe[9], const double pi[9], const double pr[9],
-                                        const double vel[9], double inv_60ds, double inv_ds, double out[3]) {
-    const double v = vel[4];
+// noncon_by with the divisions by 60 ds, 3 and ds as multiplications
+__device__ __forceinline__ void noncon(const double* pe, const double* pi, const double* pr, const double* vel, int st,
+                                       const double jm[3], const double jp[3], double inv_60ds, double inv_ds,
+                                       double out[3]) {
+    const double v = vel[0];
     auto d6f = [&](const double* q) {
-        return (q[7] - 9.0 * q[6] + 45.0 * q[5] - 45.0 * q[3] + 9.0 * q[2] - q[1]) * inv_60ds;
+        return (q[3 * st] - 9.0 * q[2 * st] + 45.0 * q[st] - 45.0 * q[-st] + 9.0 * q[-2 * st] - q[-3 * st]) * inv_60ds;
     };
     const double dpe = d6f(pe), dpi = d6f(pi), dpr = d6f(pr);
     const double der[3] = {2.0 * dpe - dpi - dpr, 2.0 * dpi - dpe - dpr, 2.0 * dpr - dpe - dpi};
-    double n[3][9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        n[0][k] = 2.0 * pe[k] - pi[k] - pr[k];
-        n[1][k] = 2.0 * pi[k] - pe[k] - pr[k];
-        n[2][k] = 2.0 * pr[k] - pe[k] - pi[k];
-    }
-    const double cl = fmax(fmax(v, vel[3]), 0.0) * (1.0 / 3.0) * inv_ds;
-    const double cr = fmin(fmin(v, vel[5]), 0.0) * (1.0 / 3.0) * inv_ds;
+    const double cl = fmax(fmax(v, vel[-st]), 0.0) * (1.0 / 3.0) * inv_ds;
+    const double cr = fmin(fmin(v, vel[st]), 0.0) * (1.0 / 3.0) * inv_ds;
     const double v3 = v * (1.0 / 3.0);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) out[c] = v3 * der[c] + (cl * jump8(n[c]) + cr * jump8(n[c] + 1));
+    for (int c = 0; c < 3; ++c) out[c] = v3 * der[c] + (cl * jm[c] + cr * jp[c]);
 }
 
 } // namespace fastm

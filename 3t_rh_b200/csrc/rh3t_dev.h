@@ -136,7 +136,7 @@ constexpr int FX_LG_DEF = 3, FY_LG_DEF = 4, RHS_LG_DEF = 5;
 // staged points per flux block: max over shapes of (TI + 5) * TJ (x) and
 // TI * (TJ + 5) (y)
 constexpr int FLUX_NPT = 144;
-// RHS halo points: max over shapes of (TI + 8) * (TJ + 8)
+// halo points of a cell tile: max over shapes of (TI + 8) * (TJ + 8)
 constexpr int RHS_NPT = 864;
 
 } // namespace rh3t

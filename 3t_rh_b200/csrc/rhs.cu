@@ -3,16 +3,29 @@
 // exchange source (source.rs:7-21) and the diffusion differences, then
 // u' = a u + b v + c dt rhs with the admissibility check (main.rs:22-33).
 //
-// A block covers TI x TJ = 256 cells (shape chosen per tile). The pressures and the transport
-// velocities of the nodes within reach of the 9-point non-conservative
-// stencils (the tile plus a 4-node halo, corners excluded) are computed once
-// into shared memory; the reference's access-table gathers (main.rs:276-277)
-// evaluate them once per use, 17 times per node.
+// A block covers TI x TJ = 256 cells (shape chosen per tile) in three phases:
+//   1. the pressures, the transport velocities and the pressure differences
+//      2 p_k - p_l - p_m of the nodes within reach of the 9-point non-conservative
+//      stencils (the tile plus a 4-node halo, corners excluded) go to shared
+//      memory once; the reference's access-table gathers (main.rs:276-277)
+//      evaluate them once per use, 17 times per node;
+//   2. the jumps of the three differences at every interface of the tile: the
+//      reference forms those at a cell's left and right (lower and upper)
+//      interface in each of the two cells they belong to (noncon.rs:259-285);
+//   3. one cell per thread.
+// Bound by latency (24 face fluxes and the stage inputs a cell) and the FP64
+// pipe. Forming a jump once, and quotients without a branch each (divrn.cuh), take
+// away a third of the FP64 operations and the registers that held two 9-point
+// windows, so three blocks fit an SM instead of two: 24 batch instances 107 us a
+// stage instead of 153 us, the 961 x 3841 half-cylinder 318 us instead of 453 us
+// (two blocks of 119 registers: 399 us, four of 64, spills: 369 us).
 //
 // mode 0 writes the rhs (6 planes of nx*ny, i*ny+j, instance k at
 // rhs_out + 6*cell_off) for l(); mode 1 applies the stage update of `stage`;
 // mode 2 does both, the rhs into padded planes at rhs_out + aoff (the
 // adjoint's record of the forward stages).
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "physics.cuh"
@@ -24,6 +37,7 @@ constexpr bool kExactR = true;
 #else
 constexpr bool kExactR = false;
 #endif
+constexpr int RHS_BLOCKS = 3; // per SM: 80 registers
 
 // divisors shared by every cell of an instance: 60 dx, dx, 60 dy, dy
 // (noncon.rs:26-44, 315-331), 6 cve, 6 cvi, a_rad (state.rs:245-276)
@@ -39,14 +53,33 @@ __device__ __forceinline__ double rhs_divisor(const Inst& I, int k) {
     default: return I.P.a_rad;
     }
 }
-__device__ __forceinline__ Recip rhs_recip(const Inst& I, const double* sR, int k) {
-    return recip_of(rhs_divisor(I, k), sR[k]);
+// sR: the two parts of their reciprocals
+__device__ __forceinline__ RecipN rhs_recip(const Inst& I, const double* sR, int k) {
+    return {rhs_divisor(I, k), sR[k], sR[RHS_NR + k]};
 }
 
-__global__ void __launch_bounds__(RHS_THREADS, 2) k_rhs_stage(const Inst* __restrict__ insts, const Tile* __restrict__ tiles,
+// Shared memory of a tile of shape lg: p_e, p_i, p_r, u, v and the three
+// differences per node, the jumps per x and y interface, the reciprocals
+__host__ __device__ __forceinline__ int rhs_nodes(int lg) { return ((RHS_THREADS >> lg) + 8) * ((1 << lg) + 8); }
+__host__ __device__ __forceinline__ int rhs_xfaces(int lg) { return RHS_THREADS + (1 << lg); }
+__host__ __device__ __forceinline__ int rhs_yfaces(int lg) { return RHS_THREADS + (RHS_THREADS >> lg); }
+int rhs_smem(int lg) { return 8 * (8 * rhs_nodes(lg) + 3 * (rhs_xfaces(lg) + rhs_yfaces(lg)) + 2 * RHS_NR); }
+
+// jumps of the three differences (planes of npt nodes) over the 8 nodes from p
+// at stride st (noncon.rs:259-285)
+__device__ __forceinline__ void jumps(const double* sN, int npt, int p, int st, double* out, int stride) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        double a[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) a[q] = sN[c * npt + p + q * st];
+        out[c * stride] = jump8(a);
+    }
+}
+
+__global__ void __launch_bounds__(RHS_THREADS, RHS_BLOCKS) k_rhs_stage(const Inst* __restrict__ insts, const Tile* __restrict__ tiles,
                                                    int nt, int stage, int mode, double* __restrict__ rhs_out) {
-    __shared__ double sP[5][RHS_NPT]; // pe, pi, pr, u, v
-    __shared__ double sR[RHS_NR];      // reciprocals of the instance's divisors (rhs_divisor)
+    extern __shared__ double rhs_mem[];
     if (blockIdx.x >= nt) return;
     const Tile t = tiles[blockIdx.x];
     const Inst& I = insts[t.inst];
@@ -56,10 +89,19 @@ __global__ void __launch_bounds__(RHS_THREADS, 2) k_rhs_stage(const Inst* __rest
     const double* __restrict__ src = stage_src(I, stage);
     const int nx = I.nx, ny = I.ny;
     const int TJ = 1 << t.lg, TI = RHS_THREADS >> t.lg;
-    const int HJ = TJ + 8, NPT = (TI + 8) * HJ;
-    if (threadIdx.x < RHS_NR) sR[threadIdx.x] = __ddiv_rn(1.0, rhs_divisor(I, threadIdx.x));
-    // ---- stage node primitives (tile + 4-node cross halo)
-    for (int p = threadIdx.x; p < NPT; p += blockDim.x) {
+    const int HJ = TJ + 8, NPT = (TI + 8) * HJ, nfx = rhs_xfaces(t.lg), nfy = rhs_yfaces(t.lg);
+    double* sP = rhs_mem;            // [5][NPT] p_e, p_i, p_r, u, v
+    double* sN = sP + 5 * NPT;       // [3][NPT] 2 p_e - p_i - p_r, 2 p_i - p_e - p_r, 2 p_r - p_e - p_i
+    double* sX = sN + 3 * NPT;       // [3][nfx] jumps at x interface (a, tj): a * TJ + tj
+    double* sY = sX + 3 * nfx;       // [3][nfy] jumps at y interface (ti, b): ti * (TJ + 1) + b
+    double* sR = sY + 3 * nfy;       // [2][RHS_NR] reciprocals of the instance's divisors
+    if (threadIdx.x < RHS_NR) {
+        const RecipN r = recip_near(rhs_divisor(I, threadIdx.x));
+        sR[threadIdx.x] = r.y;
+        sR[RHS_NR + threadIdx.x] = r.yl;
+    }
+    // ---- 1. stage node primitives (tile + 4-node cross halo)
+    for (int p = threadIdx.x; p < NPT; p += RHS_THREADS) {
         const int hi = p / HJ, hj = p - hi * HJ;
         const bool corner = (hi < 4 || hi >= TI + 4) && (hj < 4 || hj >= TJ + 4);
         const int i = t.i - 4 + hi, j = t.j0 - 4 + hj;
@@ -67,10 +109,22 @@ __global__ void __launch_bounds__(RHS_THREADS, 2) k_rhs_stage(const Inst* __rest
         double s[6];
         load6(src, plane, node_of(I, i, j), s);
         Prim d = kExactR ? prim_from_state(s, P) : fastm::prim(s, P);
-        sP[0][p] = d.pe; sP[1][p] = d.pi; sP[2][p] = d.pr; sP[3][p] = d.u; sP[4][p] = d.v;
+        sP[p] = d.pe; sP[NPT + p] = d.pi; sP[2 * NPT + p] = d.pr; sP[3 * NPT + p] = d.u; sP[4 * NPT + p] = d.v;
+        sN[p] = 2.0 * d.pe - d.pi - d.pr;
+        sN[NPT + p] = 2.0 * d.pi - d.pe - d.pr;
+        sN[2 * NPT + p] = 2.0 * d.pr - d.pe - d.pi;
     }
     __syncthreads();
     const int ti = threadIdx.x >> t.lg, tj = threadIdx.x & (TJ - 1);
+    // ---- 2. jumps: this cell's left and lower interfaces, then the tile's far edges
+    jumps(sN, NPT, ti * HJ + tj + 4, HJ, sX + threadIdx.x, nfx);
+    jumps(sN, NPT, (ti + 4) * HJ + tj, 1, sY + ti * (TJ + 1) + tj, nfy);
+    if (threadIdx.x < TJ)
+        jumps(sN, NPT, TI * HJ + threadIdx.x + 4, HJ, sX + TI * TJ + threadIdx.x, nfx);
+    else if (threadIdx.x < TJ + TI)
+        jumps(sN, NPT, (threadIdx.x - TJ + 4) * HJ + TJ, 1, sY + (threadIdx.x - TJ) * (TJ + 1) + TJ, nfy);
+    __syncthreads();
+    // ---- 3. this thread's cell
     const int i = t.i + ti, j = t.j0 + tj;
     if (i >= nx || j >= ny) return;
     const long long n = node_of(I, i, j);
@@ -86,29 +140,52 @@ __global__ void __launch_bounds__(RHS_THREADS, 2) k_rhs_stage(const Inst* __rest
         const double fb = I.fy[c * fpy + fiy], ft = I.fy[c * fpy + fiy + 1];
         rhs[c] = -(fr - fl) * sx + -(ft - fb) * sy;
     }
-    double pe[9], pi[9], pr[9], vel[9], ncx[3], ncy[3];
-    const int hc = (ti + 4) * HJ + (tj + 4);
+    double ncx[3], ncy[3];
+    const double* c0 = sP + (ti + 4) * HJ + (tj + 4);
+    {
+        const int ix = threadIdx.x, iy = ti * (TJ + 1) + tj;
+        double jm[3], jp[3];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        const int p = hc + (q - 4) * HJ;
-        pe[q] = sP[0][p]; pi[q] = sP[1][p]; pr[q] = sP[2][p]; vel[q] = sP[3][p];
-    }
-    if (kExactR) noncon9(pe, pi, pr, vel, rhs_recip(I, sR, 0), rhs_recip(I, sR, 1), ncx);
-    else fastm::noncon9(pe, pi, pr, vel, 1.0 / (60.0 * dx), 1.0 / dx, ncx);
+        for (int c = 0; c < 3; ++c) { jm[c] = sX[c * nfx + ix]; jp[c] = sX[c * nfx + ix + TJ]; }
+        if (kExactR) {
+            DivGroup dv;
+            noncon_by(c0, c0 + NPT, c0 + 2 * NPT, c0 + 3 * NPT, HJ, jm, jp, rhs_recip(I, sR, 0), rhs_recip(I, sR, 1), dv,
+                      ncx);
+            if (!(dv.ok & den_near(60.0 * dx) & den_near(dx))) {
+                const double a[3] = {jm[0], jm[1], jm[2]}, b[3] = {jp[0], jp[1], jp[2]};
+                double o[3];
+                noncon_each(c0, c0 + NPT, c0 + 2 * NPT, c0 + 3 * NPT, HJ, a, b, dx, o);
 #pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        const int p = hc + (q - 4);
-        pe[q] = sP[0][p]; pi[q] = sP[1][p]; pr[q] = sP[2][p]; vel[q] = sP[4][p];
+                for (int c = 0; c < 3; ++c) ncx[c] = o[c];
+            }
+        } else {
+            fastm::noncon(c0, c0 + NPT, c0 + 2 * NPT, c0 + 3 * NPT, HJ, jm, jp, 1.0 / (60.0 * dx), 1.0 / dx, ncx);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) { jm[c] = sY[c * nfy + iy]; jp[c] = sY[c * nfy + iy + 1]; }
+        if (kExactR) {
+            DivGroup dv;
+            noncon_by(c0, c0 + NPT, c0 + 2 * NPT, c0 + 4 * NPT, 1, jm, jp, rhs_recip(I, sR, 2), rhs_recip(I, sR, 3), dv,
+                      ncy);
+            if (!(dv.ok & den_near(60.0 * dy) & den_near(dy))) {
+                const double a[3] = {jm[0], jm[1], jm[2]}, b[3] = {jp[0], jp[1], jp[2]};
+                double o[3];
+                noncon_each(c0, c0 + NPT, c0 + 2 * NPT, c0 + 4 * NPT, 1, a, b, dy, o);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) ncy[c] = o[c];
+            }
+        } else {
+            fastm::noncon(c0, c0 + NPT, c0 + 2 * NPT, c0 + 4 * NPT, 1, jm, jp, 1.0 / (60.0 * dy), 1.0 / dy, ncy);
+        }
     }
-    if (kExactR) noncon9(pe, pi, pr, vel, rhs_recip(I, sR, 2), rhs_recip(I, sR, 3), ncy);
-    else fastm::noncon9(pe, pi, pr, vel, 1.0 / (60.0 * dy), 1.0 / dy, ncy);
 #pragma unroll
     for (int k = 0; k < 3; ++k) rhs[3 + k] = rhs[3 + k] + ncx[k] + ncy[k];
     if (I.source) {
         double s[6];
         load6(src, plane, n, s);
         double te, ti_, tr;
-        temps_from_state(s, P, te, ti_, tr);
+        temps_from_state(s, P, rhs_recip(I, sR, 4), rhs_recip(I, sR, 5), rhs_recip(I, sR, 6),
+                         den_near(6.0 * P.cve) & den_near(6.0 * P.cvi) & den_near(P.a_rad), te, ti_, tr);
         const double so[3] = {-P.omega_ei * (te - ti_) - P.omega_er * (pow4d(te) - pow4d(tr)),
                               P.omega_ei * (te - ti_), P.omega_er * (pow4d(te) - pow4d(tr))};
 #pragma unroll
@@ -159,18 +236,37 @@ __global__ void __launch_bounds__(RHS_THREADS, 2) k_rhs_stage(const Inst* __rest
     }
     bool ok = isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]) && isfinite(v[3]) && isfinite(v[4]) &&
               isfinite(v[5]) && v[0] > 0.0;
-    if (ok) { // main.rs:24-33, the five quotients by rho through one reciprocal (the same IEEE quotients)
-        const Recip r0 = recip(v[0]);
-        const double ux = div_rn(v[1], r0), uy = div_rn(v[2], r0);
-        const double k = div6_rn(ux * ux + uy * uy);
-        ok = !(div_rn(v[3], r0) - k <= 0.0 || div_rn(v[4], r0) - k <= 0.0 || div_rn(v[5], r0) - k <= 0.0);
+    if (ok) { // main.rs:24-33
+        // an energy e > rho w2 / 6 beyond any rounding passes without the exact
+        // quotients: y is 1 / rho to 2^-39, the products below to 2^-37
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v[0]));
+        y = __fma_rn(y, __fma_rn(-v[0], y, 1.0), y);
+        const double ux = v[1] * y, uy = v[2] * y, e = fmin(fmin(v[3], v[4]), v[5]) * y;
+        if (!(e > (ux * ux + uy * uy) * (1.0 / 6.0) * (1.0 + 1e-9) + 1e-290)) {
+            const Recip r0 = recip(v[0]); // the five quotients by rho through one reciprocal (IEEE quotients)
+            const double qx = div_rn(v[1], r0), qy = div_rn(v[2], r0);
+            const double k = div6_rn(qx * qx + qy * qy);
+            ok = !(div_rn(v[3], r0) - k <= 0.0 || div_rn(v[4], r0) - k <= 0.0 || div_rn(v[5], r0) - k <= 0.0);
+        }
     }
     if (!ok) report(I, 2 + 2 * stage, 1, (unsigned)((long long)i * ny + j));
 }
 
-void launch_rhs_stage(cudaStream_t s, const Inst* insts, const Tile* tc, int nt, int stage, int mode, double* rhs) {
+void launch_rhs_stage(cudaStream_t s, const Inst* insts, const Tile* tc, int nt, int stage, int mode, double* rhs,
+                      int smem) {
     if (nt <= 0) return;
-    k_rhs_stage<<<nt, RHS_THREADS, 0, s>>>(insts, tc, nt, stage, mode, rhs);
+    static bool attr[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!attr[dev]) {
+        int most = 0;
+        for (int lg = RHS_LG_MIN; lg <= RHS_LG_MAX; ++lg) most = std::max(most, rhs_smem(lg));
+        cudaFuncSetAttribute(k_rhs_stage, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        attr[dev] = true;
+    }
+    k_rhs_stage<<<nt, RHS_THREADS, smem, s>>>(insts, tc, nt, stage, mode, rhs);
 }
 
 } // namespace rh3t

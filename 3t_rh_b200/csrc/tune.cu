@@ -73,7 +73,7 @@ int time_kind(rh3t_ctx* c, Kind kind, const std::vector<Tile>& tiles, const Shap
     auto launch = [&]() {
         if (kind == KX) launch_flux(s, c->d_inst, d, n, nullptr, 0, 0, z);
         else if (kind == KY) launch_flux(s, c->d_inst, nullptr, 0, d, n, 0, z);
-        else launch_rhs_stage(s, c->d_inst, d, n, 0, 0, c->d_io2);
+        else launch_rhs_stage(s, c->d_inst, d, n, 0, 0, c->d_io2, rhs_smem(sh.lgr));
         c->launches += 1;
     };
     double best = 1e30;
