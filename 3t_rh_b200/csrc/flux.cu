@@ -2,7 +2,8 @@
 // x and y face, plus diffusion.rs:27-50 when diffusion is on).
 //
 // A block of two warps covers 64 faces (a TI x TJ tile, shape chosen per
-// tile), one face per thread:
+// tile), one face per thread (small launches: up to three threads, each with
+// two or three of the characteristic fields):
 //   1. staging: the tile's stencil points (x faces: (TI + 5) x TJ points,
 //      y faces: TI x (TJ + 5)) with their primitives and physical flux go to
 //      shared memory once (the reference evaluates them once per face, six
@@ -53,18 +54,20 @@ constexpr bool kExact = false;
 //       (recip_near, both parts) of den, b, gt cs2; FMA build 1/cs2, 1/b;
 //   T:  per point te, ti, tr (launches with a diffusive instance);
 //   gkgt, y6: no-contraction build, gk / gt and the reciprocal of 6 gk (both
-//       parts) for gk = ge, gi, gr.
+//       parts) for gk = ge, gi, gr;
+//   act: per face 0 (no flux), 1 (quotients in the branch-free form) or 2.
 constexpr int NQ = kExact ? 19 : 15, PT = 7;
 struct FluxShared {
     double2* pt;
     double *E, *G, *Q, *T, *gkgt, *y6;
+    int* act;
     int npt;
 };
 __host__ __device__ __forceinline__ int flux_e_doubles(int npt) {
     return 4 * npt > 6 * FLUX_FACES ? 4 * npt : 6 * FLUX_FACES;
 }
 __host__ __device__ __forceinline__ int flux_smem(int npt, bool diffusion) {
-    return npt * PT * 16 + 8 * (flux_e_doubles(npt) + NQ * FLUX_FACES + 10 + (diffusion ? 3 * npt : 0));
+    return npt * PT * 16 + 8 * (flux_e_doubles(npt) + NQ * FLUX_FACES + 10 + FLUX_FACES / 2 + (diffusion ? 3 * npt : 0));
 }
 __device__ __forceinline__ FluxShared flux_shared(unsigned char* smem, int npt) {
     FluxShared S;
@@ -73,7 +76,8 @@ __device__ __forceinline__ FluxShared flux_shared(unsigned char* smem, int npt) 
     S.Q = reinterpret_cast<double*>(S.pt + npt * PT);
     S.gkgt = S.Q + NQ * FLUX_FACES;
     S.y6 = S.gkgt + 3;
-    S.E = S.gkgt + 10;
+    S.act = reinterpret_cast<int*>(S.gkgt + 10);
+    S.E = S.gkgt + 10 + FLUX_FACES / 2;
     S.G = S.E;
     S.T = S.E + flux_e_doubles(npt);
     return S;
@@ -240,7 +244,16 @@ static __device__ __noinline__ double r_dot_each(const double* Qf, const double*
     return r_dot<DIR, false>(q, Gf, nullptr, P, k);
 }
 
-template <int DIR>
+// Field `m` of group `g` when NG groups of 64 threads share a tile's six fields
+// (each group about the same work: x faces: fields 1-3 energy, 0 and 5
+// acoustic, 4 transverse; y faces 2-4, 0 and 5, 1), a hex digit each
+template <int DIR, int NG> __device__ __forceinline__ int group_field(int g, int m) {
+    constexpr unsigned long long x = NG == 1 ? 0x543210ull : (NG == 2 ? 0x350421ull : 0x435201ull);
+    constexpr unsigned long long y = NG == 1 ? 0x543210ull : (NG == 2 ? 0x450132ull : 0x145302ull);
+    return (int)((DIR == 0 ? x : y) >> (4 * (g * (6 / NG) + m))) & 15;
+}
+
+template <int DIR, int NG>
 __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stage, const FluxShared& S) {
     const DevParams& P = I.P;
     const double* __restrict__ buf = stage_src(I, stage);
@@ -259,7 +272,7 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
         S.y6[3 + k] = r.yl;
     }
     // ---- 1. staging: state, primitives and physical flux of every point
-    for (int p = threadIdx.x; p < np; p += FLUX_THREADS) {
+    for (int p = threadIdx.x; p < np; p += FLUX_FACES * NG) {
         int pi, pj;
         if (DIR == 0) { pi = t.i - 3 + (p >> t.lg); pj = t.j0 + (p & (cols - 1)); }
         else { const int r = p / (cols + 5); pi = t.i + r; pj = t.j0 - 3 + (p - r * (cols + 5)); }
@@ -279,8 +292,8 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
         S.E[p] = d.e_e; S.E[npt + p] = d.e_i; S.E[2 * npt + p] = d.e_r; S.E[3 * npt + p] = sqrt(s[0]);
         if (diff) stage_temps(q, P, S.T + p, npt);
     }
-    // ---- 2. this thread's face
-    const int f = threadIdx.x;
+    // ---- 2. this thread's face (its Roe state by the first group)
+    const int f = NG == 1 ? threadIdx.x : threadIdx.x & (FLUX_FACES - 1), g = NG == 1 ? 0 : threadIdx.x / FLUX_FACES;
     int i, j, p0, ps;
     face_index<DIR>(t, f, i, j, p0, ps);
     bool valid = DIR == 0 ? (i <= nx && j < ny) : (i < nx && j <= ny);
@@ -292,7 +305,7 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
     __syncthreads();
     double* Qf = S.Q + f;
     bool near = true;
-    if (valid) {
+    if (valid && g == 0) {
         // points[3] and points[2] of the face: the staged primitives (the
         // same functions of the same states as a fresh evaluation)
         const int p3 = p0 + 3 * ps, p2 = p0 + 2 * ps;
@@ -322,14 +335,25 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
 #pragma unroll
         for (int k = 13; k < NQ; ++k) Qf[k * FLUX_FACES] = y[k - 13];
     }
+    if (NG > 1 && g == 0) S.act[f] = near ? 1 : 2;
     __syncthreads(); // E is read; G takes its place
-    if (!valid) return;
+    if (NG == 1 && !valid) return;
+    if (NG > 1) near = S.act[f] == 1;
     // ---- 3. characteristic pass (a loop, not unrolled: one copy of its code
     // stays within the instruction cache)
     double* Gf = S.G + f;
     const double2* pf = S.pt + PT * p0;
+    if (NG == 1 || valid) {
 #pragma unroll 1
-    for (int c = 0; c < 6; ++c) Gf[c * FLUX_FACES] = char_flux<DIR>(pf, PT * ps, Qf, P, c, S.gkgt, near);
+        for (int m = 0; m < 6 / NG; ++m) {
+            const int c = NG == 1 ? m : group_field<DIR, NG>(g, m);
+            Gf[c * FLUX_FACES] = char_flux<DIR>(pf, PT * ps, Qf, P, c, S.gkgt, near);
+        }
+    }
+    if (NG > 1) {
+        __syncthreads();
+        if (!valid) return;
+    }
     // ---- 4. output pass
     long long fplane, fidx;
     double *fo, *dfo;
@@ -339,31 +363,44 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
         Roe q;
         load_q(Qf, q);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) fo[k * fplane + fidx] = r_dot<DIR, kExact>(q, Gf, S.y6, P, k);
+        for (int k = 0; k < 6; ++k)
+            if (NG == 1 || k % NG == g) fo[k * fplane + fidx] = r_dot<DIR, kExact>(q, Gf, S.y6, P, k);
     } else {
 #pragma unroll 1
-        for (int k = 0; k < 6; ++k) fo[k * fplane + fidx] = r_dot_each<DIR>(Qf, Gf, P, k);
+        for (int k = g; k < 6; k += NG) fo[k * fplane + fidx] = r_dot_each<DIR>(Qf, Gf, P, k);
     }
     if (diff)
 #pragma unroll 1
-        for (int m = 0; m < 3; ++m) diffusion_out(S.T + m * npt + p0, ps, P, m, dfo + m * fplane + fidx);
+        for (int m = g; m < 3; m += NG) diffusion_out(S.T + m * npt + p0, ps, P, m, dfo + m * fplane + fidx);
 }
 
+constexpr int FLUX_NG3 = 2 * 148, FLUX_NG2 = 4 * 148; // tiles up to which 3 and 2 groups share a tile
 // blocks per SM (FMA build: 12 blocks of 80 registers 2% faster than 8)
 #ifndef FLUX_MIN_BLOCKS
 #define FLUX_MIN_BLOCKS (kExact ? 8 : 12)
 #endif
-// x faces and y faces in two launches: each kernel holds one direction's
-// code, half of what an instruction cache shared by both would need
-template <int DIR>
-__global__ void __launch_bounds__(FLUX_THREADS, FLUX_MIN_BLOCKS) k_flux(const Inst* __restrict__ insts,
-                                                                     const Tile* __restrict__ tiles, int stage,
-                                                                     int npt) {
+// x faces (blocks [0, ntx)), then y faces: in one launch the y tiles fill the
+// SMs that the last x tiles leave idle (121 x 481: two launches of 0.8 waves each
+// took 42 us, one takes 31 us).
+// NG groups of 64 threads share a tile where the launch has too few tiles to
+// fill the SMs: at one thread a face a small launch is one face's serial chain
+// (about 14 cycles an FP64 operation at a warp or two per scheduler). Three
+// groups while the tiles fit two blocks of 192 threads a SM, two while they fit
+// four of 128, one beyond (a step's fluxes, one / two / three groups: 31x121, 128
+// tiles, 48 / 40 / 40 us; 512x8 planar shock, 193 tiles, 53 / 48 / 45; 61x241, 492
+// tiles, 59 / 57 / 61; 1024x8, 385 tiles, 64 / 56 / 63; 75x297, 717 tiles, 69 / 69 /
+// 74; 121x481, 1937 tiles, 118 / 118 / 140).
+template <int NG>
+__global__ void __launch_bounds__(FLUX_FACES * NG, NG == 1 ? FLUX_MIN_BLOCKS : (NG == 2 ? 4 : 2)) k_flux(
+    const Inst* __restrict__ insts, const Tile* __restrict__ tx, int ntx, const Tile* __restrict__ ty, int stage,
+    int npx, int npy) {
     extern __shared__ __align__(16) unsigned char flux_mem[];
-    const Tile t = tiles[blockIdx.x];
+    const bool x = (int)blockIdx.x < ntx;
+    const Tile t = x ? tx[blockIdx.x] : ty[blockIdx.x - ntx];
     const Inst& I = insts[t.inst];
     if (has_error(I)) return;
-    flux_tile<DIR>(I, t, stage, flux_shared(flux_mem, npt));
+    if (x) flux_tile<0, NG>(I, t, stage, flux_shared(flux_mem, npx));
+    else flux_tile<1, NG>(I, t, stage, flux_shared(flux_mem, npy));
 }
 
 int flux_points(int dir, int lg) {
@@ -373,10 +410,19 @@ int flux_points(int dir, int lg) {
 
 void launch_flux(cudaStream_t s, const Inst* insts, const Tile* tx, int ntx, const Tile* ty, int nty, int stage,
                  const FluxSize& z) {
-    if (ntx > 0) k_flux<0><<<ntx, FLUX_THREADS, flux_smem(z.npx, z.diffusion), s>>>(insts, tx, stage, z.npx);
-    if (nty > 0) k_flux<1><<<nty, FLUX_THREADS, flux_smem(z.npy, z.diffusion), s>>>(insts, ty, stage, z.npy);
+    if (ntx + nty <= 0) return;
+    const int np = std::max(ntx > 0 ? z.npx : 0, nty > 0 ? z.npy : 0);
+    const int n = ntx + nty, smem = flux_smem(np, z.diffusion);
+    // (FMA build: one instantiation, since another might contract other sums, and
+    // an instance's result must not depend on what else the launch holds)
+    if (kExact && n <= FLUX_NG3)
+        k_flux<3><<<n, 3 * FLUX_FACES, smem, s>>>(insts, tx, ntx, ty, stage, z.npx, z.npy);
+    else if (kExact && n <= FLUX_NG2)
+        k_flux<2><<<n, 2 * FLUX_FACES, smem, s>>>(insts, tx, ntx, ty, stage, z.npx, z.npy);
+    else
+        k_flux<1><<<n, FLUX_FACES, smem, s>>>(insts, tx, ntx, ty, stage, z.npx, z.npy);
 }
 
-int flux_launches(int ntx, int nty) { return (ntx > 0 ? 1 : 0) + (nty > 0 ? 1 : 0); }
+int flux_launches(int ntx, int nty) { return ntx + nty > 0 ? 1 : 0; }
 
 } // namespace rh3t

@@ -17,7 +17,7 @@ struct FluxSize {
     bool diffusion;
 };
 int flux_points(int dir, int lg);
-// x faces, then y faces: flux_launches() kernels
+// x and y faces in one kernel: flux_launches()
 void launch_flux(cudaStream_t s, const Inst* insts, const Tile* tx, int ntx, const Tile* ty, int nty, int stage,
                  const FluxSize& z);
 int flux_launches(int ntx, int nty);

@@ -123,7 +123,6 @@ constexpr int GH_LR = 80;                        // per GhostBC slot and stage: 
 
 constexpr int CELL_TILE = 128;
 constexpr int FLUX_FACES = 64;                   // faces per flux block
-constexpr int FLUX_THREADS = 64;                 // one face per thread
 constexpr int ADJ_FLUX_THREADS = 192;            // face vjp: 6 warps, one per characteristic field
 constexpr int RHS_THREADS = 256;                 // cells per RHS block
 // admissible shapes (log2 of the j extent)

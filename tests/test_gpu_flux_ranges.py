@@ -67,3 +67,21 @@ def test_operator_bits(rh, O, name, shape):
     assert np.isfinite(rr[m]).all()
     assert np.array_equal(rhs[m], rr[m]), np.abs(rhs[m] - rr[m]).max(0)
     b.close()
+
+
+@pytest.mark.parametrize("nx", [128, 784, 800, 1576, 1592])
+def test_thread_groups(rh, O, nx):
+    """Strips with diffusion and exchange on whose flux launches have 49, 295,
+    301, 592 and 598 tiles: three, three, two, two and one thread group per tile.
+    As the planar shock's run: bitwise but for pow (1e-13)."""
+    from helpers import rel_linf
+    lx, ly = nx / 256.0, 8 / 256.0
+    p = dict(kappa_e=1e-3, kappa_i=1e-3, kappa_r=1e-3, omega_ei=1.0, omega_er=1.0, periodic_ly=ly)
+    f = rh.cases.planar_shock(nx, 8, lx, ly, x_shock=0.25, params=rh.Params(**p))
+    ref = O.Case.planar_shock(nx=nx, ny=8, lx=lx, ly=ly, x_shock=0.25, **p)
+    s = rh.Solver(f, rh.GhostGrid.build(f))
+    s.advance(3, 0.05)
+    ref.run(3, 0.05)
+    u, _ = s.download()
+    assert rel_linf(u, ref.state(), f.fluid).max() <= 1e-13
+    s.close()
