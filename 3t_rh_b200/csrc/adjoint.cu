@@ -42,13 +42,17 @@ using D8 = DualN<8>;
 // the adjoint needs derivatives, not the forward's roundings: constant
 // divisions become multiplications by reciprocals
 constexpr double K3 = 1.0 / 3.0, K6 = 1.0 / 6.0;
+// ... sums of products are fused (in both builds), and reciprocals are
+// recip_near's (within half an ulp, without a branch; divrn.cuh)
+__device__ __forceinline__ double mad(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ double inv(double x) { return recip_near(x).y; }
 
 // ---------------------------------------------------------------- pointwise vjps
 // state.rs:245-276 primitives: cotangents of (u, v, e_e, e_i, e_r, p_e, p_i,
 // p_r) -> state cotangent (added to sb)
 __device__ __forceinline__ void prim_vjp(const double s[6], const DevParams& P, double bu, double bv, double bee,
                                          double bei, double ber, double bpe, double bpi, double bpr, double sb[6]) {
-    const double rho = s[0], ir = 1.0 / rho, u = s[1] * ir, v = s[2] * ir;
+    const double rho = s[0], ir = inv(rho), u = s[1] * ir, v = s[2] * ir;
     const double w2 = u * u + v * v;
     const double ge = P.gamma_e - 1.0, gi = P.gamma_i - 1.0, gr = P.gamma_r - 1.0;
     const double gp = ge * bpe + gi * bpi + gr * bpr;
@@ -67,24 +71,25 @@ __device__ __forceinline__ void prim_vjp(const double s[6], const DevParams& P, 
 // state.rs:118-135 temperatures: cotangents of (te, ti, tr) -> sb
 __device__ __forceinline__ void temps_vjp(const double s[6], const DevParams& P, double bte, double bti, double btr,
                                           double sb[6]) {
-    const double rho = s[0], u = s[1] / rho, v = s[2] / rho;
+    const double rho = s[0], ir = inv(rho), u = s[1] * ir, v = s[2] * ir;
     const double w2 = u * u + v * v;
     double te, ti, tr;
     temps_from_state(s, P, te, ti, tr);
-    const double er_term = s[5] / rho - w2 / 6.0;
-    const double X = er_term * rho / P.a_rad;
-    const double bX = btr * 0.25 * tr / X;
+    const double ie = inv(P.cve), ii = inv(P.cvi), ia = inv(P.a_rad);
+    const double X = (s[5] * ir - w2 * K6) * rho * ia;
+    const double bX = btr * 0.25 * tr * inv(X);
     // te = E_e / (rho cve) - w2 / (6 cve), ti likewise, X = (E_r / rho - w2 / 6) rho / a
-    double brho = -s[3] * bte / (rho * rho * P.cve) - s[4] * bti / (rho * rho * P.cvi) - bX * (w2 / 6.0) / P.a_rad;
-    const double bw2 = -bte / (6.0 * P.cve) - bti / (6.0 * P.cvi) - bX * rho / (6.0 * P.a_rad);
+    const double be = bte * ie, bi = bti * ii, br = bX * ia;
+    double brho = -(s[3] * be + s[4] * bi) * ir * ir - br * (w2 * K6);
+    const double bw2 = -(be + bi + br * rho) * K6;
     const double bu = 2.0 * u * bw2, bv = 2.0 * v * bw2;
-    brho -= (bu * u + bv * v) / rho;
+    brho -= (bu * u + bv * v) * ir;
     sb[0] += brho;
-    sb[1] += bu / rho;
-    sb[2] += bv / rho;
-    sb[3] += bte / (rho * P.cve);
-    sb[4] += bti / (rho * P.cvi);
-    sb[5] += bX / P.a_rad;
+    sb[1] += bu * ir;
+    sb[2] += bv * ir;
+    sb[3] += be * ir;
+    sb[4] += bi * ir;
+    sb[5] += br;
 }
 
 // state.rs:56-85 physical flux: fb (6) -> sb
@@ -114,37 +119,35 @@ __device__ __forceinline__ void flux_vjp(const double s[6], const Prim& d, const
 // weno.rs:847-886 WENO5: cotangent gb of the result -> ub[5] (added); returns
 // the value itself (formed with the same intermediates)
 __device__ __forceinline__ double weno5_vjp(const double x[5], double eps, double gb, double ub[5]) {
-    const double t0 = x[0] - 2.0 * x[1] + x[2], r0 = x[0] - 4.0 * x[1] + 3.0 * x[2];
-    const double t1 = x[1] - 2.0 * x[2] + x[3], r1 = x[1] - x[3];
-    const double t2 = x[2] - 2.0 * x[3] + x[4], r2 = 3.0 * x[2] - 4.0 * x[3] + x[4];
+    const double x23 = 3.0 * x[2];
+    const double t0 = mad(-2.0, x[1], x[0]) + x[2], r0 = mad(-4.0, x[1], x[0]) + x23;
+    const double t1 = mad(-2.0, x[2], x[1]) + x[3], r1 = x[1] - x[3];
+    const double t2 = mad(-2.0, x[3], x[2]) + x[4], r2 = mad(-4.0, x[3], x23) + x[4];
     const double c1312 = 13.0 / 12.0;
-    const double e0 = 1.0 / (eps + (c1312 * t0 * t0 + 0.25 * r0 * r0));
-    const double e1 = 1.0 / (eps + (c1312 * t1 * t1 + 0.25 * r1 * r1));
-    const double e2 = 1.0 / (eps + (c1312 * t2 * t2 + 0.25 * r2 * r2));
+    const double q0 = 0.25 * r0, q1 = 0.25 * r1, q2 = 0.25 * r2;
+    const double e0 = inv(mad(q0, r0, mad(c1312 * t0, t0, eps)));
+    const double e1 = inv(mad(q1, r1, mad(c1312 * t1, t1, eps)));
+    const double e2 = inv(mad(q2, r2, mad(c1312 * t2, t2, eps)));
     const double a0 = 0.1 * e0 * e0, a1 = 0.6 * e1 * e1, a2 = 0.3 * e2 * e2;
-    const double iS = 1.0 / (a0 + a1 + a2);
+    const double iS = inv(a0 + a1 + a2);
     const double w0 = a0 * iS, w1 = a1 * iS, w2 = a2 * iS;
-    const double p0 = x[0] * K3 - 7.0 / 6.0 * x[1] + 11.0 / 6.0 * x[2];
-    const double p1 = -x[1] * K6 + 5.0 / 6.0 * x[2] + x[3] * K3;
-    const double p2 = x[2] * K3 + 5.0 / 6.0 * x[3] - x[4] * K6;
+    const double p0 = mad(x[0], K3, mad(11.0 / 6.0, x[2], -7.0 / 6.0 * x[1]));
+    const double p1 = mad(-K6, x[1], mad(5.0 / 6.0, x[2], x[3] * K3));
+    const double p2 = mad(x[2], K3, mad(5.0 / 6.0, x[3], -K6 * x[4]));
+    const double val = mad(w0, p0, mad(w1, p1, w2 * p2));
     const double pb0 = w0 * gb, pb1 = w1 * gb, pb2 = w2 * gb;
-    const double wb0 = p0 * gb, wb1 = p1 * gb, wb2 = p2 * gb;
-    const double m = w0 * wb0 + w1 * wb1 + w2 * wb2;
-    // alpha_k = d_k / (eps + b_k)^2, w_k = alpha_k / sum
-    const double bb0 = -2.0 * (wb0 - m) * iS * a0 * e0, bb1 = -2.0 * (wb1 - m) * iS * a1 * e1,
-                 bb2 = -2.0 * (wb2 - m) * iS * a2 * e2;
-    ub[0] += pb0 * K3;
-    ub[1] += -7.0 / 6.0 * pb0 - pb1 * K6;
-    ub[2] += 11.0 / 6.0 * pb0 + 5.0 / 6.0 * pb1 + pb2 * K3;
-    ub[3] += pb1 * K3 + 5.0 / 6.0 * pb2;
-    ub[4] += -pb2 * K6;
+    // alpha_k = d_k / (eps + b_k)^2, w_k = alpha_k / sum: b_k-bar = -2 (p_k - value) gb w_k e_k
+    const double g2 = -2.0 * gb;
+    const double bb0 = (p0 - val) * g2 * w0 * e0, bb1 = (p1 - val) * g2 * w1 * e1, bb2 = (p2 - val) * g2 * w2 * e2;
     const double c0 = 13.0 / 6.0 * t0 * bb0, d0 = 0.5 * r0 * bb0;
-    ub[0] += c0 + d0; ub[1] += -2.0 * c0 - 4.0 * d0; ub[2] += c0 + 3.0 * d0;
     const double c1 = 13.0 / 6.0 * t1 * bb1, d1 = 0.5 * r1 * bb1;
-    ub[1] += c1 + d1; ub[2] += -2.0 * c1; ub[3] += c1 - d1;
     const double c2 = 13.0 / 6.0 * t2 * bb2, d2 = 0.5 * r2 * bb2;
-    ub[2] += c2 + 3.0 * d2; ub[3] += -2.0 * c2 - 4.0 * d2; ub[4] += c2 + d2;
-    return w0 * p0 + w1 * p1 + w2 * p2;
+    ub[0] += mad(pb0, K3, c0 + d0);
+    ub[1] += mad(-7.0 / 6.0, pb0, mad(-K6, pb1, mad(-2.0, c0, mad(-4.0, d0, c1 + d1))));
+    ub[2] += mad(11.0 / 6.0, pb0, mad(5.0 / 6.0, pb1, mad(K3, pb2, mad(3.0, d0 + d2, mad(-2.0, c1, c0 + c2)))));
+    ub[3] += mad(K3, pb1, mad(5.0 / 6.0, pb2, mad(-2.0, c2, mad(-4.0, d2, c1 - d1))));
+    ub[4] += mad(-K6, pb2, c2 + d2);
+    return val;
 }
 
 // column c of R and lambda_c (weno.rs:518-545) with reciprocals
@@ -176,7 +179,7 @@ __device__ __forceinline__ void r_col_adj(int c, const Roe& q, const DevParams& 
     }
     const int k = DIR == 0 ? c - 1 : c - 2; // species 0 e, 1 i, 2 r
     const double gk = k == 0 ? ge : (k == 1 ? gi : gr);
-    const double sp = gt * w2 * K6 / gk;
+    const double sp = gt * w2 * K6 * inv(gk);
     R[0] = 1.0; R[1] = u; R[2] = v;
     if (k == 0) { R[3] = sp; R[4] = gr; R[5] = -gi; }
     else if (k == 1) { R[3] = -gr; R[4] = sp; R[5] = ge; }
@@ -209,7 +212,7 @@ __device__ __forceinline__ void roe_vjp(const double sa[6], const double sb_[6],
 __device__ __forceinline__ void roe_vjp_side(const double sa[6], const double sb_[6], const DevParams& P,
                                              const double bb[5], int side, double g[6]) {
     const Prim da = prim_from_state(sa, P), db = prim_from_state(sb_, P);
-    const double ra = sqrt(sa[0]), rb = sqrt(sb_[0]), irs = 1.0 / (ra + rb);
+    const double ra = sqrt(sa[0]), rb = sqrt(sb_[0]), irs = inv(ra + rb);
     const double xa[5] = {da.u, da.v, da.e_e, da.e_i, da.e_r}, xb[5] = {db.u, db.v, db.e_e, db.e_i, db.e_r};
     const double rs_self = side == 0 ? ra : rb;
     double br = 0.0, pp[5];
@@ -218,7 +221,7 @@ __device__ __forceinline__ void roe_vjp_side(const double sa[6], const double sb
         pp[k] = bb[k] * rs_self * irs;
         br += bb[k] * ((side == 0 ? xa[k] : xb[k]) - base) * irs;
     }
-    g[0] += br / (2.0 * rs_self);
+    g[0] = mad(br, 0.5 * inv(rs_self), g[0]);
     prim_vjp(side == 0 ? sa : sb_, P, pp[0], pp[1], pp[2], pp[3], pp[4], 0.0, 0.0, 0.0, g);
 }
 
@@ -262,7 +265,7 @@ __device__ __forceinline__ void r_base_vjp(const double base[5], const DevParams
         const int c = DIR == 0 ? 1 + k : 2 + k;
         bu += Rb[c][1];
         bv += Rb[c][2];
-        bw2 += gt * K6 / gk[k] * Rb[c][3 + k];
+        bw2 += gt * K6 * inv(gk[k]) * Rb[c][3 + k];
     }
     // eigenvalues: vel -+ cs, vel
     for (int c = 0; c < 6; ++c) bvel += lamb[c];
@@ -271,7 +274,7 @@ __device__ __forceinline__ void r_base_vjp(const double base[5], const DevParams
     else bv += bvel;
     bu += 2.0 * u * bw2;
     bv += 2.0 * v * bw2;
-    const double hc = 0.5 / cs;
+    const double hc = 0.5 * inv(cs);
     bb[0] += bu;
     bb[1] += bv;
     bb[2] += be[0] + GE * ge * hc * bcs;
@@ -318,7 +321,7 @@ __device__ __forceinline__ void r_base_vjp2(const double base[5], const DevParam
             const double gkk = k == 0 ? gk[0] : (k == 1 ? gk[1] : gk[2]);
             bu += r[1];
             bv += r[2];
-            bw2 += gt * K6 / gkk * rk;
+            bw2 += gt * K6 * inv(gkk) * rk;
         }
         bvel += lamb2[h];
     }
@@ -326,7 +329,7 @@ __device__ __forceinline__ void r_base_vjp2(const double base[5], const DevParam
     else bv += bvel;
     bu += 2.0 * u * bw2;
     bv += 2.0 * v * bw2;
-    const double hc = 0.5 / cs;
+    const double hc = 0.5 * inv(cs);
     bb[0] += bu;
     bb[1] += bv;
     bb[2] += be[0] + GE * ge * hc * bcs;
@@ -470,7 +473,7 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
         const Prim d2 = {PR[0][p2], PR[1][p2], PR[2][p2], PR[3][p2], PR[4][p2], PR[5][p2], PR[6][p2], PR[7][p2]};
         const Roe q = roe_average(S.U[0][p3].x, d3, S.U[0][p2].x, d2, P);
         const double qv[15] = {q.u,  q.v,  q.w2, q.ee, q.ei, q.er,  q.cs2,       q.cs,
-                               q.he, q.hi, q.hr, q.b,  q.den, 1.0 / q.cs2, 1.0 / q.b};
+                               q.he, q.hi, q.hr, q.b,  q.den, inv(q.cs2), inv(q.b)};
         for (int k = 0; k < 15; ++k) S.Q[k][f] = qv[k];
         for (int c = 0; c < 6; ++c) S.FB[c][f] = (RB[c][p3] - RB[c][p2]) * sc;
     }
@@ -492,15 +495,15 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
             double u[6], F[6];
             adj_point(S, p0 + k * ps, u, F);
             double cf = 0.0, cs = 0.0;
-            for (int m = 0; m < 6; ++m) { cf += Lc[m] * F[m]; cs += Lc[m] * u[m]; }
+            for (int m = 0; m < 6; ++m) { cf = mad(Lc[m], F[m], cf); cs = mad(Lc[m], u[m], cs); }
             w[k] = cs;
-            fp[k] = 0.5 * (cf + a * cs);
-            fm[k] = 0.5 * (cf - a * cs);
+            fp[k] = 0.5 * mad(a, cs, cf);
+            fm[k] = 0.5 * mad(-a, cs, cf);
         }
         // g_c = weno5(f+) + weno5(f-) and its cotangent gb = (R^T Fb)_c: both
         // reconstructions are reversed with the intermediates of their value
         double gb = 0.0;
-        for (int i2 = 0; i2 < 6; ++i2) gb += Rc[i2] * S.FB[i2][f];
+        for (int i2 = 0; i2 < 6; ++i2) gb = mad(Rc[i2], S.FB[i2][f], gb);
         double fpb[6] = {0, 0, 0, 0, 0, 0}, fmb[6] = {0, 0, 0, 0, 0, 0};
         double gval = weno5_vjp(fp, P.eps, gb, fpb);
         {
@@ -514,10 +517,10 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
         for (int k = 0; k < 6; ++k) {
             const double fbk = 0.5 * (fpb[k] + fmb[k]);
             const double wbk = 0.5 * a * (fpb[k] - fmb[k]);
-            ab += 0.5 * w[k] * (fpb[k] - fmb[k]);
+            ab = mad(0.5 * w[k], fpb[k] - fmb[k], ab);
             double u[6], F[6];
             adj_point(S, p0 + k * ps, u, F);
-            for (int m = 0; m < 6; ++m) Lb[m] += wbk * u[m] + fbk * F[m];
+            for (int m = 0; m < 6; ++m) Lb[m] = mad(wbk, u[m], mad(fbk, F[m], Lb[m]));
             S.WB[c][k][f] = wbk;
             S.FK[c][k][f] = fbk;
         }
@@ -552,8 +555,8 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
 #pragma unroll
                 for (int j = 0; j < 6; ++j) {
                     const double lb = S.LB[j][k][f];
-                    Z0[j] += lb * l0;
-                    Z1[j] += lb * l1;
+                    Z0[j] = mad(lb, l0, Z0[j]);
+                    Z1[j] = mad(lb, l1, Z1[j]);
                 }
             }
 #pragma unroll
@@ -562,8 +565,8 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
 #pragma unroll
                 for (int j = 0; j < 6; ++j) {
                     const double l = S.LS[j][i][f];
-                    a0 += l * Z0[j];
-                    a1 += l * Z1[j];
+                    a0 = mad(l, Z0[j], a0);
+                    a1 = mad(l, Z1[j], a1);
                 }
                 Rb2[0][i] -= a0;
                 Rb2[1][i] -= a1;
@@ -584,10 +587,10 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
 #pragma unroll
                 for (int m = 0; m < 6; ++m) {
                     const double l = S.LS[c2][m][f];
-                    V[0][m] += w0 * l;
-                    V[1][m] += w1 * l;
-                    VF[0][m] += q0 * l;
-                    VF[1][m] += q1 * l;
+                    V[0][m] = mad(w0, l, V[0][m]);
+                    V[1][m] = mad(w1, l, V[1][m]);
+                    VF[0][m] = mad(q0, l, VF[0][m]);
+                    VF[1][m] = mad(q1, l, VF[1][m]);
                 }
             }
         }
@@ -707,63 +710,68 @@ __global__ void __launch_bounds__(ADJ_FLUX_THREADS, 2) k_adj_flux(const Inst* __
 __device__ __forceinline__ void noncon9_vjp(const double pe[9], const double pi[9], const double pr[9],
                                             const double vel[9], double ds, const double ob[3], double pe_b[9],
                                             double pi_b[9], double pr_b[9], double vel_b[9]) {
-    const double v = vel[4];
-    const double dpe = d6(pe[1], pe[2], pe[3], pe[5], pe[6], pe[7], ds);
-    const double dpi = d6(pi[1], pi[2], pi[3], pi[5], pi[6], pi[7], ds);
-    const double dpr = d6(pr[1], pr[2], pr[3], pr[5], pr[6], pr[7], ds);
-    const double der[3] = {2.0 * dpe - dpi - dpr, 2.0 * dpi - dpe - dpr, 2.0 * dpr - dpe - dpi};
+    const double v = vel[4], ids = inv(ds), c6 = inv(60.0 * ds);
+    auto d6a = [&](const double* q) {
+        return (mad(-9.0, q[6], q[7]) + mad(45.0, q[5], mad(-45.0, q[3], mad(9.0, q[2], -q[1])))) * c6;
+    };
+    const double dpe = d6a(pe), dpi = d6a(pi), dpr = d6a(pr);
+    const double der[3] = {mad(2.0, dpe, -dpi) - dpr, mad(2.0, dpi, -dpe) - dpr, mad(2.0, dpr, -dpe) - dpi};
     double n[3][9];
     for (int k = 0; k < 9; ++k) {
-        n[0][k] = 2.0 * pe[k] - pi[k] - pr[k];
-        n[1][k] = 2.0 * pi[k] - pe[k] - pr[k];
-        n[2][k] = 2.0 * pr[k] - pe[k] - pi[k];
+        n[0][k] = mad(2.0, pe[k], -pi[k]) - pr[k];
+        n[1][k] = mad(2.0, pi[k], -pe[k]) - pr[k];
+        n[2][k] = mad(2.0, pr[k], -pe[k]) - pi[k];
     }
-    const double jm[3] = {jump8(n[0]), jump8(n[1]), jump8(n[2])};
-    const double jp[3] = {jump8(n[0] + 1), jump8(n[1] + 1), jump8(n[2] + 1)};
+    // jump8(a) = q(a7..a1) - q(a0..a6) = sum_k jc[k] a[k], q the 7-point pulse (noncon.rs:49-57)
+    constexpr double qc[7] = {-0.00714285714285723, 0.0595238095238118, -0.240476190476197, 0.759523809523819,
+                              0.509523809523803, -0.0904761904761891, 0.00952380952380977};
+    constexpr double jc[8] = {-qc[0], qc[6] - qc[1], qc[5] - qc[2], qc[4] - qc[3], qc[3] - qc[4], qc[2] - qc[5],
+                              qc[1] - qc[6], qc[0]};
+    double jm[3], jp[3];
+    for (int a = 0; a < 3; ++a) {
+        jm[a] = 0.0;
+        jp[a] = 0.0;
+        for (int k = 0; k < 8; ++k) {
+            jm[a] = mad(jc[k], n[a][k], jm[a]);
+            jp[a] = mad(jc[k], n[a][k + 1], jp[a]);
+        }
+    }
     const double xl = fmax(v, vel[3]), xr = fmin(v, vel[5]);
-    const double cl = fmax(xl, 0.0) / 3.0, cr = fmin(xr, 0.0) / 3.0;
+    const double cl = fmax(xl, 0.0) * K3, cr = fmin(xr, 0.0) * K3;
     for (int k = 0; k < 9; ++k) { pe_b[k] = 0.0; pi_b[k] = 0.0; pr_b[k] = 0.0; vel_b[k] = 0.0; }
     double clb = 0.0, crb = 0.0, derb[3], jmb[3], jpb[3];
     for (int a = 0; a < 3; ++a) {
-        vel_b[4] += ob[a] * der[a] / 3.0;
-        derb[a] = ob[a] * v / 3.0;
-        clb += ob[a] * jm[a] / ds;
-        crb += ob[a] * jp[a] / ds;
-        jmb[a] = ob[a] * cl / ds;
-        jpb[a] = ob[a] * cr / ds;
+        const double o3 = ob[a] * K3, od = ob[a] * ids;
+        vel_b[4] = mad(o3, der[a], vel_b[4]);
+        derb[a] = o3 * v;
+        clb = mad(od, jm[a], clb);
+        crb = mad(od, jp[a], crb);
+        jmb[a] = od * cl;
+        jpb[a] = od * cr;
     }
     if (xl >= 0.0) { // fmax(xl, 0) takes xl
-        if (v >= vel[3]) vel_b[4] += clb / 3.0;
-        else vel_b[3] += clb / 3.0;
+        if (v >= vel[3]) vel_b[4] += clb * K3;
+        else vel_b[3] += clb * K3;
     }
     if (xr <= 0.0) {
-        if (v <= vel[5]) vel_b[4] += crb / 3.0;
-        else vel_b[5] += crb / 3.0;
+        if (v <= vel[5]) vel_b[4] += crb * K3;
+        else vel_b[5] += crb * K3;
     }
-    // jump8(a) = q(a7..a1) - q(a0..a6) with q the 7-point pulse (noncon.rs:49-57)
-    const double qc[7] = {-0.00714285714285723, 0.0595238095238118, -0.240476190476197, 0.759523809523819,
-                          0.509523809523803, -0.0904761904761891, 0.00952380952380977};
     double nb[3][9];
     for (int a = 0; a < 3; ++a) {
-        for (int k = 0; k < 9; ++k) nb[a][k] = 0.0;
-        for (int w = 0; w < 2; ++w) {
-            const int o = w; // window start
-            const double jb = w == 0 ? jmb[a] : jpb[a];
-            for (int t = 0; t < 7; ++t) {
-                nb[a][o + 7 - t] += qc[t] * jb; // q(a7, a6, ..., a1)
-                nb[a][o + t] -= qc[t] * jb;     // q(a0, ..., a6)
-            }
-        }
+        nb[a][0] = jc[0] * jmb[a];
+        for (int k = 1; k < 8; ++k) nb[a][k] = mad(jc[k], jmb[a], jc[k - 1] * jpb[a]);
+        nb[a][8] = jc[7] * jpb[a];
     }
     // der = M dp with M symmetric [[2,-1,-1],[-1,2,-1],[-1,-1,2]]
     const double dpb[3] = {2.0 * derb[0] - derb[1] - derb[2], 2.0 * derb[1] - derb[0] - derb[2],
                            2.0 * derb[2] - derb[0] - derb[1]};
-    const double c6 = 1.0 / (60.0 * ds);
     const double w6[7] = {-1.0, 9.0, -45.0, 0.0, 45.0, -9.0, 1.0}; // points 1..7
     for (int t = 0; t < 7; ++t) {
-        pe_b[1 + t] += w6[t] * c6 * dpb[0];
-        pi_b[1 + t] += w6[t] * c6 * dpb[1];
-        pr_b[1 + t] += w6[t] * c6 * dpb[2];
+        if (t == 3) continue;
+        pe_b[1 + t] = w6[t] * (c6 * dpb[0]);
+        pi_b[1 + t] = w6[t] * (c6 * dpb[1]);
+        pr_b[1 + t] = w6[t] * (c6 * dpb[2]);
     }
     for (int k = 0; k < 9; ++k) {
         pe_b[k] += 2.0 * nb[0][k] - nb[1][k] - nb[2][k];
