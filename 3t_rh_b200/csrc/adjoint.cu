@@ -367,7 +367,7 @@ __device__ __forceinline__ void atomic_add6(double* W, long long plane, long lon
 // warps:
 //   1. staging: point states and physical fluxes of the tile, each face's Roe
 //      state and flux cotangent Fb (from rbar);
-//   2. warp c = characteristic field c, faces lane and lane + 32: the forward
+//   2. three threads per face, two characteristic fields c each: the forward
 //      reconstruction of field c, then its reverse: w-bar and f-bar of the six
 //      points, L-bar of row c, lambda-bar; L row c and g_c kept for step 3;
 //   3a. three threads per face: L-bar folded into R-bar (L = R^-1), the Roe
@@ -393,6 +393,7 @@ struct AdjFluxShared {
     double FK[6][6][AFP];  // f-bar [c][k]
     int act[FLUX_FACES];
 };
+static_assert(ADJ_FLUX_THREADS == 3 * FLUX_FACES, "three threads per face in steps 2 and 3a");
 static_assert(14 * FLUX_NPT + FLUX_NPT / 8 + 1 <= 36 * AFP, "step-1 staging fits in LS");
 
 template <int DIR>
@@ -478,54 +479,91 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
         for (int c = 0; c < 6; ++c) S.FB[c][f] = (RB[c][p3] - RB[c][p2]) * sc;
     }
     __syncthreads();
-    // ---- 2. warp c: field c of faces lane and lane + 32
-    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int h = 0; h < FLUX_FACES / 32; ++h) {
-        const int f = lane + 32 * h;
-        if (!S.act[f]) continue;
-        int i, j, p0, ps;
-        adj_face_index<DIR>(t, f, i, j, p0, ps);
-        const Roe q = adj_load_q(S, f);
-        double Lc[6], Rc[6], lam;
-        fastm::l_row<DIR>(c, q, S.Q[13][f], S.Q[14][f], P, Lc);
-        r_col_adj<DIR>(c, q, P, Rc, lam);
-        const double a = fabs(lam);
-        double w[6], fp[6], fm[6];
-        for (int k = 0; k < 6; ++k) {
-            double u[6], F[6];
-            adj_point(S, p0 + k * ps, u, F);
-            double cf = 0.0, cs = 0.0;
-            for (int m = 0; m < 6; ++m) { cf = mad(Lc[m], F[m], cf); cs = mad(Lc[m], u[m], cs); }
-            w[k] = cs;
-            fp[k] = 0.5 * mad(a, cs, cf);
-            fm[k] = 0.5 * mad(-a, cs, cf);
+    // ---- 2. two fields of one face per thread, so that a point's data are
+    // loaded once for both (x faces: 0 and 5, 1 and 2, 3 and 4; y faces 0 and 5,
+    // 2 and 3, 4 and 1)
+    {
+        const int f = threadIdx.x & (FLUX_FACES - 1), g = threadIdx.x / FLUX_FACES; // g warp-uniform
+        if (S.act[f]) {
+            const int cc[2] = {DIR == 0 ? (g == 0 ? 0 : 2 * g - 1) : (g == 0 ? 0 : 2 * g),
+                               g == 0 ? 5 : (DIR == 0 ? 2 * g : (g == 1 ? 3 : 1))};
+            int i, j, p0, ps;
+            adj_face_index<DIR>(t, f, i, j, p0, ps);
+            double Lc[2][6], lam[2], gb[2], fp[2][6], fm[2][6], w[2][6];
+            {
+                const Roe q = adj_load_q(S, f);
+                double FB[6];
+#pragma unroll
+                for (int m = 0; m < 6; ++m) FB[m] = S.FB[m][f];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    double Rc[6];
+                    fastm::l_row<DIR>(cc[e], q, S.Q[13][f], S.Q[14][f], P, Lc[e]);
+                    r_col_adj<DIR>(cc[e], q, P, Rc, lam[e]);
+                    gb[e] = 0.0; // the cotangent of g_c, (R^T Fb)_c
+#pragma unroll
+                    for (int m = 0; m < 6; ++m) gb[e] = mad(Rc[m], FB[m], gb[e]);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                double u[6], F[6];
+                adj_point(S, p0 + k * ps, u, F);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const double a = fabs(lam[e]);
+                    double cf = 0.0, cs = 0.0;
+#pragma unroll
+                    for (int m = 0; m < 6; ++m) { cf = mad(Lc[e][m], F[m], cf); cs = mad(Lc[e][m], u[m], cs); }
+                    w[e][k] = cs;
+                    fp[e][k] = 0.5 * mad(a, cs, cf);
+                    fm[e][k] = 0.5 * mad(-a, cs, cf);
+                }
+            }
+            // g_c = weno5(f+) + weno5(f-): both reconstructions are reversed
+            // with the intermediates of their value
+            double wb[2][6], fb[2][6], Lb[2][6];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = cc[e];
+                const double a = fabs(lam[e]);
+                double fpb[6] = {0, 0, 0, 0, 0, 0}, ubm[5] = {0, 0, 0, 0, 0};
+                double gval = weno5_vjp(fp[e], P.eps, gb[e], fpb);
+                const double xm[5] = {fm[e][5], fm[e][4], fm[e][3], fm[e][2], fm[e][1]};
+                gval += weno5_vjp(xm, P.eps, gb[e], ubm);
+                S.G[c][f] = gval;
+                double ab = 0.0;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    const double fmb = k == 0 ? 0.0 : ubm[5 - k];
+                    const double d = fpb[k] - fmb;
+                    fb[e][k] = 0.5 * (fpb[k] + fmb);
+                    wb[e][k] = 0.5 * a * d;
+                    ab = mad(0.5 * w[e][k], d, ab);
+                    S.WB[c][k][f] = wb[e][k];
+                    S.FK[c][k][f] = fb[e][k];
+                }
+                S.LAMB[c][f] = lam[e] < 0.0 ? -ab : ab;
+#pragma unroll
+                for (int m = 0; m < 6; ++m) {
+                    S.LS[c][m][f] = Lc[e][m];
+                    Lb[e][m] = 0.0;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                double u[6], F[6];
+                adj_point(S, p0 + k * ps, u, F);
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int m = 0; m < 6; ++m) Lb[e][m] = mad(wb[e][k], u[m], mad(fb[e][k], F[m], Lb[e][m]));
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int m = 0; m < 6; ++m) S.LB[cc[e]][m][f] = Lb[e][m];
         }
-        // g_c = weno5(f+) + weno5(f-) and its cotangent gb = (R^T Fb)_c: both
-        // reconstructions are reversed with the intermediates of their value
-        double gb = 0.0;
-        for (int i2 = 0; i2 < 6; ++i2) gb = mad(Rc[i2], S.FB[i2][f], gb);
-        double fpb[6] = {0, 0, 0, 0, 0, 0}, fmb[6] = {0, 0, 0, 0, 0, 0};
-        double gval = weno5_vjp(fp, P.eps, gb, fpb);
-        {
-            const double xm[5] = {fm[5], fm[4], fm[3], fm[2], fm[1]};
-            double ubm[5] = {0, 0, 0, 0, 0};
-            gval += weno5_vjp(xm, P.eps, gb, ubm);
-            fmb[5] += ubm[0]; fmb[4] += ubm[1]; fmb[3] += ubm[2]; fmb[2] += ubm[3]; fmb[1] += ubm[4];
-        }
-        S.G[c][f] = gval;
-        double ab = 0.0, Lb[6] = {0, 0, 0, 0, 0, 0};
-        for (int k = 0; k < 6; ++k) {
-            const double fbk = 0.5 * (fpb[k] + fmb[k]);
-            const double wbk = 0.5 * a * (fpb[k] - fmb[k]);
-            ab = mad(0.5 * w[k], fpb[k] - fmb[k], ab);
-            double u[6], F[6];
-            adj_point(S, p0 + k * ps, u, F);
-            for (int m = 0; m < 6; ++m) Lb[m] = mad(wbk, u[m], mad(fbk, F[m], Lb[m]));
-            S.WB[c][k][f] = wbk;
-            S.FK[c][k][f] = fbk;
-        }
-        for (int m = 0; m < 6; ++m) { S.LS[c][m][f] = Lc[m]; S.LB[c][m][f] = Lb[m]; }
-        S.LAMB[c][f] = lam < 0.0 ? -ab : ab;
     }
     __syncthreads();
     // ---- 3a. per face, three threads (two columns of R each): L-bar folded

@@ -123,7 +123,7 @@ constexpr int GH_LR = 80;                        // per GhostBC slot and stage: 
 
 constexpr int CELL_TILE = 128;
 constexpr int FLUX_FACES = 64;                   // faces per flux block
-constexpr int ADJ_FLUX_THREADS = 192;            // face vjp: 6 warps, one per characteristic field
+constexpr int ADJ_FLUX_THREADS = 192;            // face vjp: three threads per face
 constexpr int RHS_THREADS = 256;                 // cells per RHS block
 // admissible shapes (log2 of the j extent)
 constexpr int FX_LG_MIN = 2, FX_LG_MAX = 4;      // x faces 16x4, 8x8, 4x16
