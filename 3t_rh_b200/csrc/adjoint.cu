@@ -957,9 +957,9 @@ __constant__ int kAWOff[6] = {0, 1, 9, 36, 100, 225};
 
 struct AdjGhostWarp {
     double L[36], R[36], lam[6];             // L[6c + j]; R column c at R[6c + i]
-    double U6[6][56];                        // rotated stencil states
+    double U6[6][57];                        // rotated stencil states (odd rows: six rows' entries in different banks)
     double D[56][6];                         // d_c of stencil node a at row d_row(a)
-    double ACC[6][56], STD[6][56];           // ACC: S d; STD: D-bar
+    double ACC[6][57];                       // S d, then D-bar
     double alpha[6][5], beta[6][5], V[6][5][5];
     double v[5][6], x[5][6], ub[5][6], xb[5][6], vinf[6], vinfb[6];
     double Lb[6][6], Rb[6][6];
@@ -969,7 +969,7 @@ struct AdjGhostWarp {
     double w[226];    // w_{r,k}, term b at kAWOff[r] + k m + b (kept from the dot products)
 };
 static_assert(sizeof(AdjGhostWarp) % 16 == 0, "rows of D stay 16-byte aligned");
-constexpr int AG_SMEM = AG_WARPS * (int)sizeof(AdjGhostWarp); // four blocks per SM
+constexpr int AG_SMEM = AG_WARPS * (int)sizeof(AdjGhostWarp); // five blocks per SM
 
 __device__ __forceinline__ int aorder(int a) { return a < 1 ? 0 : (a < 5 ? 1 : (a < 14 ? 2 : (a < 30 ? 3 : 4))); }
 
@@ -1234,6 +1234,12 @@ __device__ __forceinline__ void adj_dot_pair(AdjGhostWarp& G, const double* __re
     }
 }
 
+// alpha / asum, is = inv(asum): the alphas (eps + beta)^-10 can lie near the
+// ends of the exponent range
+__device__ __forceinline__ double weight_of(double alpha, double asum, double is) {
+    return den_near(asum) ? alpha * is : div_ieee(alpha, asum);
+}
+
 // L2 prefetch of a ghost's record by the bulk-copy engine (16-byte aligned,
 // size a multiple of 16; nothing waits on it)
 __device__ __forceinline__ void prefetch_record_l2(const double* rec) {
@@ -1308,7 +1314,7 @@ __device__ void ghost_vjp_warp(const Inst& I, const GhostRec& Rg, const double* 
         double xq;
         if (P.weno_q == 10.0) { const double x2 = x * x, x4 = x2 * x2, x8 = x4 * x4; xq = x8 * x2; }
         else xq = pow(x, P.weno_q);
-        G.alpha[c][r] = rec[GH_D + r] / xq;
+        G.alpha[c][r] = rec[GH_D + r] / xq; // (an overflowing xq gives 0)
         for (int k = r + 1; k < 5; ++k) G.V[c][r][k] = 0.0;
     }
     __syncwarp();
@@ -1316,8 +1322,9 @@ __device__ void ghost_vjp_warp(const Inst& I, const GhostRec& Rg, const double* 
         const int k = lane / 6, c = lane - 6 * (lane / 6);
         double asum = 0.0;
         for (int r = 0; r < 5; ++r) asum += G.alpha[c][r];
+        const double is = inv(asum);
         double res = 0.0;
-        for (int r = 0; r < 5; ++r) res += (G.alpha[c][r] / asum) * G.V[c][r][k];
+        for (int r = 0; r < 5; ++r) res = mad(weight_of(G.alpha[c][r], asum, is), G.V[c][r][k], res);
         G.v[k][c] = res;
     }
     __syncwarp();
@@ -1400,17 +1407,17 @@ __device__ void ghost_vjp_warp(const Inst& I, const GhostRec& Rg, const double* 
     double asum = 0.0, om = 0.0, omb = 0.0;
     if (lane < 30) {
         for (int r = 0; r < 5; ++r) asum += G.alpha[oc][r];
-        om = G.alpha[oc][orr] / asum;
-        for (int k = 0; k < 5; ++k) omb += G.V[oc][orr][k] * G.vb[k][oc];
+        const double is = inv(asum);
+        om = weight_of(G.alpha[oc][orr], asum, is);
+        for (int k = 0; k < 5; ++k) omb = mad(G.V[oc][orr][k], G.vb[k][oc], omb);
         G.omm[oc][orr] = om * omb;
     }
     __syncwarp();
     if (lane < 30) {
         double m = 0.0;
         for (int r = 0; r < 5; ++r) m += G.omm[oc][r];
-        const double ab = (omb - m) / asum;
-        // alpha = d (eps + beta)^-q
-        G.beta[oc][orr] = -P.weno_q * ab * G.alpha[oc][orr] / (P.eps + G.beta[oc][orr]); // now beta-bar
+        // alpha = d (eps + beta)^-q, alpha-bar = (omb - m) / asum
+        G.beta[oc][orr] = -P.weno_q * (omb - m) * om * inv(P.eps + G.beta[oc][orr]); // now beta-bar
         for (int k = 0; k < 5; ++k) G.V[oc][orr][k] = om * G.vb[k][oc];                 // now V-bar
     }
     __syncwarp();
@@ -1426,31 +1433,38 @@ __device__ void ghost_vjp_warp(const Inst& I, const GhostRec& Rg, const double* 
         }
         for (int c = 0; c < 6; ++c) {
             double acc = G.beta[c][r0] * (2.0 * G.ACC[c][lane]);
-            for (int k = 0; k <= r0; ++k) acc += G.V[c][r0][k] * wv0[k];
-            G.STD[c][lane] = acc; // D-bar
+            for (int k = 0; k <= r0; ++k) acc = mad(G.V[c][r0][k], wv0[k], acc);
+            G.ACC[c][lane] = acc; // D-bar
         }
         if (lane + 32 < 55) {
             for (int c = 0; c < 6; ++c) {
                 double acc = G.beta[c][4] * (2.0 * G.ACC[c][lane + 32]);
 #pragma unroll
-                for (int k = 0; k < 5; ++k) acc += G.V[c][4][k] * wv1[k];
-                G.STD[c][lane + 32] = acc;
+                for (int k = 0; k < 5; ++k) acc = mad(G.V[c][4][k], wv1[k], acc);
+                G.ACC[c][lane + 32] = acc;
             }
         }
     }
     __syncwarp();
-    // D = L rot(u_a): Lb += DB rot(u_a)^T (18 lanes, entries (c, q) and (c, q + 1)),
-    // rot(u_a)-bar = L^T DB
-    if (lane < 18) {
-        const int c = lane / 3, q = 2 * (lane - 3 * (lane / 3));
-        double acc0 = 0.0, acc1 = 0.0;
-        for (int a = 0; a < 55; ++a) {
-            const double sd = G.STD[c][a];
-            acc0 += sd * G.U6[q][a];
-            acc1 += sd * G.U6[q + 1][a];
+    // D = L rot(u_a): Lb += DB rot(u_a)^T (three entries a lane, half of the nodes
+    // each), rot(u_a)-bar = L^T DB
+    {
+        const int t = lane % 12, h = lane / 12, c = t >> 1, q = 3 * (t & 1); // entries (c, q..q+2), nodes of half h
+        double acc[3] = {0.0, 0.0, 0.0};
+        if (h < 2) {
+            const int a1 = h == 0 ? 28 : 55;
+#pragma unroll 4
+            for (int a = 28 * h; a < a1; ++a) {
+                const double sd = G.ACC[c][a];
+#pragma unroll
+                for (int e = 0; e < 3; ++e) acc[e] = mad(sd, G.U6[q + e][a], acc[e]);
+            }
         }
-        G.Lb[c][q] += acc0;
-        G.Lb[c][q + 1] += acc1;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const double o = __shfl_down_sync(0xffffffffu, acc[e], 12);
+            if (h == 0) G.Lb[c][q + e] += acc[e] + o;
+        }
     }
     {
         // both of a lane's nodes per row of L (one read of L)
@@ -1458,12 +1472,12 @@ __device__ void ghost_vjp_warp(const Inst& I, const GhostRec& Rg, const double* 
         double ur0[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, ur1[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-            const double d0 = G.STD[c][lane], d1 = two ? G.STD[c][lane + 32] : 0.0;
+            const double d0 = G.ACC[c][lane], d1 = two ? G.ACC[c][lane + 32] : 0.0;
 #pragma unroll
             for (int q = 0; q < 6; ++q) {
                 const double l = L[6 * c + q];
-                ur0[q] += l * d0;
-                ur1[q] += l * d1;
+                ur0[q] = mad(l, d0, ur0[q]);
+                ur1[q] = mad(l, d1, ur1[q]);
             }
         }
         const double sb0[6] = {ur0[0], ur0[1] * nx - ur0[2] * ny, ur0[1] * ny + ur0[2] * nx, ur0[3], ur0[4], ur0[5]};
