@@ -463,7 +463,7 @@ class Solver(_SnapshotIO):
         self._check(self.L.rh3t_upload_state(self.h, v.ctypes.data, field.time))
 
     def download(self, field=None):
-        out = np.zeros((self.grid.len(), 6))
+        out = np.empty((self.grid.len(), 6))
         t = C.c_double()
         self._check(self.L.rh3t_download_state(self.h, out.ctypes.data, C.byref(t)))
         if field is not None:
@@ -473,8 +473,8 @@ class Solver(_SnapshotIO):
         return out, t.value
 
     def l(self, with_ghosts=False):
-        rhs = np.zeros((self.grid.len(), 6))
-        gv = np.zeros((self.n_ghosts, 6)) if with_ghosts else None
+        rhs = np.empty((self.grid.len(), 6))
+        gv = np.empty((self.n_ghosts, 6)) if with_ghosts else None
         self._check(self.L.rh3t_l(self.h, rhs.ctypes.data, _ptr(gv)))
         return (rhs, gv) if with_ghosts else rhs
 
@@ -597,7 +597,7 @@ class Batch(_SnapshotIO):
         (float64, C-contiguous, e.g. pinned host memory) receive the copy
         when given."""
         if out is None:
-            out = np.zeros((int(self.offsets[-1]), 6))
+            out = np.empty((int(self.offsets[-1]), 6))
         elif out.dtype != np.float64 or not out.flags.c_contiguous or out.size != int(self.offsets[-1]) * 6:
             raise ValueError("out must be a C-contiguous float64 array of total_cells x 6")
         t = np.zeros(self.n) if times is None else times
@@ -607,7 +607,7 @@ class Batch(_SnapshotIO):
     def download(self, k=None):
         """[(value, time)] per instance, or one instance's (value, time)."""
         if k is not None:
-            out = np.zeros((int(self.cells[k]), 6))
+            out = np.empty((int(self.cells[k]), 6))
             t = C.c_double()
             self._check(self.L.rh3t_download_instance(self.h, int(k), out.ctypes.data, C.byref(t)))
             return out, t.value
@@ -615,8 +615,8 @@ class Batch(_SnapshotIO):
         return [(v[self.offsets[k]:self.offsets[k + 1]], float(t[k])) for k in range(self.n)]
 
     def l(self, k, with_ghosts=False):
-        rhs = np.zeros((int(self.cells[k]), 6))
-        gv = np.zeros((self.n_ghosts[k], 6)) if with_ghosts else None
+        rhs = np.empty((int(self.cells[k]), 6))
+        gv = np.empty((self.n_ghosts[k], 6)) if with_ghosts else None
         self._check(self.L.rh3t_l_instance(self.h, int(k), rhs.ctypes.data, _ptr(gv)))
         return (rhs, gv) if with_ghosts else rhs
 
@@ -677,7 +677,7 @@ class Batch(_SnapshotIO):
         its l() (nx*ny x 6); returns (ubar, pbar) with pbar = (FarField state
         (6), omega_ei, omega_er)."""
         rb = _arr(rbar, np.float64)
-        ub = np.zeros((int(self.cells[k]), 6))
+        ub = np.empty((int(self.cells[k]), 6))
         pb = np.zeros(8)
         self._check(self.L.rh3t_l_vjp(self.h, int(k), rb.ctypes.data, ub.ctypes.data, pb.ctypes.data))
         return ub, pb
@@ -704,7 +704,7 @@ class Batch(_SnapshotIO):
             dJ_du = np.concatenate([_arr(x, np.float64).reshape(-1, 6) for x in dJ_du])
         lam = _arr(dJ_du, np.float64)
         if out is None:
-            g0 = np.zeros((int(self.offsets[-1]), 6))
+            g0 = np.empty((int(self.offsets[-1]), 6))
         elif out.dtype != np.float64 or not out.flags.c_contiguous or out.size != int(self.offsets[-1]) * 6:
             raise ValueError("out must be a C-contiguous float64 array of total_cells x 6")
         else:
