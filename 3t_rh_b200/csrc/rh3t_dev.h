@@ -130,8 +130,9 @@ constexpr int FX_LG_MIN = 2, FX_LG_MAX = 4;      // x faces 16x4, 8x8, 4x16
 constexpr int FY_LG_MIN = 4, FY_LG_MAX = 6;      // y faces 4x16, 2x32, 1x64
 constexpr int RHS_LG_MIN = 4, RHS_LG_MAX = 6;    // cells 16x16, 8x32, 4x64
 // defaults: y faces 4x16 (61x241 instances: 26.2 us a launch against 30.7 us at
-// 1x64, 121x481: 123 against 130 us), x faces 8x8, cells 8x32
-constexpr int FX_LG_DEF = 3, FY_LG_DEF = 4, RHS_LG_DEF = 5;
+// 1x64, 121x481: 123 against 130 us), x faces 8x8, cells
+// 16x16 (961x3841: 288 us a launch against 299 us at 8x32, 402 us at 4x64)
+constexpr int FX_LG_DEF = 3, FY_LG_DEF = 4, RHS_LG_DEF = 4;
 // staged points per flux block: max over shapes of (TI + 5) * TJ (x) and
 // TI * (TJ + 5) (y)
 constexpr int FLUX_NPT = 144;

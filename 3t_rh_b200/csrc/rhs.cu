@@ -8,17 +8,22 @@
 //      2 p_k - p_l - p_m of the nodes within reach of the 9-point non-conservative
 //      stencils (the tile plus a 4-node halo, corners excluded) go to shared
 //      memory once; the reference's access-table gathers (main.rs:276-277)
-//      evaluate them once per use, 17 times per node;
+//      evaluate them once per use, 17 times per node. A 16 x 16 tile has 512 such
+//      nodes, two a thread, and a thread loads both before it uses either;
 //   2. the jumps of the three differences at every interface of the tile: the
 //      reference forms those at a cell's left and right (lower and upper)
-//      interface in each of the two cells they belong to (noncon.rs:259-285);
+//      interface in each of the two cells they belong to (noncon.rs:259-285). The
+//      tile's far edges go one difference to a thread, three to seven warps, instead of
+//      three to each thread of the two warps that the others then wait for;
 //   3. one cell per thread.
 // Bound by latency (24 face fluxes and the stage inputs a cell) and the FP64
 // pipe. Forming a jump once, and quotients without a branch each (divrn.cuh), take
 // away a third of the FP64 operations and the registers that held two 9-point
-// windows, so three blocks fit an SM instead of two: 24 batch instances 107 us a
-// stage instead of 153 us, the 961 x 3841 half-cylinder 318 us instead of 453 us
-// (two blocks of 119 registers: 399 us, four of 64, spills: 369 us).
+// windows, so three blocks fit an SM instead of two. Per stage, 24 batch instances
+// 98 us (both windows a cell: 153 us; node loop over the whole halo and far edges on
+// two warps: 105 us), the 961 x 3841 half-cylinder 288 us (453 us; 312 us). Two blocks
+// of 119 registers were 25% slower, four of 64 (spills) 16%; the face fluxes
+// loaded ahead of phases 1 or 2, or prefetched to L2, gave nothing.
 //
 // mode 0 writes the rhs (6 planes of nx*ny, i*ny+j, instance k at
 // rhs_out + 6*cell_off) for l(); mode 1 applies the stage update of `stage`;
@@ -38,6 +43,7 @@ constexpr bool kExactR = true;
 constexpr bool kExactR = false;
 #endif
 constexpr int RHS_BLOCKS = 3; // per SM: 80 registers
+static_assert(RHS_THREADS == 1 << 8, "log2 TI = 8 - lg");
 
 // divisors shared by every cell of an instance: 60 dx, dx, 60 dy, dy
 // (noncon.rs:26-44, 315-331), 6 cve, 6 cvi, a_rad (state.rs:245-276)
@@ -101,28 +107,46 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_BLOCKS) k_rhs_stage(const Ins
         sR[RHS_NR + threadIdx.x] = r.yl;
     }
     // ---- 1. stage node primitives (tile + 4-node cross halo)
-    for (int p = threadIdx.x; p < NPT; p += RHS_THREADS) {
-        const int hi = p / HJ, hj = p - hi * HJ;
-        const bool corner = (hi < 4 || hi >= TI + 4) && (hj < 4 || hj >= TJ + 4);
+    const int mid = (TI + 8) << t.lg, nodes = mid + 8 * TI;
+    auto place = [&](int q, int& hi, int& hj) {
+        const int r = q - mid;
+        hi = r < 0 ? q >> t.lg : 4 + (r >> 3);
+        hj = r < 0 ? 4 + (q & (TJ - 1)) : (r & 7) + (r & 4 ? TJ : 0);
         const int i = t.i - 4 + hi, j = t.j0 - 4 + hj;
-        if (corner || i < -RH3T_PAD || i >= nx + RH3T_PAD || j < -RH3T_PAD || j >= ny + RH3T_PAD) continue;
-        double s[6];
-        load6(src, plane, node_of(I, i, j), s);
-        Prim d = kExactR ? prim_from_state(s, P) : fastm::prim(s, P);
+        return q < nodes && i >= -RH3T_PAD && i < nx + RH3T_PAD && j >= -RH3T_PAD && j < ny + RH3T_PAD;
+    };
+    auto put = [&](int p, const double* s) {
+        const Prim d = kExactR ? prim_from_state(s, P) : fastm::prim(s, P);
         sP[p] = d.pe; sP[NPT + p] = d.pi; sP[2 * NPT + p] = d.pr; sP[3 * NPT + p] = d.u; sP[4 * NPT + p] = d.v;
         sN[p] = 2.0 * d.pe - d.pi - d.pr;
         sN[NPT + p] = 2.0 * d.pi - d.pe - d.pr;
         sN[2 * NPT + p] = 2.0 * d.pr - d.pe - d.pi;
+    };
+    for (int q = threadIdx.x; q < nodes; q += 2 * RHS_THREADS) {
+        int h0, j0, h1, j1;
+        const bool a = place(q, h0, j0), b = place(q + RHS_THREADS, h1, j1);
+        double s[6], z[6];
+        if (a) load6(src, plane, node_of(I, t.i - 4 + h0, t.j0 - 4 + j0), s);
+        if (b) load6(src, plane, node_of(I, t.i - 4 + h1, t.j0 - 4 + j1), z);
+        if (a) put(h0 * HJ + j0, s);
+        if (b) put(h1 * HJ + j1, z);
     }
     __syncthreads();
     const int ti = threadIdx.x >> t.lg, tj = threadIdx.x & (TJ - 1);
     // ---- 2. jumps: this cell's left and lower interfaces, then the tile's far edges
     jumps(sN, NPT, ti * HJ + tj + 4, HJ, sX + threadIdx.x, nfx);
     jumps(sN, NPT, (ti + 4) * HJ + tj, 1, sY + ti * (TJ + 1) + tj, nfy);
-    if (threadIdx.x < TJ)
-        jumps(sN, NPT, TI * HJ + threadIdx.x + 4, HJ, sX + TI * TJ + threadIdx.x, nfx);
-    else if (threadIdx.x < TJ + TI)
-        jumps(sN, NPT, (threadIdx.x - TJ + 4) * HJ + TJ, 1, sY + (threadIdx.x - TJ) * (TJ + 1) + TJ, nfy);
+    if (threadIdx.x < 3 * (TJ + TI)) {
+        const int e = threadIdx.x - 3 * TJ;
+        const bool x = e < 0;
+        const int lg = x ? t.lg : 8 - t.lg, q = x ? threadIdx.x : e, c = q >> lg, k = q & ((1 << lg) - 1);
+        const double* a = sN + c * NPT + (x ? TI * HJ + k + 4 : (k + 4) * HJ + TJ);
+        const int st = x ? HJ : 1;
+        double w[8];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) w[m] = a[m * st];
+        *(x ? sX + c * nfx + TI * TJ + k : sY + c * nfy + k * (TJ + 1) + TJ) = jump8(w);
+    }
     __syncthreads();
     // ---- 3. this thread's cell
     const int i = t.i + ti, j = t.j0 + tj;
