@@ -282,10 +282,10 @@ __device__ __forceinline__ void r_base_vjp(const double base[5], const DevParams
     bb[4] += be[2] + GR * gr * hc * bcs;
 }
 
-// r_base_vjp for the two columns c0, c0 + 1 of R-bar (the other columns
+// r_base_vjp for the two columns cc[0], cc[1] of R-bar (the other columns
 // zero): the part of the Roe base cotangent they carry, added to bb
 template <int DIR>
-__device__ __forceinline__ void r_base_vjp2(const double base[5], const DevParams& P, int c0, const double Rb2[2][6],
+__device__ __forceinline__ void r_base_vjp2(const double base[5], const DevParams& P, const int cc[2], const double Rb2[2][6],
                                             const double lamb2[2], double bb[5]) {
     const double GE = P.gamma_e, GI = P.gamma_i, GR = P.gamma_r;
     const double gi = GI - 1.0, ge = GE - 1.0, gr = GR - 1.0;
@@ -297,7 +297,7 @@ __device__ __forceinline__ void r_base_vjp2(const double base[5], const DevParam
     const double Gk[3] = {GE, GI, GR}, gk[3] = {ge, gi, gr};
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        const int c = c0 + h;
+        const int c = cc[h];
         const double* r = Rb2[h];
         if (c == 0 || c == 5) { // acoustic: (1, [vel -+ cs], ..., G_k e_k + w2/6 -+ vel cs/3)
             const double sg = c == 0 ? -1.0 : 1.0;
@@ -369,26 +369,30 @@ __device__ __forceinline__ void atomic_add6(double* W, long long plane, long lon
 //      state and flux cotangent Fb (from rbar);
 //   2. three threads per face, two characteristic fields c each: the forward
 //      reconstruction of field c, then its reverse: w-bar and f-bar of the six
-//      points, L-bar of row c, lambda-bar; L row c and g_c kept for step 3;
-//   3a. three threads per face: L-bar folded into R-bar (L = R^-1), the Roe
-//      base cotangent and the Roe average's vjp -> W at points 2 and 3
+//      points, lambda-bar; L row c goes to shared memory;
+//   3a. the same thread, the same two columns c of R-bar: L-bar folded in
+//      (L = R^-1) through its field's projections, the Roe base cotangent and,
+//      of the face's three, the Roe average's vjp -> W at points 2 and 3
 //      (atomic), the diffusion flux's vjp, and per point k of the face
 //      sum_c w-bar_ck L_c and sum_c f-bar_ck L_c;
 //   3b. one thread per point: the sums of 3a over the faces that use it, the
-//      physical flux's vjp -> W (atomic).
-// per-face rows are padded to FLUX_FACES + 1 doubles: the three threads of a
-// face in step 3a read different rows at the same face and land in different
-// banks
-constexpr int AFP = FLUX_FACES + 1;
+//      physical flux's vjp -> W (atomic). The warps that step 3a leaves without a
+//      Roe vjp take the first points.
+// A thread's place among a face's three is the same for a whole warp: rows of
+// per-face values are read along the faces, without bank conflicts, and no
+// branch on a field diverges.
+// Bound by latency at 12 warps per SM (168 registers; 81 KB of shared memory a
+// block) and shared-memory traffic. Eight 121 x 481 instances: 569 us a launch. With the
+// three threads of a face side by side in step 3a 682 us; whole warps 629 us;
+// the flux cotangents of step 1 and the first points of 3b on the idle warps
+// 619 us; L-bar through the projections, without its own rows and sums, 569 us.
+constexpr int AFP = FLUX_FACES;
 struct AdjFluxShared {
     double2 U[3][FLUX_NPT];
     double2 F[3][FLUX_NPT];
     double Q[15][AFP];     // Roe state u v w2 ee ei er cs2 cs he hi hr b den, 1/cs2, 1/b
     double FB[6][AFP];     // face flux cotangent
-    double G[6][AFP];      // g_c
-    double LAMB[6][AFP];   // lambda-bar_c
     double LS[6][6][AFP];  // L row c
-    double LB[6][6][AFP];  // L-bar row c
     double WB[6][6][AFP];  // w-bar [c][k]
     double FK[6][6][AFP];  // f-bar [c][k]
     int act[FLUX_FACES];
@@ -476,20 +480,27 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
         const double qv[15] = {q.u,  q.v,  q.w2, q.ee, q.ei, q.er,  q.cs2,       q.cs,
                                q.he, q.hi, q.hr, q.b,  q.den, inv(q.cs2), inv(q.b)};
         for (int k = 0; k < 15; ++k) S.Q[k][f] = qv[k];
-        for (int c = 0; c < 6; ++c) S.FB[c][f] = (RB[c][p3] - RB[c][p2]) * sc;
+    }
+    if (threadIdx.x >= FLUX_FACES) {
+        const int f = threadIdx.x & (FLUX_FACES - 1), c0 = threadIdx.x < 2 * FLUX_FACES ? 0 : 3;
+        int i, j, p0, ps;
+        adj_face_index<DIR>(t, f, i, j, p0, ps);
+        for (int c = c0; c < c0 + 3; ++c) S.FB[c][f] = (RB[c][p0 + 3 * ps] - RB[c][p0 + 2 * ps]) * sc;
     }
     __syncthreads();
     // ---- 2. two fields of one face per thread, so that a point's data are
     // loaded once for both (x faces: 0 and 5, 1 and 2, 3 and 4; y faces 0 and 5,
     // 2 and 3, 4 and 1)
     {
-        const int f = threadIdx.x & (FLUX_FACES - 1), g = threadIdx.x / FLUX_FACES; // g warp-uniform
-        if (S.act[f]) {
-            const int cc[2] = {DIR == 0 ? (g == 0 ? 0 : 2 * g - 1) : (g == 0 ? 0 : 2 * g),
-                               g == 0 ? 5 : (DIR == 0 ? 2 * g : (g == 1 ? 3 : 1))};
+        const int f = threadIdx.x & (FLUX_FACES - 1), part = threadIdx.x / FLUX_FACES; // part warp-uniform
+        const int cc[2] = {DIR == 0 ? (part == 0 ? 0 : 2 * part - 1) : (part == 0 ? 0 : 2 * part),
+                           part == 0 ? 5 : (DIR == 0 ? 2 * part : (part == 1 ? 3 : 1))};
+        const bool on = S.act[f] != 0;
+        double w[2][6], v[2][6], gval[2], lamb[2]; // L_c u_k, L_c F_k, g_c, lambda-bar_c
+        if (on) {
             int i, j, p0, ps;
             adj_face_index<DIR>(t, f, i, j, p0, ps);
-            double Lc[2][6], lam[2], gb[2], fp[2][6], fm[2][6], w[2][6];
+            double Lc[2][6], lam[2], gb[2], fp[2][6], fm[2][6];
             {
                 const Roe q = adj_load_q(S, f);
                 double FB[6];
@@ -516,102 +527,68 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
 #pragma unroll
                     for (int m = 0; m < 6; ++m) { cf = mad(Lc[e][m], F[m], cf); cs = mad(Lc[e][m], u[m], cs); }
                     w[e][k] = cs;
+                    v[e][k] = cf;
                     fp[e][k] = 0.5 * mad(a, cs, cf);
                     fm[e][k] = 0.5 * mad(-a, cs, cf);
                 }
             }
             // g_c = weno5(f+) + weno5(f-): both reconstructions are reversed
             // with the intermediates of their value
-            double wb[2][6], fb[2][6], Lb[2][6];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int c = cc[e];
                 const double a = fabs(lam[e]);
                 double fpb[6] = {0, 0, 0, 0, 0, 0}, ubm[5] = {0, 0, 0, 0, 0};
-                double gval = weno5_vjp(fp[e], P.eps, gb[e], fpb);
+                gval[e] = weno5_vjp(fp[e], P.eps, gb[e], fpb);
                 const double xm[5] = {fm[e][5], fm[e][4], fm[e][3], fm[e][2], fm[e][1]};
-                gval += weno5_vjp(xm, P.eps, gb[e], ubm);
-                S.G[c][f] = gval;
+                gval[e] += weno5_vjp(xm, P.eps, gb[e], ubm);
                 double ab = 0.0;
 #pragma unroll
                 for (int k = 0; k < 6; ++k) {
                     const double fmb = k == 0 ? 0.0 : ubm[5 - k];
                     const double d = fpb[k] - fmb;
-                    fb[e][k] = 0.5 * (fpb[k] + fmb);
-                    wb[e][k] = 0.5 * a * d;
                     ab = mad(0.5 * w[e][k], d, ab);
-                    S.WB[c][k][f] = wb[e][k];
-                    S.FK[c][k][f] = fb[e][k];
+                    S.WB[c][k][f] = 0.5 * a * d;
+                    S.FK[c][k][f] = 0.5 * (fpb[k] + fmb);
                 }
-                S.LAMB[c][f] = lam[e] < 0.0 ? -ab : ab;
+                lamb[e] = lam[e] < 0.0 ? -ab : ab;
 #pragma unroll
-                for (int m = 0; m < 6; ++m) {
-                    S.LS[c][m][f] = Lc[e][m];
-                    Lb[e][m] = 0.0;
-                }
+                for (int m = 0; m < 6; ++m) S.LS[c][m][f] = Lc[e][m];
             }
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                double u[6], F[6];
-                adj_point(S, p0 + k * ps, u, F);
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-#pragma unroll
-                    for (int m = 0; m < 6; ++m) Lb[e][m] = mad(wb[e][k], u[m], mad(fb[e][k], F[m], Lb[e][m]));
-            }
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-#pragma unroll
-                for (int m = 0; m < 6; ++m) S.LB[cc[e]][m][f] = Lb[e][m];
         }
-    }
-    __syncthreads();
-    // ---- 3a. per face, three threads (two columns of R each): L-bar folded
-    // into R-bar (L = R^-1), the Roe base cotangent; then the Roe average's
-    // vjp and the diffusion flux's vjp on the first of the three
-    {
-        const int f = threadIdx.x / 3, part = threadIdx.x - 3 * (threadIdx.x / 3);
-        const bool on = f < FLUX_FACES && S.act[f];
+        __syncthreads();
+        // ---- 3a. the same two columns c of R-bar: Fb g_c^T, and L-bar folded in
+        // (L = R^-1): R-bar -= L^T Z with Z = L-bar L^T, L-bar = sum_k w-bar_k u_k^T +
+        // f-bar_k F_k^T, so Z_jc = sum_k w-bar_jk (L_c u_k) + f-bar_jk (L_c F_k): the
+        // projections of step 2 and no L-bar. Then the Roe base cotangent, the
+        // Roe average's vjp and the diffusion flux's vjp
         double bb[5] = {0, 0, 0, 0, 0};
         if (on) {
-            // own columns c0, c0 + 1 of R-bar: Fb g_c^T, then -= sum_j L[j][i] Z[j][c]
-            // with Z[j][c] = sum_k Lb[j][k] L[c][k]
-            const int c0 = 2 * part;
-            double Rb2[2][6], lamb2[2], Z0[6] = {}, Z1[6] = {};
-            lamb2[0] = S.LAMB[c0][f];
-            lamb2[1] = S.LAMB[c0 + 1][f];
-            const double g0 = S.G[c0][f], g1 = S.G[c0 + 1][f];
+            double Rb2[2][6];
 #pragma unroll
             for (int m = 0; m < 6; ++m) {
                 const double fb = S.FB[m][f];
-                Rb2[0][m] = fb * g0;
-                Rb2[1][m] = fb * g1;
+                Rb2[0][m] = fb * gval[0];
+                Rb2[1][m] = fb * gval[1];
             }
 #pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                const double l0 = S.LS[c0][k][f], l1 = S.LS[c0 + 1][k][f];
+            for (int j = 0; j < 6; ++j) {
+                double z0 = 0.0, z1 = 0.0;
 #pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    const double lb = S.LB[j][k][f];
-                    Z0[j] = mad(lb, l0, Z0[j]);
-                    Z1[j] = mad(lb, l1, Z1[j]);
+                for (int k = 0; k < 6; ++k) {
+                    const double wb = S.WB[j][k][f], fb = S.FK[j][k][f];
+                    z0 = mad(wb, w[0][k], mad(fb, v[0][k], z0));
+                    z1 = mad(wb, w[1][k], mad(fb, v[1][k], z1));
                 }
-            }
 #pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                double a0 = 0.0, a1 = 0.0;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
+                for (int i = 0; i < 6; ++i) {
                     const double l = S.LS[j][i][f];
-                    a0 = mad(l, Z0[j], a0);
-                    a1 = mad(l, Z1[j], a1);
+                    Rb2[0][i] = mad(-l, z0, Rb2[0][i]);
+                    Rb2[1][i] = mad(-l, z1, Rb2[1][i]);
                 }
-                Rb2[0][i] -= a0;
-                Rb2[1][i] -= a1;
             }
-            const Roe q = adj_load_q(S, f);
-            const double base[5] = {q.u, q.v, q.ee, q.ei, q.er};
-            r_base_vjp2<DIR>(base, P, c0, Rb2, lamb2, bb);
+            const double base[5] = {S.Q[0][f], S.Q[1][f], S.Q[3][f], S.Q[4][f], S.Q[5][f]};
+            r_base_vjp2<DIR>(base, P, cc, Rb2, lamb, bb);
         }
         // per face and point k of this part: V_k = sum_c wbar_ck L_c and
         // VF_k = sum_c fbar_ck L_c (the point sums of 3b read these)
@@ -632,26 +609,22 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
                 }
             }
         }
-        __syncthreads(); // LB, WB, FK, G and LAMB are read: reuse them
+        __syncthreads(); // Q, WB and FK are read: reuse them
         if (on) {
 #pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                if (part == 0) S.FK[0][m][f] = bb[m];
-                if (part == 1) S.G[m][f] = bb[m];
-                if (part == 2) S.LAMB[m][f] = bb[m];
-            }
+            for (int m = 0; m < 5; ++m) S.Q[5 * part + m][f] = bb[m];
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
                 for (int m = 0; m < 6; ++m) {
-                    S.LB[2 * part + h][m][f] = V[h][m];
-                    S.WB[2 * part + h][m][f] = VF[h][m];
+                    S.WB[2 * part + h][m][f] = V[h][m];
+                    S.FK[2 * part + h][m][f] = VF[h][m];
                 }
         }
         __syncthreads();
         if (on && part < 2) { // the Roe average's vjp: point 3 on part 0, point 2 on part 1
 #pragma unroll
-            for (int m = 0; m < 5; ++m) bb[m] = S.FK[0][m][f] + (S.G[m][f] + S.LAMB[m][f]);
+            for (int m = 0; m < 5; ++m) bb[m] = S.Q[m][f] + (S.Q[5 + m][f] + S.Q[10 + m][f]);
             int i, j, p0, ps;
             adj_face_index<DIR>(t, f, i, j, p0, ps);
             double u3[6], u2[6], F_[6];
@@ -687,7 +660,7 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
         }
     }
     // ---- 3b. per point: sum over the faces and fields that use it
-    for (int p = threadIdx.x; p < np; p += blockDim.x) {
+    for (int p = (threadIdx.x + FLUX_FACES) % ADJ_FLUX_THREADS; p < np; p += blockDim.x) {
         // faces of this point: x tiles: same column, rows pr-5..pr; y tiles: same row, cols pc-5..pc
         int pr, pc, pi, pj;
         if (DIR == 0) { pr = p >> t.lg; pc = p & (cols - 1); pi = t.i - 3 + pr; pj = t.j0 + pc; }
@@ -709,8 +682,8 @@ __device__ void adj_flux_tile(const Inst& I, const Tile& t, const double* __rest
             any = true;
 #pragma unroll
             for (int m = 0; m < 6; ++m) {
-                ub[m] += S.LB[k][m][f]; // V_k of face f
-                fb[m] += S.WB[k][m][f]; // VF_k
+                ub[m] += S.WB[k][m][f]; // V_k of face f
+                fb[m] += S.FK[k][m][f]; // VF_k
             }
         }
         if (!any) continue;
