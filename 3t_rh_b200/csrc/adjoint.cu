@@ -337,25 +337,6 @@ __device__ __forceinline__ void r_base_vjp2(const double base[5], const DevParam
     bb[4] += be[2] + GR * gr * hc * bcs;
 }
 
-// L = R^-1, so dL = -L dR L and the cotangent Lb of L is one of R:
-// Rb -= L^T Lb L^T. Rb[c][i] = dJ/dR[i][c], Lb[c][j] = dJ/dL[c][j],
-// L[c][j] = L[6c + j].
-__device__ __forceinline__ void fold_l_into_r(const double* L, const double Lb[6][6], double Rb[6][6]) {
-    double Z[6][6]; // Z[j][c] = sum_k Lb[j][k] L[c][k]
-    for (int j = 0; j < 6; ++j)
-        for (int c = 0; c < 6; ++c) {
-            double acc = 0.0;
-            for (int k = 0; k < 6; ++k) acc += Lb[j][k] * L[6 * c + k];
-            Z[j][c] = acc;
-        }
-    for (int c = 0; c < 6; ++c)
-        for (int i = 0; i < 6; ++i) {
-            double acc = 0.0;
-            for (int j = 0; j < 6; ++j) acc += L[6 * j + i] * Z[j][c];
-            Rb[c][i] -= acc;
-        }
-}
-
 __device__ __forceinline__ void atomic_add6(double* W, long long plane, long long n, const double v[6]) {
 #pragma unroll
     for (int c = 0; c < 6; ++c)

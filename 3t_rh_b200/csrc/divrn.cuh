@@ -71,15 +71,6 @@ __device__ __forceinline__ Recip recip(double b) {
     return d;
 }
 
-// a Recip from a divisor and its stored reciprocal RN(1/b)
-__device__ __forceinline__ Recip recip_of(double b, double y) {
-    Recip d;
-    d.b = b;
-    d.y = y;
-    d.ok = div_in_range(b);
-    return d;
-}
-
 // a / d.b, correctly rounded
 __device__ __forceinline__ double div_rn(double a, const Recip& d) {
     if (!(d.ok && div_in_range(a))) return div_edge(a, d.b, d.y, d.ok);

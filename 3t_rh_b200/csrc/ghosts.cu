@@ -63,7 +63,7 @@ struct GhostSlot { // one ghost: half a warp
 };
 struct GhostWarp {
     GhostSlot g[2];
-    unsigned long long bar[2];
+    unsigned long long bar, pad;
 };
 static_assert(sizeof(GhostSlot) % 16 == 0 && sizeof(GhostWarp) % 16 == 0, "tables stay 16-byte aligned");
 static_assert(GH_COPY * 8 % 16 == 0 && GH_REC * 8 % 16 == 0 && 2 * GR_CHUNKS == GH_D, "record layout");
@@ -88,10 +88,10 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t b
 __device__ __forceinline__ void load_tables(GhostWarp& W, const double* __restrict__ hrec, int heavy0, int heavy1) {
     constexpr uint32_t bytes = GH_COPY * 8;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&W.bar[0])), "r"(2 * bytes)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&W.bar)), "r"(2 * bytes)
                  : "memory");
-    bulk_copy(W.g[0].rec, hrec + (size_t)heavy0 * GH_REC, bytes, &W.bar[0]);
-    bulk_copy(W.g[1].rec, hrec + (size_t)heavy1 * GH_REC, bytes, &W.bar[0]);
+    bulk_copy(W.g[0].rec, hrec + (size_t)heavy0 * GH_REC, bytes, &W.bar);
+    bulk_copy(W.g[1].rec, hrec + (size_t)heavy1 * GH_REC, bytes, &W.bar);
 }
 
 // a / b for operands of any sign, correctly rounded (divrn.cuh: |b| > 0 there)
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restr
     static_assert(sizeof(GhostRec) % 8 == 0 && kRecWords <= 16, "GhostRec copied as words by half a warp");
 
     if (lane == 0) {
-        mbar_init(&W.bar[0], 1);
+        mbar_init(&W.bar, 1);
         mbar_fence_init();
     }
     // per pair, loaded while the pair before it runs
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restr
             for (int j = 0; j < 6; ++j) a += L[6 * l + j] * uinf[j];
             G.vinf[l] = a;
         }
-        const bool ok_copy = __all_sync(0xffffffffu, mbar_wait(&W.bar[0], (uint32_t)(it & 1)));
+        const bool ok_copy = __all_sync(0xffffffffu, mbar_wait(&W.bar, (uint32_t)(it & 1)));
         if (!ok_copy) {
             if (l == 0 && write) report(I, 1 + 2 * stage, MBAR_TIMEOUT_CODE, (unsigned)G.cur.gid);
             return;

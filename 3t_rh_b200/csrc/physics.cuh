@@ -432,7 +432,7 @@ __device__ __forceinline__ void r_row(int row, const Roe& q, const RecipN& r6k, 
 // once per face and shared by the rows (divrn.cuh: every quotient is still
 // the IEEE one).
 struct RoeDiv {
-    Recip den, b, c6, c3, cg, gt;
+    Recip den, b, c6, c3, cg;
 };
 __device__ __forceinline__ RoeDiv roe_div(const Roe& q, const DevParams& P) {
     const double gt = (P.gamma_i - 1.0) + (P.gamma_e - 1.0) + (P.gamma_r - 1.0);
@@ -452,7 +452,6 @@ __device__ __forceinline__ RoeDiv roe_div(const Roe& q, const DevParams& P) {
         r.c3 = recip(3.0 * q.cs2);
     }
     r.cg = recip(gt * q.cs2);
-    r.gt = recip(gt);
     return r;
 }
 
@@ -731,41 +730,8 @@ __device__ __forceinline__ double jump8(const double* a) {
     return q_pulse7(a[7], a[6], a[5], a[4], a[3], a[2], a[1]) - q_pulse7(a[0], a[1], a[2], a[3], a[4], a[5], a[6]);
 }
 
-// noncon.rs:26-44
-__device__ __forceinline__ double d6(double qm3, double qm2, double qm1, double qp1, double qp2, double qp3,
-                                     double dx) {
-    return (qp3 - 9.0 * qp2 + 45.0 * qp1 - 45.0 * qm1 + 9.0 * qm2 - qm3) / (60.0 * dx);
-}
-
-// noncon.rs:288-332 nonconservative_direction_pre on a 9-point window
-// (pe, pi, pr, transport velocity vel per point, index 4 = cell).
-__device__ __forceinline__ void noncon9(const double pe[9], const double pi[9], const double pr[9],
-                                        const double vel[9], double ds, double out[3]) {
-    double v = vel[4];
-    double dpe = d6(pe[1], pe[2], pe[3], pe[5], pe[6], pe[7], ds);
-    double dpi = d6(pi[1], pi[2], pi[3], pi[5], pi[6], pi[7], ds);
-    double dpr = d6(pr[1], pr[2], pr[3], pr[5], pr[6], pr[7], ds);
-    double der_ee = 2.0 * dpe - dpi - dpr;
-    double der_ei = 2.0 * dpi - dpe - dpr;
-    double der_er = 2.0 * dpr - dpe - dpi;
-    double nee[9], nei[9], ner[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        nee[k] = 2.0 * pe[k] - pi[k] - pr[k];
-        nei[k] = 2.0 * pi[k] - pe[k] - pr[k];
-        ner[k] = 2.0 * pr[k] - pe[k] - pi[k];
-    }
-    double jm_ee = jump8(nee), jm_ei = jump8(nei), jm_er = jump8(ner);
-    double jp_ee = jump8(nee + 1), jp_ei = jump8(nei + 1), jp_er = jump8(ner + 1);
-    double coef_left = fmax(fmax(v, vel[3]), 0.0) / 3.0;
-    double coef_right = fmin(fmin(v, vel[5]), 0.0) / 3.0;
-    out[0] = v / 3.0 * der_ee + (coef_left * jm_ee + coef_right * jp_ee) / ds;
-    out[1] = v / 3.0 * der_ei + (coef_left * jm_ei + coef_right * jp_ei) / ds;
-    out[2] = v / 3.0 * der_er + (coef_left * jm_er + coef_right * jp_er) / ds;
-}
-
-// noncon9 from the jumps at the cell's two interfaces (jm, jp; each interface's
-// are formed once and shared by its two cells) and from the pressures and
+// noncon.rs:288-332 nonconservative_direction_pre (derivatives of noncon.rs:26-44)
+// from the jumps at the cell's two interfaces (jm, jp; each interface's are formed once and shared by its two cells) and from the pressures and
 // the transport velocity in memory at centre p, stride st. r60ds, rds: the
 // divisors 60 ds and ds.
 template <class DV, class R>
