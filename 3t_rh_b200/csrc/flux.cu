@@ -22,10 +22,10 @@
 // warps each on other fields the barriers were the top stall, 2.1-2.6 warps per
 // issued instruction), and the quotients a face's rows share are formed once.
 // 8 blocks of 128 registers: 10 blocks of 96 spill (3% slower), 6 blocks of 150
-// 4% slower. Without a branch per quotient (divrn.cuh) and in this form the 24
-// batch instances' fluxes take 1.30 ms a step instead of 2.08 ms, the
-// 961 x 3841 half-cylinder's 4.75 ms instead of 7.44 ms (same bits); FMA build
-// 0.94 ms instead of 1.17 ms.
+// 4% slower. Without a branch per quotient (divrn.cuh), in this form and in one launch
+// the fluxes of 24 batch instances take 1.24 ms a step instead of 2.08 ms, of the
+// 961 x 3841 half-cylinder 4.67 ms instead of 7.44 ms (same bits); FMA build
+// 0.90 ms instead of 1.17 ms.
 //
 // RH3T_EXACT selects the reference's expressions; otherwise the fastm forms
 // (shared reciprocals, one division per WENO5) are used.
