@@ -148,6 +148,20 @@ __device__ __forceinline__ bool num_near(double a) {
     return h - 0x23d00000u <= 0x384fffffu || (h | (unsigned)__double2loint(a)) == 0u;
 }
 
+// Divisors b > 0 with an exponent in [-100, 100] (leading 20 fraction bits not all
+// ones) admit numerators down to 2^-880: the quotient is at least 2^-981 and the
+// residual a multiple of 2^-986, so both are normal and exact as above, and what
+// a yl loses as a subnormal (2^-1075) is 2^-41 ulp of the quotient: the first
+// quotient is within (1/2 + 2^-40) ulp, and the argument holds with its margin.
+__device__ __forceinline__ bool den_mid_near(double b) {
+    const unsigned h = (unsigned)__double2hiint(b);
+    return h - 0x39b00000u <= 0x0c8fffffu && (h & 0xfffffu) != 0xfffffu;
+}
+__device__ __forceinline__ bool num_small_near(double a) {
+    const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return h - 0x08f00000u <= 0x532fffffu || (h | (unsigned)__double2loint(a)) == 0u;
+}
+
 // a / d.b, correctly rounded
 __device__ __forceinline__ double div_near(double a, const RecipN& d) {
     const double q = __fma_rn(a, d.y, __dmul_rn(a, d.yl));
@@ -177,7 +191,7 @@ __device__ __forceinline__ double div_once(double c, double b) {
 // as -y, so that a zero numerator keeps its sign): the residual is a small
 // multiple of ulp(q), or of 2^-1074, so it is exact down to the subnormals, where a / 3 is
 // never a tie. a / 6 likewise, except that a subnormal quotient can be a
-// tie: for a zero or |a| >= 2^-1000 (num6_near).
+// tie: for a zero or a finite |a| >= 2^-1000 (num6_near).
 __device__ __forceinline__ double div3_near(double a) {
     const double y = 0x1.5555555555555p-2;
     const double q = __dmul_rn(a, y);
@@ -190,7 +204,7 @@ __device__ __forceinline__ double div6_near(double a) {
 }
 __device__ __forceinline__ bool num6_near(double a) {
     const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    return h >= 0x01700000u || (h | (unsigned)__double2loint(a)) == 0u;
+    return h - 0x01700000u <= 0x7e7fffffu || (h | (unsigned)__double2loint(a)) == 0u;
 }
 
 } // namespace rh3t

@@ -55,7 +55,7 @@ constexpr bool kExact = false;
 //   T:  per point te, ti, tr (launches with a diffusive instance);
 //   gkgt, y6: no-contraction build, gk / gt and the reciprocal of 6 gk (both
 //       parts) for gk = ge, gi, gr;
-//   act: per face 0 (no flux), 1 (quotients in the branch-free form) or 2.
+//   act: per face near_face's answer (launches with several thread groups a tile).
 constexpr int NQ = kExact ? 19 : 15, PT = 7;
 struct FluxShared {
     double2* pt;
@@ -169,10 +169,18 @@ static __device__ __noinline__ double char_flux_each(const double2* pf, int ps, 
     return r0 + r1;
 }
 
-// g_c; near: the face's quotients are within the branch-free form's range
+// entries 0 (acoustic rows only) to 2 of the row of L, for a face with a tiny velocity
+template <int DIR>
+static __device__ __noinline__ LVel char_row_velocity(const double* Qf, const DevParams& P, int c) {
+    Roe q;
+    load_q(Qf, q);
+    return l_row_velocity<DIR>(c, q, P);
+}
+
+// g_c; mode: near_face's answer
 template <int DIR>
 __device__ __forceinline__ double char_flux(const double2* pf, int ps, const double* Qf, const DevParams& P, int c,
-                                            const double* gkgt, bool near) {
+                                            const double* gkgt, int mode) {
     Roe q;
     load_q(Qf, q);
     double Lc[6], fp[6], fm[6];
@@ -187,6 +195,12 @@ __device__ __forceinline__ double char_flux(const double2* pf, int ps, const dou
         rd.cg = {gt * q.cs2, Qf[17 * FLUX_FACES], Qf[18 * FLUX_FACES]};
         rd.scale();
         l_row<DIR>(c, q, rd, gkgt[energy_index<DIR>(c)], P, Lc);
+        if (mode == 2) {
+            const LVel l = char_row_velocity<DIR>(Qf, P, c);
+            if (c == 0 || c == 5) Lc[0] = l.l0;
+            Lc[1] = l.l1;
+            Lc[2] = l.l2;
+        }
         split_fluxes(pf, ps, Lc, a, fp, fm);
     } else {
         fastm::l_row<DIR>(c, q, Qf[13 * FLUX_FACES], Qf[14 * FLUX_FACES], P, Lc);
@@ -195,6 +209,7 @@ __device__ __forceinline__ double char_flux(const double2* pf, int ps, const dou
     if (!kExact)
         return fastm::weno5(fp[0], fp[1], fp[2], fp[3], fp[4], P.eps) +
                fastm::weno5(fm[5], fm[4], fm[3], fm[2], fm[1], P.eps);
+    bool near = mode != 0;
     const double r0 = weno5_near(fp[0], fp[1], fp[2], fp[3], fp[4], P.eps, near);
     const double r1 = weno5_near(fm[5], fm[4], fm[3], fm[2], fm[1], P.eps, near);
     return near ? r0 + r1 : char_flux_each<DIR>(pf, ps, Qf, P, c, gkgt[energy_index<DIR>(c)]);
@@ -304,7 +319,7 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
     }
     __syncthreads();
     double* Qf = S.Q + f;
-    bool near = true;
+    int near = 1; // near_face's answer
     if (valid && g == 0) {
         // points[3] and points[2] of the face: the staged primitives (the
         // same functions of the same states as a fresh evaluation)
@@ -320,7 +335,7 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
             q = roe_average_sqrt(rho3, d3, rho2, d2, P);
             RoeDivN rd;
             const double gt = (P.gamma_i - 1.0) + (P.gamma_e - 1.0) + (P.gamma_r - 1.0);
-            near = near_face(q, gt, rd) & near_params(P);
+            near = near_params(P) ? near_face(q, gt, rd) : 0;
             y[0] = rd.den.y; y[1] = rd.den.yl; y[2] = rd.b.y; y[3] = rd.b.yl; y[4] = rd.cg.y; y[5] = rd.cg.yl;
         } else {
             const double a6[6] = {rho3, d3.u, d3.v, d3.e_e, d3.e_i, d3.e_r};
@@ -335,10 +350,10 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
 #pragma unroll
         for (int k = 13; k < NQ; ++k) Qf[k * FLUX_FACES] = y[k - 13];
     }
-    if (NG > 1 && g == 0) S.act[f] = near ? 1 : 2;
+    if (NG > 1 && g == 0) S.act[f] = near;
     __syncthreads(); // E is read; G takes its place
     if (NG == 1 && !valid) return;
-    if (NG > 1) near = S.act[f] == 1;
+    if (NG > 1) near = S.act[f];
     // ---- 3. characteristic pass (a loop, not unrolled: one copy of its code
     // stays within the instruction cache)
     double* Gf = S.G + f;
@@ -376,9 +391,7 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
 
 constexpr int FLUX_NG3 = 2 * 148, FLUX_NG2 = 4 * 148; // tiles up to which 3 and 2 groups share a tile
 // blocks per SM (FMA build: 12 blocks of 80 registers 2% faster than 8)
-#ifndef FLUX_MIN_BLOCKS
-#define FLUX_MIN_BLOCKS (kExact ? 8 : 12)
-#endif
+constexpr int FLUX_MIN_BLOCKS = kExact ? 8 : 12;
 // x faces (blocks [0, ntx)), then y faces: in one launch the y tiles fill the
 // SMs that the last x tiles leave idle (121 x 481: two launches of 0.8 waves each
 // took 42 us, one takes 31 us).

@@ -259,6 +259,18 @@ __device__ __forceinline__ NearD operator*(NearD a, NearD b) { return a.v * b.v;
 __device__ __forceinline__ NearD operator/(NearD a, NearD b) { return div_near(a.v, recip_near(b.v)); }
 __device__ __forceinline__ NearD quot3(NearD x) { return div3_near(x.v); }
 __device__ __forceinline__ NearD quot6(NearD x) { return div6_near(x.v); }
+// the entries of L with a tiny velocity in the numerator
+static __device__ __noinline__ void lr_velocity(const Roe* q, const DevParams& P, double* LR) {
+#pragma unroll 1
+    for (int row = 0; row < 6; ++row) {
+        if (row == 4) continue;
+        const LVel l = l_row_velocity<0>(row, *q, P);
+        if (row == 0 || row == 5) LR[6 * row * CHUNK] = l.l0;
+        LR[(6 * row + 1) * CHUNK] = l.l1;
+        LR[(6 * row + 2) * CHUNK] = l.l2;
+    }
+}
+
 // L, R and lambda at the nearest fluid node of heavy ghost Rg in its (normal,
 // tangential) frame (bc1.rs:294-312)
 __device__ __forceinline__ void local_lr(const Inst& I, const GhostRec& Rg, int stage, double* LR) {
@@ -274,7 +286,8 @@ __device__ __forceinline__ void local_lr(const Inst& I, const GhostRec& Rg, int 
     const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
     const double gt = gi + ge + gr;
     RoeDivN rd;
-    if (near_face(q, gt, rd) & near_params(P) & near_divisor(gt)) {
+    const int mode = near_params(P) && den_mid_near(gt) ? near_face(q, gt, rd) : 0;
+    if (mode != 0) {
         if (!kExactG) {
             const RoeT<NearD> n = {q.u, q.v, q.w2, q.ee, q.ei, q.er, q.cs2, q.cs, q.he, q.hi, q.hr, q.b, q.den};
 #pragma unroll
@@ -289,6 +302,10 @@ __device__ __forceinline__ void local_lr(const Inst& I, const GhostRec& Rg, int 
                 }
                 LR[(GH_LR_LAM + row) * CHUNK] = lam.v;
             }
+            if (mode == 2) {
+                const Roe t = q;
+                lr_velocity(&t, P, LR);
+            }
             return;
         }
         rd.scale();
@@ -301,6 +318,10 @@ __device__ __forceinline__ void local_lr(const Inst& I, const GhostRec& Rg, int 
             l_row<0>(row, q, rd, row >= 1 && row <= 3 ? div_near(gl, rgt) : 0.0, P, Lr);
             r_row<0, true>(row, q, row >= 3 ? recip_near(6.0 * gk) : rgt, P, Rr);
             store_lr(LR, row, Lr, Rr, q);
+        }
+        if (mode == 2) {
+            const Roe t = q;
+            lr_velocity(&t, P, LR);
         }
     } else {
         const Roe t = q;

@@ -92,7 +92,9 @@ struct Prim {
 struct DivEach {
     bool ok = true;
     __device__ __forceinline__ Recip den(double b) { return recip(b); }
+    __device__ __forceinline__ Recip den_mid(double b) { return recip(b); }
     __device__ __forceinline__ double div(double a, const Recip& d) { return div_rn(a, d); }
+    __device__ __forceinline__ double div_small(double a, const Recip& d) { return div_rn(a, d); }
     __device__ __forceinline__ double div3(double a) { return div3_rn(a); }
     __device__ __forceinline__ double div6(double a) { return div6_rn(a); }
 };
@@ -106,9 +108,19 @@ struct DivGroup {
         ok = ok & num_near(a);
         return div_near(a, d);
     }
+    // velocities, which fall to zero ahead of a front through every magnitude: a
+    // narrower range of divisors leaves more room below (divrn.cuh)
+    __device__ __forceinline__ RecipN den_mid(double b) {
+        ok = ok & den_mid_near(b);
+        return recip_near(b);
+    }
+    __device__ __forceinline__ double div_small(double a, const RecipN& d) { // d by den_mid
+        ok = ok & num_small_near(a);
+        return div_near(a, d);
+    }
     __device__ __forceinline__ double div3(double a) { return div3_near(a); } // any finite a
     __device__ __forceinline__ double div6(double a) {
-        ok = ok & num_near(a);
+        ok = ok & num6_near(a);
         return div6_near(a);
     }
 };
@@ -117,9 +129,9 @@ struct DivGroup {
 // each formed once.
 template <class DV> __device__ __forceinline__ Prim prim_by(const double s[6], const DevParams& P, DV& dv) {
     Prim d;
-    const auto r0 = dv.den(s[0]);
-    d.u = dv.div(s[1], r0);
-    d.v = dv.div(s[2], r0);
+    const auto r0 = dv.den_mid(s[0]);
+    d.u = dv.div_small(s[1], r0);
+    d.v = dv.div_small(s[2], r0);
     double w2 = sqd(d.u) + sqd(d.v);
     const double w6 = dv.div6(w2), rw6 = dv.div6(s[0] * w2);
     d.e_e = dv.div(s[3], r0) - w6;
@@ -158,8 +170,8 @@ __device__ __forceinline__ Prim prim_from_state(const double s[6], const DevPara
 template <class DV, class R>
 __device__ __forceinline__ void temps_by(const double s[6], const DevParams& P, const R& r6e, const R& r6i,
                                          const R& ra, DV& dv, double& te, double& ti, double& er) {
-    const auto r0 = dv.den(s[0]);
-    const double u = dv.div(s[1], r0), v = dv.div(s[2], r0);
+    const auto r0 = dv.den_mid(s[0]);
+    const double u = dv.div_small(s[1], r0), v = dv.div_small(s[2], r0);
     const double w2 = sqd(u) + sqd(v);
     te = dv.div(s[3], dv.den(s[0] * P.cve)) - dv.div(w2, r6e);
     ti = dv.div(s[4], dv.den(s[0] * P.cvi)) - dv.div(w2, r6i);
@@ -220,9 +232,9 @@ __device__ __forceinline__ Roe roe_by(double rho1, const Prim& d3, double rho2, 
                                       DV& dv) {
     Roe q;
     double rho_sum = rho1 + rho2;
-    const auto rs = dv.den(rho_sum);
-    q.u = dv.div(d3.u * rho1 + d2.u * rho2, rs);
-    q.v = dv.div(d3.v * rho1 + d2.v * rho2, rs);
+    const auto rs = dv.den_mid(rho_sum);
+    q.u = dv.div_small(d3.u * rho1 + d2.u * rho2, rs);
+    q.v = dv.div_small(d3.v * rho1 + d2.v * rho2, rs);
     q.w2 = sqd(q.u) + sqd(q.v);
     q.ee = dv.div(d3.e_e * rho1 + d2.e_e * rho2, rs);
     q.ei = dv.div(d3.e_i * rho1 + d2.e_i * rho2, rs);
@@ -456,25 +468,33 @@ __device__ __forceinline__ RoeDiv roe_div(const Roe& q, const DevParams& P) {
 }
 
 // The branch-free form for a whole face: reciprocals of the five divisors
-// (rd), and whether every quotient of its rows of L and R is covered by the
-// argument in divrn.cuh. The divisors are within 2^-100..2^101 and u, v are
-// zero or within 2^-430..2^101, so with the gammas' factors gk, gt within
-// 2^-20..2^21 (near_params) the numerators u, v, w2, vel cs and their
-// multiples by gk, gt, cs are zero or at least 2^-904 and the quotients at least
-// 2^-1005: residuals are multiples of 2^-1008, so nothing underflows.
+// (rd), and whether the quotients of its rows of L and R are covered by the
+// argument in divrn.cuh: 1 if all are, 2 if all but the entries of L that
+// l_row_velocity forms, 0 otherwise. The divisors are within 2^-100..2^101, u and v
+// are zero or within 2^-790..2^101 and w2 is zero or at least 2^-800, so with the
+// gammas' factors gk, gt within 2^-20..2^22 (near_params) the numerators (gk, gt,
+// gk gt times u, v or w2, and gt w2 +- 6 vel cs, whose terms cancel to no less
+// than an ulp of 2^-840) are zero or at least 2^-904 and the quotients at least
+// 2^-1005: residuals are multiples of 2^-1008, so nothing underflows. A smaller
+// velocity is in the numerators of l_row_velocity's entries alone (those of R are
+// divided by 3, or hold w2). Such faces are common: ahead of a front a velocity
+// falls to zero through every magnitude (20 steps into the 121 x 481 half-cylinder a
+// third of the nodes hold one below 2^-430). With a face 0 for any velocity below
+// 2^-430 that state's fluxes took 294 us a step (general form throughout: 206 us),
+// now 132 us; the test of a third answer costs other states 0.8%.
 __device__ __forceinline__ bool near_params(const DevParams& P) {
     const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
     const double lo = 0x1p-20, hi = 0x1p20;
     return ge >= lo && ge <= hi && gi >= lo && gi <= hi && gr >= lo && gr <= hi && P.eps >= 0x1p-100 &&
            P.eps <= 0x1p100 && den_near(6.0 * ge) && den_near(6.0 * gi) && den_near(6.0 * gr);
 }
-__device__ __forceinline__ bool near_divisor(double b) {
-    const unsigned h = (unsigned)__double2hiint(b);
-    return h - 0x39b00000u <= 0x0c8fffffu && (h & 0xfffffu) != 0xfffffu;
-}
 __device__ __forceinline__ bool near_velocity(double a) {
     const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    return h - 0x25100000u <= 0x212fffffu || (h | (unsigned)__double2loint(a)) == 0u;
+    return h - 0x0e900000u <= 0x37afffffu || (h | (unsigned)__double2loint(a)) == 0u;
+}
+__device__ __forceinline__ bool near_square(double w2) {
+    const unsigned h = (unsigned)__double2hiint(w2);
+    return h >= 0x0df00000u || (h | (unsigned)__double2loint(w2)) == 0u;
 }
 struct RoeDivN {
     RecipN den, b, c6, c3, cg;
@@ -484,12 +504,14 @@ struct RoeDivN {
         c3 = {0.25 * den.b, 4.0 * den.y, 4.0 * den.yl};
     }
 };
-__device__ __forceinline__ bool near_face(const Roe& q, double gt, RoeDivN& rd) {
-    const double cg = gt * q.cs2;
+__device__ __forceinline__ int near_face(const Roe& q, double gt, RoeDivN& rd) {
+    const double cg = gt * q.cs2, most = 0x1p101;
     rd.den = recip_near(q.den);
     rd.b = recip_near(q.b);
     rd.cg = recip_near(cg);
-    return near_divisor(q.den) & near_divisor(q.b) & near_divisor(cg) & near_velocity(q.u) & near_velocity(q.v);
+    const bool ok = den_mid_near(q.den) & den_mid_near(q.b) & den_mid_near(cg) & near_square(q.w2) &
+                    (fabs(q.u) < most) & (fabs(q.v) < most);
+    return ok ? (near_velocity(q.u) & near_velocity(q.v) ? 1 : 2) : 0;
 }
 
 __device__ __forceinline__ double quot(double a, const Recip& d) { return div_rn(a, d); }
@@ -552,6 +574,31 @@ __device__ __forceinline__ void l_row(int row, const Roe& q, const RD& rd, doubl
             L[3 + j] = quot(-gk * gj, rd.cg) - quot(n2, rd.b) * f;
         }
     }
+}
+
+// The entries of row `row` whose numerators a velocity below near_velocity's range
+// can take out of the branch-free form's, by IEEE quotients: the first three of an
+// acoustic row, the second and third of an energy row
+struct LVel {
+    double l0, l1, l2;
+};
+template <int DIR>
+__device__ __forceinline__ LVel l_row_velocity(int row, const Roe& q, const DevParams& P) {
+    const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
+    const double gt = gi + ge + gr;
+    const double u = q.u, v = q.v, w2 = q.w2, cs = q.cs, cs2 = q.cs2;
+    const int mode = row_mode<DIR>(row);
+    if (mode == 0 || mode == 5) {
+        const double s = mode == 0 ? 1.0 : -1.0;
+        return {__ddiv_rn(gt * w2 + s * (6.0 * (DIR == 0 ? u : v) * cs), q.den),
+                __ddiv_rn(DIR == 0 ? -2.0 * gt * u + -s * (6.0 * cs) : -2.0 * gt * u, q.den),
+                __ddiv_rn(DIR == 0 ? -2.0 * gt * v : -2.0 * gt * v + -s * (6.0 * cs), q.den)};
+    }
+    const int k = mode - 2;
+    const double gk = k == 0 ? ge : (k == 1 ? gi : gr), hk = k == 0 ? q.he : (k == 1 ? q.hi : q.hr);
+    const double c3 = 3.0 * cs2, h = hk - cs2 * w2;
+    return {0.0, __ddiv_rn(gk * u, c3) + __ddiv_rn(2.0 * gk * gt * u, q.b) * h,
+            __ddiv_rn(gk * v, c3) + __ddiv_rn(2.0 * gk * gt * v, q.b) * h};
 }
 
 // ---------------------------------------------------------------- fast forms
@@ -731,9 +778,10 @@ __device__ __forceinline__ double jump8(const double* a) {
 }
 
 // noncon.rs:288-332 nonconservative_direction_pre (derivatives of noncon.rs:26-44)
-// from the jumps at the cell's two interfaces (jm, jp; each interface's are formed once and shared by its two cells) and from the pressures and
-// the transport velocity in memory at centre p, stride st. r60ds, rds: the
-// divisors 60 ds and ds.
+// from the jumps at the cell's two interfaces (jm, jp; each interface's are
+// formed once and shared by its two cells) and from the pressures and the transport
+// velocity in memory at centre p, stride st. r60ds, rds: the divisors 60 ds and ds
+// (den_mid).
 template <class DV, class R>
 __device__ __forceinline__ void noncon_by(const double* pe, const double* pi, const double* pr, const double* vel,
                                           int st, const double jm[3], const double jp[3], const R& r60ds,
@@ -748,13 +796,13 @@ __device__ __forceinline__ void noncon_by(const double* pe, const double* pi, co
     const double coef_right = dv.div3(fmin(fmin(v, vel[st]), 0.0));
     const double v3 = dv.div3(v);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) out[c] = v3 * der[c] + dv.div(coef_left * jm[c] + coef_right * jp[c], rds);
+    for (int c = 0; c < 3; ++c) out[c] = v3 * der[c] + dv.div_small(coef_left * jm[c] + coef_right * jp[c], rds);
 }
 static __device__ __noinline__ void noncon_each(const double* pe, const double* pi, const double* pr,
                                                 const double* vel, int st, const double* jm, const double* jp,
                                                 double ds, double* out) {
     DivEach dv;
-    noncon_by(pe, pi, pr, vel, st, jm, jp, dv.den(60.0 * ds), dv.den(ds), dv, out);
+    noncon_by(pe, pi, pr, vel, st, jm, jp, dv.den(60.0 * ds), dv.den_mid(ds), dv, out);
 }
 
 // dt.rs:5-34 get_local_dt (same association order; CVE^3 = CVE*(CVE*CVE)),
@@ -788,8 +836,8 @@ __device__ __forceinline__ T local_dt_t(const T s[6], double dx, double dy, cons
 template <class DV>
 __device__ __forceinline__ double local_dt_by(const double s[6], double dx, double dy, const DevParams& P, DV& dv) {
     const double OEI = P.omega_ei, OER = P.omega_er;
-    const auto r0 = dv.den(s[0]);
-    const double u = dv.div(s[1], r0), v = dv.div(s[2], r0);
+    const auto r0 = dv.den_mid(s[0]);
+    const double u = dv.div_small(s[1], r0), v = dv.div_small(s[2], r0);
     const double w6 = dv.div6(sqd(u) + sqd(v));
     const double ee = dv.div(s[3], r0) - w6, ei = dv.div(s[4], r0) - w6, er = dv.div(s[5], r0) - w6;
     const double GE = P.gamma_e, GI = P.gamma_i, GR = P.gamma_r, A = P.a_rad, CVE = P.cve, CVI = P.cvi;

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_BLOCKS) k_rhs_stage(const Ins
             DivGroup dv;
             noncon_by(c0, c0 + NPT, c0 + 2 * NPT, c0 + 3 * NPT, HJ, jm, jp, rhs_recip(I, sR, 0), rhs_recip(I, sR, 1), dv,
                       ncx);
-            if (!(dv.ok & den_near(60.0 * dx) & den_near(dx))) {
+            if (!(dv.ok & den_near(60.0 * dx) & den_mid_near(dx))) {
                 const double a[3] = {jm[0], jm[1], jm[2]}, b[3] = {jp[0], jp[1], jp[2]};
                 double o[3];
                 noncon_each(c0, c0 + NPT, c0 + 2 * NPT, c0 + 3 * NPT, HJ, a, b, dx, o);
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_BLOCKS) k_rhs_stage(const Ins
             DivGroup dv;
             noncon_by(c0, c0 + NPT, c0 + 2 * NPT, c0 + 4 * NPT, 1, jm, jp, rhs_recip(I, sR, 2), rhs_recip(I, sR, 3), dv,
                       ncy);
-            if (!(dv.ok & den_near(60.0 * dy) & den_near(dy))) {
+            if (!(dv.ok & den_near(60.0 * dy) & den_mid_near(dy))) {
                 const double a[3] = {jm[0], jm[1], jm[2]}, b[3] = {jp[0], jp[1], jp[2]};
                 double o[3];
                 noncon_each(c0, c0 + NPT, c0 + 2 * NPT, c0 + 4 * NPT, 1, a, b, dy, o);
