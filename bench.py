@@ -63,17 +63,13 @@ CFL = 0.05
 # --warmup 3 --no-cpu --no-e2e` (FMA build, when x and y faces were one
 # launch); None where no capture exists
 FLUX_TRAFFIC_BYTES = {"fma": {"cyl961": 651.5e6}, "exact": {}}
-# DRAM bytes per heavy ghost of one stage's ghost update (k_ghost_prep +
-# k_ghosts) and per active face of one stage's k_flux<0> + k_flux<1>, from
-# ncu captures on the batch24 workload (84,000 heavy ghosts, 860,240 x and
-# 854,216 y faces), scaled by the heavy-ghost and face counts of the batched
-# workloads. The no-contraction capture holds k_ghosts and both flux
-# kernels; its ghost figure takes k_ghost_prep's bytes from the FMA-build
-# capture (the same loads and stores in both builds).
-GHOST_TRAFFIC_PER_HEAVY = {"fma": (902.88e6 + 7.24e6 + 15.32e6 + 9.25e6) / 84000,
-                           "exact": (902.77e6 + 7.46e6 + 15.32e6 + 9.25e6) / 84000}
-FLUX_TRAFFIC_PER_FACE = {"fma": (74.60e6 + 43.63e6) / 1714456,
-                         "exact": (48.41e6 + 12.05e6 + 45.41e6 + 9.40e6) / 1714456}
+# DRAM bytes per heavy ghost of one stage's k_ghosts and per active face of one
+# stage's k_flux, from an ncu capture of the no-contraction build on the batch24
+# workload (84,000 heavy ghosts, 860,240 x and 854,216 y faces), scaled by the
+# heavy-ghost and face counts of the batched workloads; the FMA build makes the
+# same loads and stores.
+GHOST_TRAFFIC_PER_HEAVY = dict.fromkeys(("fma", "exact"), (911.40e6 + 74.15e6) / 84000)
+FLUX_TRAFFIC_PER_FACE = dict.fromkeys(("fma", "exact"), (89.16e6 + 57.14e6) / 1714456)
 FALLBACK_HBM_GBS = 6650.0
 
 
@@ -420,7 +416,7 @@ def scale_record(rh, torch, flops, local, exact, wl="cyl961", steps=20):
     prof = s.profile_steps(5, CFL)
     nxf, nyf = flops.face_counts(f.fluid, f.grid.nx, f.grid.ny)
     fl_launch = flops.flux_launch_flops(nxf, nyf, False)
-    flux_ms, flux_n = prof["flux"][0], 3 * 5  # per stage: the x-face and the y-face launch
+    flux_ms, flux_n = prof["flux"][0], 3 * 5  # one launch per stage
     total = sum(v[0] for v in prof.values())
     s.close()
     return {"workload": WORKLOADS[wl]["name"], "fluid_cells": cells, "steps": steps, "ms_per_step": ms / steps,
@@ -583,7 +579,7 @@ def run_batch(args, rh, flops, torch, dist, world, rank, local):
     clocks = sampler.summary()
     k_prof = min(args.steps, 10)
     prof = b.profile_steps(k_prof, CFL)
-    flux_ms, flux_n = prof["flux"][0], 3 * k_prof  # per stage: the x-face and the y-face launch
+    flux_ms, flux_n = prof["flux"][0], 3 * k_prof  # one launch per stage
     achieved = fl_launch / (flux_ms / flux_n * 1e-3) / 1e12
     peak = rh.api.fp64_peak_tflops(local)
     total_prof_ms = sum(v[0] for v in prof.values())
@@ -594,13 +590,13 @@ def run_batch(args, rh, flops, torch, dist, world, rank, local):
     hbm, hbm_src = hbm_peak()
     g_achieved = g_bytes / (ghost_stage_ms * 1e-3) / 1e9
     bkey = "exact" if args.exact else "fma"
-    rl_flux = {"bound": "fp64", "kernel": "k_flux<0> + k_flux<1> (x and y interface WENO5 fluxes of one stage, "
+    rl_flux = {"bound": "fp64", "kernel": "k_flux (x and y interface WENO5 fluxes of one stage, "
                "all instances)",
                "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                "traffic": None if FLUX_TRAFFIC_PER_FACE[bkey] is None else FLUX_TRAFFIC_PER_FACE[bkey] * n_faces,
-               "traffic_unit": "bytes per stage (both launches)",
+               "traffic_unit": "bytes per stage",
                "peak_source": "measured DFMA loop on this GPU (rh3t_fp64_peak)",
-               "flops_per_stage": fl_launch, "stage_ms": flux_ms / flux_n, "launches_per_stage": 2,
+               "flops_per_stage": fl_launch, "stage_ms": flux_ms / flux_n, "launches_per_stage": 1,
                "flop_count": "algorithmic: every add, sub, mul, div, sqrt of the reference's expressions = 1 "
                              "(a division costs 3-14 FP64 issue slots here)"}
     if args.exact:
@@ -608,7 +604,7 @@ def run_batch(args, rh, flops, torch, dist, world, rank, local):
         # stream without FMA peaks at half the DFMA FLOP rate
         rl_flux["no_fma_ceiling"] = peak / 2.0
         rl_flux["frac_of_no_fma_ceiling"] = achieved / (peak / 2.0)
-    rl_ghost = {"bound": "hbm", "kernel": "k_ghost_prep + k_ghosts (one stage's ghost update, all instances)",
+    rl_ghost = {"bound": "hbm", "kernel": "k_ghosts (one stage's ghost update, all instances)",
                 "achieved": g_achieved, "peak": hbm, "unit": "GB/s", "frac": g_achieved / hbm,
                 "traffic": None if GHOST_TRAFFIC_PER_HEAVY[bkey] is None else GHOST_TRAFFIC_PER_HEAVY[bkey] * n_heavy,
                 "traffic_unit": "bytes per stage", "peak_source": hbm_src,
@@ -798,7 +794,7 @@ def main():
 
     # roofline of the dominant kernel: live per-launch durations (CUDA events)
     prof = s.profile_steps(min(args.steps, 20), CFL)
-    flux_ms, flux_n = prof["flux"][0], 3 * min(args.steps, 20)  # per stage: the x-face and the y-face launch
+    flux_ms, flux_n = prof["flux"][0], 3 * min(args.steps, 20)  # one launch per stage
     fl_launch = flops.flux_launch_flops(nxf, nyf, diff)
     achieved = fl_launch / (flux_ms / flux_n * 1e-3) / 1e12
     peak = rh.api.fp64_peak_tflops(local)
@@ -839,13 +835,13 @@ def main():
                        "ghost_build_s": round(build_s, 3)},
             "arithmetic": "no FMA contraction, IEEE quotients, correctly rounded pow (the reference's "
                           "roundings)" if args.exact else "FMA contraction, shared reciprocals",
-            "roofline": {"bound": "fp64", "kernel": "k_flux<0> + k_flux<1> (x and y interface WENO5 fluxes of one "
+            "roofline": {"bound": "fp64", "kernel": "k_flux (x and y interface WENO5 fluxes of one "
                          "stage)", "achieved": achieved,
                          "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "traffic": FLUX_TRAFFIC_BYTES["exact" if args.exact else "fma"].get(args.workload),
-                         "traffic_unit": "bytes per stage (both launches)",
+                         "traffic_unit": "bytes per stage",
                          "peak_source": "measured DFMA loop on this GPU (rh3t_fp64_peak)",
-                         "flops_per_stage": fl_launch, "stage_ms": flux_ms / flux_n, "launches_per_stage": 2,
+                         "flops_per_stage": fl_launch, "stage_ms": flux_ms / flux_n, "launches_per_stage": 1,
                          **({"no_fma_ceiling": peak / 2.0, "frac_of_no_fma_ceiling": achieved / (peak / 2.0)}
                             if args.exact else {}),
                          "kernel_share": {k: v[0] / total_prof_ms for k, v in prof.items()},
