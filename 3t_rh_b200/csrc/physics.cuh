@@ -40,13 +40,14 @@ __device__ __forceinline__ double cr_powi(double x, int n) {
     if (!isfinite(x) || x == 0.0) return pow(x, (double)n);
     DD r = {1.0, 0.0}, a = {x, 0.0};
     bool first = true;
+    const bool negative = x < 0.0 && (n & 1);
     while (n > 0) {
         if (n & 1) { r = first ? a : dd_mul(r, a); first = false; }
         n >>= 1;
         if (n) a = (a.lo == 0.0) ? dd_sq(a.hi) : dd_mul(a, a);
     }
     // overflow (the low parts are NaN then): infinity, as the reference's powf
-    if (!isfinite(r.hi)) return (n & 1) && x < 0.0 ? -INFINITY : INFINITY;
+    if (!isfinite(r.hi)) return negative ? -INFINITY : INFINITY;
     return __dadd_rn(r.hi, r.lo);
 }
 // x^(1/4): sqrt(sqrt(x)) is within one ulp; of it and its two neighbours pick
