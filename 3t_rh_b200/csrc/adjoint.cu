@@ -128,7 +128,8 @@ __device__ __forceinline__ double weno5_vjp(const double x[5], double eps, doubl
     const double e0 = inv(mad(q0, r0, mad(c1312 * t0, t0, eps)));
     const double e1 = inv(mad(q1, r1, mad(c1312 * t1, t1, eps)));
     const double e2 = inv(mad(q2, r2, mad(c1312 * t2, t2, eps)));
-    const double a0 = 0.1 * e0 * e0, a1 = 0.6 * e1 * e1, a2 = 0.3 * e2 * e2;
+    // the alphas by a quarter (exactly): inv() flushes the reciprocal of a sum above 2^1022 to zero
+    const double a0 = 0.1 / 4 * e0 * e0, a1 = 0.6 / 4 * e1 * e1, a2 = 0.3 / 4 * e2 * e2;
     const double iS = inv(a0 + a1 + a2);
     const double w0 = a0 * iS, w1 = a1 * iS, w2 = a2 * iS;
     const double p0 = mad(x[0], K3, mad(11.0 / 6.0, x[2], -7.0 / 6.0 * x[1]));
