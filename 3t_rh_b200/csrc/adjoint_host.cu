@@ -119,11 +119,12 @@ void enqueue_recorded_step(rh3t_ctx* c, double* rec) {
     int nh, nc;
     ghost_ranges(c, nh, nc);
     for (int st = 0; st < 3; ++st) {
-        launch_ghosts(s, c->d_inst, c->d_gpart, nh, c->d_gpart + c->n_gheavy, nc, c->d_hrec, c->d_lr, st);
+        launch_ghosts(s, c->d_inst, c->d_gpart, nh, c->d_gpart + c->n_gheavy, nc, c->d_hrec, c->d_lr, st,
+                      c->ghosts_ordered);
         launch_adj_copy(s, c->d_inst, 0, c->n_inst, mp, st, rec + st * np, 0);
         const int nf = enqueue_flux(c, s, st, r);
         enqueue_rhs(c, s, st, 2, rec + (3 + st) * np, r);
-        c->launches += ghost_launches(nh, nc) + nf + 2;
+        c->launches += ghost_launches(nh, nc, c->ghosts_ordered) + nf + 2;
     }
     c->launches += 1;
 }
@@ -147,7 +148,8 @@ extern "C" int rh3t_l_vjp(rh3t_ctx* c, int32_t k, const double* rbar, double* ub
     CK(c, cudaMemcpyAsync(&sc->t_stage[0], &sc->t_after, sizeof(double), cudaMemcpyDeviceToDevice, s));
     int nh, nc;
     ghost_ranges(c, nh, nc);
-    launch_ghosts(s, c->d_inst, c->d_gpart, nh, c->d_gpart + c->n_gheavy, nc, c->d_hrec, c->d_lr, 0);
+    launch_ghosts(s, c->d_inst, c->d_gpart, nh, c->d_gpart + c->n_gheavy, nc, c->d_hrec, c->d_lr, 0,
+                  c->ghosts_ordered);
     launch_adj_copy(s, c->d_inst, 0, c->n_inst, max_plane(c), 0, a->U2, 0); // X = U2 as scratch
     CK(c, cudaMemsetAsync(a->rbar, 0, np * sizeof(double), s));
     CK(c, cudaMemsetAsync(a->U0, 0, np * sizeof(double), s));
@@ -156,7 +158,7 @@ extern "C" int rh3t_l_vjp(rh3t_ctx* c, int32_t k, const double* rbar, double* ub
     launch_adj_aos(s, c->d_inst, k, 1, n, c->d_io, a->rbar, 0);
     enqueue_vjp_l(c, a->U2, a->rbar, a->U0);
     launch_adj_aos(s, c->d_inst, k, 1, n, c->d_io, a->U0, 1);
-    c->launches += ghost_launches(nh, nc) + 3;
+    c->launches += ghost_launches(nh, nc, c->ghosts_ordered) + 3;
     CK(c, cudaMemcpyAsync(ubar, c->d_io + 6 * H.cell_off, (size_t)n * 6 * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (pbar8) CK(c, cudaMemcpyAsync(pbar8, a->pbar + 8 * k, 8 * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(c, cudaGetLastError());

@@ -166,8 +166,9 @@ int enqueue_ghosts(rh3t_ctx* c, cudaStream_t s, int stage, Span r) {
     const HostInst& a = c->hi[r.k0];
     int nh, nc;
     ghost_counts(c, r, nh, nc);
-    launch_ghosts(s, c->d_inst, c->d_gpart + a.gh0, nh, c->d_gpart + c->n_gheavy + a.gc0, nc, c->d_hrec, c->d_lr, stage);
-    return ghost_launches(nh, nc);
+    launch_ghosts(s, c->d_inst, c->d_gpart + a.gh0, nh, c->d_gpart + c->n_gheavy + a.gc0, nc, c->d_hrec,
+                  c->d_lr + (size_t)a.gh0 * GH_LR, stage, c->ghosts_ordered);
+    return ghost_launches(nh, nc, c->ghosts_ordered);
 }
 
 void enqueue_dt(rh3t_ctx* c, cudaStream_t s, int mode, Span r) {
@@ -194,7 +195,7 @@ long long launches_per_step(const rh3t_ctx* c) {
     ghost_counts(c, all(c), nh, nc);
     const HostInst &a = c->hi[0], &b = c->hi[c->n_inst - 1];
     const int nf = flux_launches(b.tx0 + b.ntx - a.tx0, b.ty0 + b.nty - a.ty0);
-    return 1 + 3 * (ghost_launches(nh, nc) + nf + 1);
+    return 1 + 3 * (ghost_launches(nh, nc, c->ghosts_ordered) + nf + 1);
 }
 
 // bc1.rs:930-1037 / 471-545: nearest fluid node to the mirror point 2 P0 - Pg
@@ -236,6 +237,7 @@ struct Built {
     std::vector<GhostRec> recs; // table order
     std::vector<double> hrec;   // n_heavy * GH_REC
     int n_heavy = 0;
+    bool ordered = false;       // the ghost update's order matters (kernels.cuh launch_ghosts)
 };
 
 // Tile shapes of an nx x ny grid before any tuning: the default, unless another
@@ -350,6 +352,7 @@ int build_instance(const rh3t_instance& d, int inst, HostInst& H, Inst& I, Built
                 return RH3T_ERR_GEOMETRY;
             }
             R.src = node(ni, nj);
+            B.ordered = B.ordered || !fluid[(size_t)ni * ny + nj];
         } else if (kind == BC_REFLECTIVE_WALL || kind == BC_ZEROTH_ORDER) {
             long oi = 0, oj = 0;
             if (!mirror_source(*grid, fluid, i, j, R.p0x, R.p0y, oi, oj)) {
@@ -373,6 +376,11 @@ int build_instance(const rh3t_instance& d, int inst, HostInst& H, Inst& I, Built
         } else {
             R.src = R.node;
         }
+    }
+    if (!B.ordered && nh) { // a node that is a cheap ghost and a heavy one
+        std::vector<uint8_t> of((size_t)plane, 0);
+        for (const GhostRec& R : B.recs) of[R.node] |= R.heavy >= 0 ? 2 : 1;
+        for (const GhostRec& R : B.recs) B.ordered = B.ordered || of[R.node] == 3;
     }
     // heavy records: rows of S and w | d | pad | stencil nodes
     B.hrec.assign((size_t)nh * GH_REC, 0.0);
@@ -654,6 +662,7 @@ extern "C" int rh3t_batch_create(int32_t n, const rh3t_instance* desc, int32_t d
         for (GhostRec& R : B[k].recs)
             if (R.heavy >= 0) R.heavy += heavy_base;
         heavy_base += B[k].n_heavy;
+        c->ghosts_ordered = c->ghosts_ordered || B[k].ordered;
         ghost_base += H.n_ghosts;
         c->max_ghosts = std::max(c->max_ghosts, H.n_ghosts);
     }
@@ -699,7 +708,7 @@ extern "C" int rh3t_batch_create(int32_t n, const rh3t_instance* desc, int32_t d
     DA(c->d_ghosts, std::max(c->n_ghosts, 1));
     DA(c->d_gpart, std::max(c->n_ghosts, 1));
     DA(c->d_hrec, std::max((long long)c->n_heavy * GH_REC, 1LL));
-    DA(c->d_lr, std::max((long long)c->n_heavy * GH_LR, 1LL));
+    DA(c->d_lr, std::max((long long)c->n_gheavy * GH_LR, 1LL));
     DA(c->d_io, c->total_cells * 6);
     DA(c->d_io2, (c->total_cells + c->max_ghosts) * 6); // rhs planes, then ghost values
 #undef DA

@@ -54,7 +54,7 @@ struct rh3t_ctx {
     rh3t::GhostRec* d_ghosts = nullptr; // table order (instance-major, gid within)
     rh3t::GhostRec* d_gpart = nullptr;  // heavy ghosts by heavy slot, then the cheap ones
     double* d_hrec = nullptr;           // heavy records (GH_REC doubles each)
-    double* d_lr = nullptr;             // ghost update's scratch (GH_LR doubles per heavy record)
+    double* d_lr = nullptr;             // ghost update's scratch (GH_LR doubles per heavy ghost)
     rh3t::Tile* d_tx = nullptr;
     rh3t::Tile* d_ty = nullptr;
     rh3t::Tile* d_tc = nullptr;
@@ -67,6 +67,7 @@ struct rh3t_ctx {
     long long max_faces = 0;      // max over instances of max((nx+1)*ny, nx*(ny+1))
     struct AdjBuffers* adj = nullptr;
     struct rh3t_io* io = nullptr; // snapshot and diagnostic buffers (io.cu)
+    bool ghosts_ordered = false;        // a table needs the ghost update in order (kernels.cuh launch_ghosts)
     int n_ghosts = 0, n_heavy = 0, n_gheavy = 0, n_gcheap = 0, max_ghosts = 0;
     cudaGraphExec_t graph = nullptr;
     cudaStream_t xfer[2] = {nullptr, nullptr};  // host-copy streams of rh3t_step_host_batch (in, out)

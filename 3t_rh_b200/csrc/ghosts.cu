@@ -365,6 +365,10 @@ constexpr unsigned long long kTaskC[2] = {0x3210543210543210ull, 0x0054321054321
 constexpr unsigned long long kTaskR[2] = {0x2222333333444444ull, 0x0000000011111122ull};
 __device__ __forceinline__ int task_digit(unsigned long long k, int l) { return (int)(k >> (4 * l)) & 15; }
 
+// What a launch does: all of the update in one, unless a table makes the order of
+// its parts matter (launch_ghosts)
+enum { GH_PART_ALL = 0, GH_PART_LR = 1, GH_PART_REST = 2 };
+
 // Warps take the heavy ghosts in turn, two at a time (half-warps 0 and 1; an
 // odd last ghost runs on both halves and is written by the first). What the
 // next pair needs is fetched in four places, so that no load waits on the one
@@ -385,7 +389,8 @@ __device__ __forceinline__ int task_digit(unsigned long long k, int l) { return 
 __global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restrict__ insts,
                                                              const GhostRec* __restrict__ heavy, int nh,
                                                              const GhostRec* __restrict__ cheap, int nc,
-                                                             const double* __restrict__ hrec, double* lrbuf, int stage) {
+                                                             const double* __restrict__ hrec, double* lrbuf, int stage,
+                                                             int part) {
     extern __shared__ __align__(128) unsigned char gh_smem[];
     const int lane = threadIdx.x & 31, half = lane >> 4, l = lane & 15, warp = threadIdx.x >> 5;
     GhostWarp& W = reinterpret_cast<GhostWarp*>(gh_smem)[warp];
@@ -425,22 +430,20 @@ __global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restr
     for (int i0 = first; i0 < npair; i0 += CHUNK * stride) {
     // ---- 1. L, R, lambda of the chunk's ghosts, one per lane, staged in the
     // table buffer and stored by half-warps
-    {
-        const bool mine = l < CHUNK && i0 + l * stride < npair;
-        int slot = 0;
-        if (mine) {
+    if (part != GH_PART_REST) {
+        if (l < CHUNK && i0 + l * stride < npair) {
             const GhostRec Rg = heavy[min(2 * (i0 + l * stride) + half, nh - 1)];
-            slot = Rg.heavy;
             local_lr(insts[Rg.inst], Rg, stage, G.rec + l);
         }
         __syncwarp();
         for (int t = 0; t < CHUNK && i0 + t * stride < npair; ++t) {
-            double* o = lrbuf + (size_t)__shfl_sync(0xffffffffu, slot, (lane & 16) + t) * GH_LR;
+            double* o = lrbuf + (size_t)min(2 * (i0 + t * stride) + half, nh - 1) * GH_LR;
 #pragma unroll
             for (int j = 0; j < 5; ++j)
                 if (l + 16 * j < 78) o[l + 16 * j] = G.rec[(l + 16 * j) * CHUNK + t];
         }
         __syncwarp();
+        if (part == GH_PART_LR) continue;
     }
     // the chunk's first pair
     {
@@ -455,7 +458,7 @@ __global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restr
         for (int j = 0; j < 4; ++j)
             if (l + 16 * j < 55) load6(buf, I.plane, __ldg(&st[l + 16 * j]), s[j]);
 #pragma unroll
-        for (int j = 0; j < 5; ++j) lr[j] = __ldcg(lrbuf + (size_t)slot * GH_LR + l + 16 * j);
+        for (int j = 0; j < 5; ++j) lr[j] = __ldcg(lrbuf + (size_t)min(2 * i0 + half, nh - 1) * GH_LR + l + 16 * j);
         ui_l = l < 6 ? I.bcs[__ldg(&R0.bc)].state[l] : 0.0;
         eps = I.P.eps;
         weno_q = I.P.weno_q;
@@ -619,7 +622,8 @@ __global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restr
             for (int j = 0; j < 4; ++j)
                 if (l + 16 * j < 55) load6(nbuf, nplane, st[j], s[j]);
 #pragma unroll
-            for (int j = 0; j < 5; ++j) lr[j] = __ldcg(lrbuf + (size_t)n_heavy * GH_LR + l + 16 * j);
+            for (int j = 0; j < 5; ++j)
+                lr[j] = __ldcg(lrbuf + (size_t)min(2 * (i + stride) + half, nh - 1) * GH_LR + l + 16 * j);
             if (l < 6) ui_l = nbcs[n_bc].state[l];
             n_skip = nerr->key != ~0ull;
         }
@@ -708,7 +712,7 @@ __global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restr
 }
 
 void launch_ghosts(cudaStream_t s, const Inst* insts, const GhostRec* heavy, int nh, const GhostRec* cheap, int nc,
-                   const double* hrec, double* lrbuf, int stage) {
+                   const double* hrec, double* lrbuf, int stage, bool ordered) {
     if (nh + nc <= 0) return;
     static int sm_count[64] = {0};
     int dev = 0;
@@ -720,12 +724,25 @@ void launch_ghosts(cudaStream_t s, const Inst* insts, const GhostRec* heavy, int
         cudaFuncSetAttribute(k_ghosts, cudaFuncAttributeMaxDynamicSharedMemorySize, GH_SMEM);
         sm_count[dev] = n > 0 ? n : 1;
     }
-    const int n = std::max((nh + 1) / 2, (6 * nc + GH_WARPS * 32 - 1) / (GH_WARPS * 32));
-    k_ghosts<<<std::min(n, sm_count[dev]), GH_WARPS * 32, GH_SMEM, s>>>(insts, heavy, nh, cheap, nc, hrec, lrbuf,
-                                                                         stage);
+    auto launch = [&](int h, int c, int part) {
+        const int n = std::max((h + 1) / 2, (6 * c + GH_WARPS * 32 - 1) / (GH_WARPS * 32));
+        if (n > 0)
+            k_ghosts<<<std::min(n, sm_count[dev]), GH_WARPS * 32, GH_SMEM, s>>>(insts, heavy, h, cheap, c, hrec, lrbuf,
+                                                                                 stage, part);
+    };
+    if (!ordered) {
+        launch(nh, nc, GH_PART_ALL);
+        return;
+    }
+    launch(nh, 0, GH_PART_LR);
+    launch(0, nc, GH_PART_ALL);
+    launch(nh, 0, GH_PART_REST);
 }
 
-int ghost_launches(int nh, int nc) { return nh + nc > 0 ? 1 : 0; }
+int ghost_launches(int nh, int nc, bool ordered) {
+    if (!ordered) return nh + nc > 0 ? 1 : 0;
+    return (nh > 0 ? 2 : 0) + (nc > 0 ? 1 : 0);
+}
 
 // one warp: the ghost update's bounded wait on a fresh mbarrier whose phase
 // completes (arrive: one arrival, no bytes expected) or never does; out[0] =

@@ -6,10 +6,14 @@
 namespace rh3t {
 // heavy: Wall / Outflow / FarField records; cheap: all other kinds (ghosts.cu)
 // hrec: heavy records (GH_REC doubles per GhostBC slot); lrbuf: scratch, GH_LR
-// doubles per slot. One kernel: ghost_launches().
+// doubles per heavy ghost. One kernel, in which ghosts are written in any order while
+// others are formed: every node read has to be fluid, and every ghost node
+// another. ordered: for a table where that does not hold (a nearest node that is not
+// fluid, a node that is a cheap ghost and a heavy one), L, R and lambda, the cheap
+// ghosts and the heavy ones in three launches. ghost_launches(): how many.
 void launch_ghosts(cudaStream_t s, const Inst* insts, const GhostRec* heavy, int nh, const GhostRec* cheap, int nc,
-                   const double* hrec, double* lrbuf, int stage);
-int ghost_launches(int nh, int nc);
+                   const double* hrec, double* lrbuf, int stage, bool ordered);
+int ghost_launches(int nh, int nc, bool ordered);
 // Shared memory of a flux launch: stencil points of its largest x and y tile
 // (flux_points of direction and shape), and whether an instance has diffusion on
 struct FluxSize {

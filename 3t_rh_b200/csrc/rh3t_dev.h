@@ -119,7 +119,7 @@ struct Tile {
 // (int32, + 1 pad).
 constexpr int GH_ROWS = 0, GH_D = 1204, GH_COPY = 1210, GH_ST = 1210;
 constexpr int GH_REC = 1238;                     // doubles per record (9904 bytes)
-constexpr int GH_LR = 80;                        // per GhostBC slot and stage: L, R, lambda (78), pad (ghost update's scratch)
+constexpr int GH_LR = 80;                        // per heavy ghost and stage: L, R, lambda (78), pad (ghost update's scratch)
 
 constexpr int CELL_TILE = 128;
 constexpr int FLUX_FACES = 64;                   // faces per flux block
