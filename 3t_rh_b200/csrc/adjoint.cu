@@ -35,6 +35,7 @@
 #include "kernels.cuh"
 #include "physics.cuh"
 #include "ghost_rows.cuh"
+#include "per_device.h"
 
 namespace rh3t {
 
@@ -1555,15 +1556,17 @@ void launch_adj_l(cudaStream_t s, const Inst* insts, int k0, int n, long long ma
                   const GhostRec* cheap, int nc, const double* hrec, const double* X, const double* rbar, double* W,
                   double* Ub, double* pbar, double* slots, int wall_outflow) {
     if (n <= 0) return;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_adj_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_CELL_SMEM);
-        cudaFuncSetAttribute(k_adj_flux, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjFluxShared));
-        cudaFuncSetAttribute(k_adj_ghost_lr, cudaFuncAttributeMaxDynamicSharedMemorySize, AG_LR_SMEM);
-        cudaFuncSetAttribute(k_adj_ghosts<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AG_SMEM);
-        cudaFuncSetAttribute(k_adj_ghosts<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AG_SMEM);
-        attr = true;
-    }
+    static OncePerDevice attributes;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    attributes(dev, [] {
+        constexpr cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        return cudaFuncSetAttribute(k_adj_cells, a, ADJ_CELL_SMEM) == cudaSuccess &&
+               cudaFuncSetAttribute(k_adj_flux, a, (int)sizeof(AdjFluxShared)) == cudaSuccess &&
+               cudaFuncSetAttribute(k_adj_ghost_lr, a, AG_LR_SMEM) == cudaSuccess &&
+               cudaFuncSetAttribute(k_adj_ghosts<false>, a, AG_SMEM) == cudaSuccess &&
+               cudaFuncSetAttribute(k_adj_ghosts<true>, a, AG_SMEM) == cudaSuccess;
+    });
     if (nh > 0)
         k_adj_ghost_lr<<<(nh + AG_LR_THREADS - 1) / AG_LR_THREADS, AG_LR_THREADS, AG_LR_SMEM, s>>>(insts, heavy, nh,
                                                                                                   X, slots);

@@ -40,6 +40,7 @@
 #include "physics.cuh"
 #include "ghost_rows.cuh"
 #include "mbar.cuh"
+#include "per_device.h"
 
 namespace rh3t {
 
@@ -714,20 +715,17 @@ __global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restr
 void launch_ghosts(cudaStream_t s, const Inst* insts, const GhostRec* heavy, int nh, const GhostRec* cheap, int nc,
                    const double* hrec, double* lrbuf, int stage, bool ordered) {
     if (nh + nc <= 0) return;
-    static int sm_count[64] = {0};
-    int dev = 0;
+    static OncePerDevice attributes;
+    int dev = 0, sms = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    if (sm_count[dev] == 0) {
-        int n = 0;
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(k_ghosts, cudaFuncAttributeMaxDynamicSharedMemorySize, GH_SMEM);
-        sm_count[dev] = n > 0 ? n : 1;
-    }
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    attributes(dev, [] {
+        return cudaFuncSetAttribute(k_ghosts, cudaFuncAttributeMaxDynamicSharedMemorySize, GH_SMEM) == cudaSuccess;
+    });
     auto launch = [&](int h, int c, int part) {
         const int n = std::max((h + 1) / 2, (6 * c + GH_WARPS * 32 - 1) / (GH_WARPS * 32));
         if (n > 0)
-            k_ghosts<<<std::min(n, sm_count[dev]), GH_WARPS * 32, GH_SMEM, s>>>(insts, heavy, h, cheap, c, hrec, lrbuf,
+            k_ghosts<<<std::min(n, std::max(sms, 1)), GH_WARPS * 32, GH_SMEM, s>>>(insts, heavy, h, cheap, c, hrec, lrbuf,
                                                                                  stage, part);
     };
     if (!ordered) {

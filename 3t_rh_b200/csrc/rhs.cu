@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "per_device.h"
 #include "physics.cuh"
 
 namespace rh3t {
@@ -280,16 +281,14 @@ __global__ void __launch_bounds__(RHS_THREADS, RHS_BLOCKS) k_rhs_stage(const Ins
 void launch_rhs_stage(cudaStream_t s, const Inst* insts, const Tile* tc, int nt, int stage, int mode, double* rhs,
                       int smem) {
     if (nt <= 0) return;
-    static bool attr[64] = {false};
+    static OncePerDevice attributes;
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    if (!attr[dev]) {
+    attributes(dev, [] {
         int most = 0;
         for (int lg = RHS_LG_MIN; lg <= RHS_LG_MAX; ++lg) most = std::max(most, rhs_smem(lg));
-        cudaFuncSetAttribute(k_rhs_stage, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        attr[dev] = true;
-    }
+        return cudaFuncSetAttribute(k_rhs_stage, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
+    });
     k_rhs_stage<<<nt, RHS_THREADS, smem, s>>>(insts, tc, nt, stage, mode, rhs);
 }
 
