@@ -523,6 +523,7 @@ __global__ void __launch_bounds__(GH_WARPS * 32, 1) k_ghosts(const Inst* __restr
         const bool ok_copy = __all_sync(0xffffffffu, mbar_wait(&W.bar, (uint32_t)(it & 1)));
         if (!ok_copy) {
             if (l == 0 && write) report(I, 1 + 2 * stage, MBAR_TIMEOUT_CODE, (unsigned)G.cur.gid);
+            (void)mbar_wait(&W.bar, (uint32_t)(it & 1)); // (once more: they write this block's shared memory)
             return;
         }
         __syncwarp();

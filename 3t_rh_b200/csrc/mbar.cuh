@@ -1,6 +1,5 @@
 // Shared-memory mbarriers (PTX mbarrier.*) with bounded waits, used by the
-// ghost update (bulk-copy completion) and the interface fluxes (the hand-off
-// of staged tiles between warps). Every wait gives up after a fixed number of
+// ghost update (bulk-copy completion). Every wait gives up after a fixed number of
 // try_wait rounds and returns false; the caller then records a timeout in the
 // instance's error key and leaves its loop, so no warp waits without end.
 #pragma once
