@@ -55,8 +55,8 @@ __device__ __forceinline__ double near_quotient(int cat, double a, double b, dou
         const double t = scalbn(a, sh - ilogb(a));
         const double got3 = div3_near(t), got6 = div6_near(t);
         if (cat == 4 && !same_bits(got3, __ddiv_rn(t, 3.0))) return got3;
-        if (cat == 5 && num6_near(t) && !same_bits(got6, __ddiv_rn(t, 6.0))) return got6;
-        return cat == 4 ? div3_near(a) : (num6_near(a) ? div6_near(a) : want);
+        if (cat == 5 && !same_bits(got6, __ddiv_rn(t, 6.0))) return got6;
+        return cat == 4 ? div3_near(a) : div6_near(a);
     }
     if (!den_near(b) || !num_near(a)) return want;
     const double q = div_near(a, recip_near(b));

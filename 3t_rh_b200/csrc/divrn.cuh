@@ -190,21 +190,22 @@ __device__ __forceinline__ double div_once(double c, double b) {
 // a / 3 for every finite a (the residual taken as 3 q - a and the correction
 // as -y, so that a zero numerator keeps its sign): the residual is a small
 // multiple of ulp(q), or of 2^-1074, so it is exact down to the subnormals, where a / 3 is
-// never a tie. a / 6 likewise, except that a subnormal quotient can be a
-// tie: for a zero or a finite |a| >= 2^-1000 (num6_near).
+// never a tie. a / 6 likewise, except that a subnormal quotient can be a tie,
+// a = (6 k + 3) 2^-1074: q is k there (a y lies just below the tie) and the residual
+// three units, which y, less than 1 / 6, would leave at k. For an odd k the next
+// double above y, more than 1 / 6, takes it to the even k + 1; the residuals of other
+// quotients there are four units at most, and either y rounds them alike.
 __device__ __forceinline__ double div3_near(double a) {
     const double y = 0x1.5555555555555p-2;
     const double q = __dmul_rn(a, y);
     return __fma_rn(__fma_rn(3.0, q, -a), -y, q);
 }
 __device__ __forceinline__ double div6_near(double a) {
-    const double y = 0x1.5555555555555p-3;
-    const double q = __dmul_rn(a, y);
+    const double q = __dmul_rn(a, 0x1.5555555555555p-3);
+    const int odd = (__double2hiint(q) & 0x7ff00000) == 0 ? __double2loint(q) & 1 : 0; // of a subnormal q
+    const double y = __hiloint2double(0x3fc55555, 0x55555555 + odd);
     return __fma_rn(__fma_rn(6.0, q, -a), -y, q);
 }
-__device__ __forceinline__ bool num6_near(double a) {
-    const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    return h - 0x01700000u <= 0x7e7fffffu || (h | (unsigned)__double2loint(a)) == 0u;
-}
+__device__ __forceinline__ bool finite_near(double a) { return ((unsigned)__double2hiint(a) & 0x7fffffffu) < 0x7ff00000u; }
 
 } // namespace rh3t

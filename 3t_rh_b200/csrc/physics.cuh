@@ -121,7 +121,7 @@ struct DivGroup {
     }
     __device__ __forceinline__ double div3(double a) { return div3_near(a); } // any finite a
     __device__ __forceinline__ double div6(double a) {
-        ok = ok & num6_near(a);
+        ok = ok & finite_near(a);
         return div6_near(a);
     }
 };
@@ -741,8 +741,9 @@ __device__ __forceinline__ double weno5(double u0, double u1, double u2, double 
 // weno5 in the branch-free form (divrn.cuh); ok is cleared when an operand is
 // outside its range (then the value is not used). Numerators need no test: the
 // 0.1, 0.6, 0.3 and the alphas they give are bounded by the divisors' range;
-// u / 3 holds for every finite u, and a u that is not finite makes one of the
-// three divisors infinite or NaN.
+// u / 3 and u / 6 hold for every finite u, and a u that is not finite makes one of the
+// three divisors infinite or NaN. (0.25 r^2 in one FMA differs from its rounded
+// product where that is subnormal alone, which no divisor in range can show.)
 __device__ __forceinline__ double weno5_near(double u0, double u1, double u2, double u3, double u4, double eps,
                                              bool& ok) {
     // products by 2, 4 and 1/4 are exact, so their sums are one FMA each
@@ -761,7 +762,7 @@ __device__ __forceinline__ double weno5_near(double u0, double u1, double u2, do
     const double p0 = div3_near(u0) - 7.0 / 6.0 * u1 + 11.0 / 6.0 * u2;
     const double p1 = div6_near(-u1) + 5.0 / 6.0 * u2 + div3_near(u3);
     const double p2 = div3_near(u2) + 5.0 / 6.0 * u3 - div6_near(u4);
-    ok = ok & den_near(s0) & den_near(s1) & den_near(s2) & den_near(sum_o) & num6_near(u1) & num6_near(u4);
+    ok = ok & den_near(s0) & den_near(s1) & den_near(s2) & den_near(sum_o);
     return w0 * p0 + w1 * p1 + w2 * p2;
 }
 
