@@ -142,6 +142,15 @@ __device__ __forceinline__ bool den_near(double b) {
     return h - 0x23d00000u <= 0x384fffffu && (h & 0xfffffu) != 0xfffffu;
 }
 
+// div_near(a, recip_near(b)) rounds correctly beyond the operands that den_near and
+// num_near admit: for b as den_near wants it and a zero, or with an exponent of -969 or
+// more and a quotient within 2^-1000..2^1000. The residual a - b q is a multiple of
+// 2^(e - 105), e the exponent of a, so it is exact; q is normal; and what a yl loses as a
+// subnormal (2^-1075) is at most 2^-23 ulp of the quotient: the first quotient
+// is within (1/2 + 2^-22) ulp, and the argument holds with its margin
+// ((1 + 2^-22) (1 + 2^-25) (1 - 2^-19) < 1). The tests of a group bound numerators and
+// divisors so that this holds for each of its quotients.
+
 // a is zero, or its exponent is in [-450, 450]
 __device__ __forceinline__ bool num_near(double a) {
     const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
@@ -149,10 +158,7 @@ __device__ __forceinline__ bool num_near(double a) {
 }
 
 // Divisors b > 0 with an exponent in [-100, 100] (leading 20 fraction bits not all
-// ones) admit numerators down to 2^-880: the quotient is at least 2^-981 and the
-// residual a multiple of 2^-986, so both are normal and exact as above, and what
-// a yl loses as a subnormal (2^-1075) is 2^-41 ulp of the quotient: the first
-// quotient is within (1/2 + 2^-40) ulp, and the argument holds with its margin.
+// ones) admit numerators down to 2^-880: the quotient is at least 2^-981.
 __device__ __forceinline__ bool den_mid_near(double b) {
     const unsigned h = (unsigned)__double2hiint(b);
     return h - 0x39b00000u <= 0x0c8fffffu && (h & 0xfffffu) != 0xfffffu;
@@ -160,6 +166,13 @@ __device__ __forceinline__ bool den_mid_near(double b) {
 __device__ __forceinline__ bool num_small_near(double a) {
     const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
     return h - 0x08f00000u <= 0x532fffffu || (h | (unsigned)__double2loint(a)) == 0u;
+}
+
+// b > 0, exponent in [-100, 450], leading 20 fraction bits not all ones: the numerators'
+// lower bound is the caller's
+__device__ __forceinline__ bool den_wide_near(double b) {
+    const unsigned h = (unsigned)__double2hiint(b);
+    return h - 0x39b00000u <= 0x226fffffu && (h & 0xfffffu) != 0xfffffu;
 }
 
 // a / d.b, correctly rounded

@@ -169,18 +169,18 @@ static __device__ __noinline__ double char_flux_each(const double2* pf, int ps, 
     return r0 + r1;
 }
 
-// entries 0 (acoustic rows only) to 2 of the row of L, for a face with a tiny velocity
+// entries 0 to 2 of the row of L, for a face with a tiny velocity
 template <int DIR>
-static __device__ __noinline__ LVel char_row_velocity(const double* Qf, const DevParams& P, int c) {
+static __device__ __noinline__ LVel char_row_velocity(const double* Qf, const DevParams& P, int c, bool square) {
     Roe q;
     load_q(Qf, q);
-    return l_row_velocity<DIR>(c, q, P);
+    return l_row_velocity<DIR>(c, q, P, square);
 }
 
-// g_c; mode: near_face's answer
+// g_c; mode: near_face's answer, not FACE_GENERAL; lo: weno_window
 template <int DIR>
 __device__ __forceinline__ double char_flux(const double2* pf, int ps, const double* Qf, const DevParams& P, int c,
-                                            const double* gkgt, int mode) {
+                                            const double* gkgt, int mode, unsigned lo) {
     Roe q;
     load_q(Qf, q);
     double Lc[6], fp[6], fm[6];
@@ -195,9 +195,9 @@ __device__ __forceinline__ double char_flux(const double2* pf, int ps, const dou
         rd.cg = {gt * q.cs2, Qf[17 * FLUX_FACES], Qf[18 * FLUX_FACES]};
         rd.scale();
         l_row<DIR>(c, q, rd, gkgt[energy_index<DIR>(c)], P, Lc);
-        if (mode == 2) {
-            const LVel l = char_row_velocity<DIR>(Qf, P, c);
-            if (c == 0 || c == 5) Lc[0] = l.l0;
+        if (mode != FACE_NEAR) {
+            const LVel l = char_row_velocity<DIR>(Qf, P, c, mode == FACE_SQUARE);
+            if (c == 0 || c == 5 || mode == FACE_SQUARE) Lc[0] = l.l0;
             Lc[1] = l.l1;
             Lc[2] = l.l2;
         }
@@ -209,9 +209,9 @@ __device__ __forceinline__ double char_flux(const double2* pf, int ps, const dou
     if (!kExact)
         return fastm::weno5(fp[0], fp[1], fp[2], fp[3], fp[4], P.eps) +
                fastm::weno5(fm[5], fm[4], fm[3], fm[2], fm[1], P.eps);
-    bool near = mode != 0;
-    const double r0 = weno5_near(fp[0], fp[1], fp[2], fp[3], fp[4], P.eps, near);
-    const double r1 = weno5_near(fm[5], fm[4], fm[3], fm[2], fm[1], P.eps, near);
+    bool near = true;
+    const double r0 = weno5_near(fp[0], fp[1], fp[2], fp[3], fp[4], P.eps, lo, near);
+    const double r1 = weno5_near(fm[5], fm[4], fm[3], fm[2], fm[1], P.eps, lo, near);
     return near ? r0 + r1 : char_flux_each<DIR>(pf, ps, Qf, P, c, gkgt[energy_index<DIR>(c)]);
 }
 
@@ -319,7 +319,7 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
     }
     __syncthreads();
     double* Qf = S.Q + f;
-    int near = 1; // near_face's answer
+    int near = FACE_NEAR; // near_face's answer
     if (valid && g == 0) {
         // points[3] and points[2] of the face: the staged primitives (the
         // same functions of the same states as a fresh evaluation)
@@ -335,7 +335,7 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
             q = roe_average_sqrt(rho3, d3, rho2, d2, P);
             RoeDivN rd;
             const double gt = (P.gamma_i - 1.0) + (P.gamma_e - 1.0) + (P.gamma_r - 1.0);
-            near = near_params(P) ? near_face(q, gt, rd) : 0;
+            near = near_gammas(P) && near_eps(P) ? near_face(q, gt, rd) : FACE_GENERAL;
             y[0] = rd.den.y; y[1] = rd.den.yl; y[2] = rd.b.y; y[3] = rd.b.yl; y[4] = rd.cg.y; y[5] = rd.cg.yl;
         } else {
             const double a6[6] = {rho3, d3.u, d3.v, d3.e_e, d3.e_i, d3.e_r};
@@ -357,12 +357,21 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
     // ---- 3. characteristic pass (a loop, not unrolled: one copy of its code
     // stays within the instruction cache)
     double* Gf = S.G + f;
+    const unsigned lo = kExact ? weno_window(P.eps) : 0u;
     const double2* pf = S.pt + PT * p0;
-    if (NG == 1 || valid) {
+    // (a face in the general form: a loop of its own with one thread a face; in the loop
+    // of all with several, where its registers spill: NG 2 64 B of stores against 0)
+    if (kExact && NG == 1 && near == FACE_GENERAL) {
+#pragma unroll 1
+        for (int c = 0; c < 6; ++c)
+            Gf[c * FLUX_FACES] = char_flux_each<DIR>(pf, PT * ps, Qf, P, c, S.gkgt[energy_index<DIR>(c)]);
+    } else if (NG == 1 || valid) {
 #pragma unroll 1
         for (int m = 0; m < 6 / NG; ++m) {
             const int c = NG == 1 ? m : group_field<DIR, NG>(g, m);
-            Gf[c * FLUX_FACES] = char_flux<DIR>(pf, PT * ps, Qf, P, c, S.gkgt, near);
+            Gf[c * FLUX_FACES] = kExact && NG > 1 && near == FACE_GENERAL
+                                     ? char_flux_each<DIR>(pf, PT * ps, Qf, P, c, S.gkgt[energy_index<DIR>(c)])
+                                     : char_flux<DIR>(pf, PT * ps, Qf, P, c, S.gkgt, near, lo);
         }
     }
     if (NG > 1) {
@@ -374,7 +383,7 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
     double *fo, *dfo;
     if (DIR == 0) { fplane = (long long)(nx + 1) * ny; fidx = (long long)i * ny + j; fo = I.fx; dfo = I.dfx; }
     else { fplane = (long long)nx * (ny + 1); fidx = (long long)i * (ny + 1) + j; fo = I.fy; dfo = I.dfy; }
-    if (!kExact || near) {
+    if (!kExact || near > 0) {
         Roe q;
         load_q(Qf, q);
 #pragma unroll

@@ -265,7 +265,7 @@ static __device__ __noinline__ void lr_velocity(const Roe* q, const DevParams& P
 #pragma unroll 1
     for (int row = 0; row < 6; ++row) {
         if (row == 4) continue;
-        const LVel l = l_row_velocity<0>(row, *q, P);
+        const LVel l = l_row_velocity<0>(row, *q, P, false);
         if (row == 0 || row == 5) LR[6 * row * CHUNK] = l.l0;
         LR[(6 * row + 1) * CHUNK] = l.l1;
         LR[(6 * row + 2) * CHUNK] = l.l2;
@@ -287,8 +287,8 @@ __device__ __forceinline__ void local_lr(const Inst& I, const GhostRec& Rg, int 
     const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
     const double gt = gi + ge + gr;
     RoeDivN rd;
-    const int mode = near_params(P) && den_mid_near(gt) ? near_face(q, gt, rd) : 0;
-    if (mode != 0) {
+    const int mode = near_gammas(P) && den_mid_near(gt) ? near_face(q, gt, rd) : FACE_GENERAL;
+    if (mode > 0) {
         if (!kExactG) {
             const RoeT<NearD> n = {q.u, q.v, q.w2, q.ee, q.ei, q.er, q.cs2, q.cs, q.he, q.hi, q.hr, q.b, q.den};
 #pragma unroll
@@ -303,7 +303,7 @@ __device__ __forceinline__ void local_lr(const Inst& I, const GhostRec& Rg, int 
                 }
                 LR[(GH_LR_LAM + row) * CHUNK] = lam.v;
             }
-            if (mode == 2) {
+            if (mode == FACE_VELOCITY) {
                 const Roe t = q;
                 lr_velocity(&t, P, LR);
             }
@@ -320,7 +320,7 @@ __device__ __forceinline__ void local_lr(const Inst& I, const GhostRec& Rg, int 
             r_row<0, true>(row, q, row >= 3 ? recip_near(6.0 * gk) : rgt, P, Rr);
             store_lr(LR, row, Lr, Rr, q);
         }
-        if (mode == 2) {
+        if (mode == FACE_VELOCITY) {
             const Roe t = q;
             lr_velocity(&t, P, LR);
         }

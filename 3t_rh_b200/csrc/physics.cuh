@@ -469,33 +469,40 @@ __device__ __forceinline__ RoeDiv roe_div(const Roe& q, const DevParams& P) {
 }
 
 // The branch-free form for a whole face: reciprocals of the five divisors
-// (rd), and whether the quotients of its rows of L and R are covered by the
-// argument in divrn.cuh: 1 if all are, 2 if all but the entries of L that
-// l_row_velocity forms, 0 otherwise. The divisors are within 2^-100..2^101, u and v
-// are zero or within 2^-790..2^101 and w2 is zero or at least 2^-800, so with the
-// gammas' factors gk, gt within 2^-20..2^22 (near_params) the numerators (gk, gt,
-// gk gt times u, v or w2, and gt w2 +- 6 vel cs, whose terms cancel to no less
-// than an ulp of 2^-840) are zero or at least 2^-904 and the quotients at least
-// 2^-1005: residuals are multiples of 2^-1008, so nothing underflows. A smaller
-// velocity is in the numerators of l_row_velocity's entries alone (those of R are
-// divided by 3, or hold w2). Such faces are common: ahead of a front a velocity
-// falls to zero through every magnitude (20 steps into the 121 x 481 half-cylinder a
-// third of the nodes hold one below 2^-430). With a face 0 for any velocity below
-// 2^-430 that state's fluxes took 294 us a step (general form throughout: 206 us),
-// now 132 us; the test of a third answer costs other states 0.8%.
-__device__ __forceinline__ bool near_params(const DevParams& P) {
+// (rd), and which quotients of its rows of L and R are covered by the argument in
+// divrn.cuh: FACE_NEAR for all, FACE_VELOCITY for all but the entries of L with a
+// velocity in the numerator, FACE_SQUARE for all but those and the entries of L and R
+// with w2; FACE_GENERAL for none.
+//
+// The divisors 12 cs2, 6 cs2, 3 cs2 and gt cs2 lie within 2^-102..2^101, |u| and |v| are
+// below 2^101, and gk, gt within 2^-40..2^22 (near_gammas). b = gt (36 ge gi gr +
+// gt w2^2) cs2 grows like the sixth power of the speed (in m/s, ordinary flows have
+// b near 2^100, in cm/s near 2^145) and may reach 2^451. Let w2 be zero or at least
+// 2^-800, u and v zero or at least 2^-790, or, where b is 2^101 or more, 2^-440 and
+// 2^-430. Then the numerators over b (gk gt w2, 2 gk gt u or v, constants) are at least
+// 2^-879 and the quotients 2^-980, or 2^-519 and 2^-970 for the large b; over
+// the other divisors gk w2, gt w2, gk u, gt u are at least 2^-840, and gt w2 +- 6 vel cs is
+// zero or at least an ulp of its smaller term, 2^-892, over 2^101 at most: 2^-993.
+//
+// Smaller velocities are common: ahead of a front a velocity falls to zero through
+// every magnitude (20 steps into the 121 x 481 half-cylinder a third of the nodes
+// hold one below 2^-430). Fluxes of eight 121 x 481 half-cylinders, us a step, with
+// a test of every quotient and no branch-free form / both forms for a face beyond a
+// narrower range / now: the developed flow 1165 / 780 / 722, at 2^17 times its speed
+// 1161 / 2023 / 789, with eps 1e-40 1167 / 2003 / 717, gas at rest with velocities of 2^-420
+// 1226 / 1959 / 1040, a gamma of 1 + 2^-21 1160 / 2010 / 723, of 1 + 2^-41 1162 / 2010 / 1282;
+// 402 x 283 double Mach 305 / 296 / 203.
+enum { FACE_SQUARE = -1, FACE_GENERAL = 0, FACE_NEAR = 1, FACE_VELOCITY = 2 }; // above 0: R is covered
+__device__ __forceinline__ bool near_gammas(const DevParams& P) {
     const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
-    const double lo = 0x1p-20, hi = 0x1p20;
-    return ge >= lo && ge <= hi && gi >= lo && gi <= hi && gr >= lo && gr <= hi && P.eps >= 0x1p-100 &&
-           P.eps <= 0x1p100 && den_near(6.0 * ge) && den_near(6.0 * gi) && den_near(6.0 * gr);
+    const double lo = 0x1p-40, hi = 0x1p20;
+    return ge >= lo && ge <= hi && gi >= lo && gi <= hi && gr >= lo && gr <= hi && den_near(6.0 * ge) &&
+           den_near(6.0 * gi) && den_near(6.0 * gr);
 }
-__device__ __forceinline__ bool near_velocity(double a) {
+// |a| is zero or its high word at least lo (a finite)
+__device__ __forceinline__ bool zero_or_from(double a, unsigned lo) {
     const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    return h - 0x0e900000u <= 0x37afffffu || (h | (unsigned)__double2loint(a)) == 0u;
-}
-__device__ __forceinline__ bool near_square(double w2) {
-    const unsigned h = (unsigned)__double2hiint(w2);
-    return h >= 0x0df00000u || (h | (unsigned)__double2loint(w2)) == 0u;
+    return h >= lo || (h | (unsigned)__double2loint(a)) == 0u;
 }
 struct RoeDivN {
     RecipN den, b, c6, c3, cg;
@@ -510,9 +517,12 @@ __device__ __forceinline__ int near_face(const Roe& q, double gt, RoeDivN& rd) {
     rd.den = recip_near(q.den);
     rd.b = recip_near(q.b);
     rd.cg = recip_near(cg);
-    const bool ok = den_mid_near(q.den) & den_mid_near(q.b) & den_mid_near(cg) & near_square(q.w2) &
-                    (fabs(q.u) < most) & (fabs(q.v) < most);
-    return ok ? (near_velocity(q.u) & near_velocity(q.v) ? 1 : 2) : 0;
+    const bool ok = den_mid_near(q.den) & den_wide_near(q.b) & den_mid_near(cg) & (fabs(q.u) < most) & (fabs(q.v) < most);
+    const bool big = q.b >= 0x1p101;
+    const unsigned sq = big ? 0x24700000u : 0x0df00000u, vel = big ? 0x25100000u : 0x0e900000u; // 2^-440, -800; -430, -790
+    if (!ok) return FACE_GENERAL;
+    if (!zero_or_from(q.w2, sq)) return FACE_SQUARE;
+    return zero_or_from(q.u, vel) & zero_or_from(q.v, vel) ? FACE_NEAR : FACE_VELOCITY;
 }
 
 __device__ __forceinline__ double quot(double a, const Recip& d) { return div_rn(a, d); }
@@ -577,14 +587,14 @@ __device__ __forceinline__ void l_row(int row, const Roe& q, const RD& rd, doubl
     }
 }
 
-// The entries of row `row` whose numerators a velocity below near_velocity's range
-// can take out of the branch-free form's, by IEEE quotients: the first three of an
-// acoustic row, the second and third of an energy row
+// The entries of row `row` with a velocity in the numerator, by IEEE quotients: the
+// first three of an acoustic row, the second and third of an energy row; the
+// first of an energy row holds w2 (formed if square)
 struct LVel {
     double l0, l1, l2;
 };
 template <int DIR>
-__device__ __forceinline__ LVel l_row_velocity(int row, const Roe& q, const DevParams& P) {
+__device__ __forceinline__ LVel l_row_velocity(int row, const Roe& q, const DevParams& P, bool square) {
     const double gi = P.gamma_i - 1.0, ge = P.gamma_e - 1.0, gr = P.gamma_r - 1.0;
     const double gt = gi + ge + gr;
     const double u = q.u, v = q.v, w2 = q.w2, cs = q.cs, cs2 = q.cs2;
@@ -598,7 +608,9 @@ __device__ __forceinline__ LVel l_row_velocity(int row, const Roe& q, const DevP
     const int k = mode - 2;
     const double gk = k == 0 ? ge : (k == 1 ? gi : gr), hk = k == 0 ? q.he : (k == 1 ? q.hi : q.hr);
     const double c3 = 3.0 * cs2, h = hk - cs2 * w2;
-    return {0.0, __ddiv_rn(gk * u, c3) + __ddiv_rn(2.0 * gk * gt * u, q.b) * h,
+    double l0 = 0.0;
+    if (square) l0 = __ddiv_rn(gk, gt) - __ddiv_rn(gk * w2, 6.0 * cs2) - __ddiv_rn(gk * gt * w2, q.b) * h;
+    return {l0, __ddiv_rn(gk * u, c3) + __ddiv_rn(2.0 * gk * gt * u, q.b) * h,
             __ddiv_rn(gk * v, c3) + __ddiv_rn(2.0 * gk * gt * v, q.b) * h};
 }
 
@@ -738,14 +750,31 @@ __device__ __forceinline__ double weno5(double u0, double u1, double u2, double 
     return w0 * p0 + w1 * p1 + w2 * p2;
 }
 
-// weno5 in the branch-free form (divrn.cuh); ok is cleared when an operand is
-// outside its range (then the value is not used). Numerators need no test: the
-// 0.1, 0.6, 0.3 and the alphas they give are bounded by the divisors' range;
+// eps^2, the least divisor of a WENO5, is 2^-960 or more
+__device__ __forceinline__ bool near_eps(const DevParams& P) { return P.eps >= 0x1p-480 && P.eps <= 0x1p224; }
+// High word of the first of the 901 binades that the divisors (eps + beta)^2 of a WENO5
+// may lie in: 2^-450, or that of eps^2 where it is less. 0.1, 0.6 and 0.3 over them
+// are within 2^-455..2^960 and within 2^905 of each other, so the weights are at least
+// 2^-906, wherever the range lies
+__device__ __forceinline__ unsigned weno_window(double eps) {
+    const unsigned e = 2u * ((unsigned)__double2hiint(eps) >> 20) - 1023u;
+    return (e < 573u ? e : 573u) << 20;
+}
+__device__ __forceinline__ bool den_in(double b, unsigned lo) {
+    const unsigned h = (unsigned)__double2hiint(b);
+    return h - lo <= 0x384fffffu && (h & 0xfffffu) != 0xfffffu;
+}
+
+// weno5 in the branch-free form (divrn.cuh), for an eps that near_eps accepts (lo: its
+// weno_window, formed once a face: in here it cost 0.5% of the fluxes' time); ok is
+// cleared when an operand is outside its range (then the value is not used).
+// Numerators need no test: the 0.1, 0.6, 0.3 and the alphas they give are bounded by
+// the divisors' range, and so is the alphas' sum but for its leading fraction bits;
 // u / 3 and u / 6 hold for every finite u, and a u that is not finite makes one of the
 // three divisors infinite or NaN. (0.25 r^2 in one FMA differs from its rounded
 // product where that is subnormal alone, which no divisor in range can show.)
 __device__ __forceinline__ double weno5_near(double u0, double u1, double u2, double u3, double u4, double eps,
-                                             bool& ok) {
+                                             unsigned lo, bool& ok) {
     // products by 2, 4 and 1/4 are exact, so their sums are one FMA each
     const double c1312 = 13.0 / 12.0, u23 = __dmul_rn(3.0, u2);
     const double t2 = __dadd_rn(__fma_rn(-2.0, u3, u2), u4), r2 = __dadd_rn(__fma_rn(-4.0, u3, u23), u4);
@@ -762,7 +791,7 @@ __device__ __forceinline__ double weno5_near(double u0, double u1, double u2, do
     const double p0 = div3_near(u0) - 7.0 / 6.0 * u1 + 11.0 / 6.0 * u2;
     const double p1 = div6_near(-u1) + 5.0 / 6.0 * u2 + div3_near(u3);
     const double p2 = div3_near(u2) + 5.0 / 6.0 * u3 - div6_near(u4);
-    ok = ok & den_near(s0) & den_near(s1) & den_near(s2) & den_near(sum_o);
+    ok = ok & den_in(s0, lo) & den_in(s1, lo) & den_in(s2, lo) & ((__double2hiint(sum_o) & 0xfffff) != 0xfffff);
     return w0 * p0 + w1 * p1 + w2 * p2;
 }
 
