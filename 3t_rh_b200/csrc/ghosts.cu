@@ -717,16 +717,16 @@ void launch_ghosts(cudaStream_t s, const Inst* insts, const GhostRec* heavy, int
                    const double* hrec, double* lrbuf, int stage, bool ordered) {
     if (nh + nc <= 0) return;
     static OncePerDevice attributes;
-    int dev = 0, sms = 0;
+    int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = multiprocessors(dev);
     attributes(dev, [] {
         return cudaFuncSetAttribute(k_ghosts, cudaFuncAttributeMaxDynamicSharedMemorySize, GH_SMEM) == cudaSuccess;
     });
     auto launch = [&](int h, int c, int part) {
         const int n = std::max((h + 1) / 2, (6 * c + GH_WARPS * 32 - 1) / (GH_WARPS * 32));
         if (n > 0)
-            k_ghosts<<<std::min(n, std::max(sms, 1)), GH_WARPS * 32, GH_SMEM, s>>>(insts, heavy, h, cheap, c, hrec, lrbuf,
+            k_ghosts<<<std::min(n, sms), GH_WARPS * 32, GH_SMEM, s>>>(insts, heavy, h, cheap, c, hrec, lrbuf,
                                                                                  stage, part);
     };
     if (!ordered) {

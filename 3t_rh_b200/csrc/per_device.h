@@ -4,6 +4,8 @@
 #pragma once
 #include <atomic>
 
+#include <cuda_runtime.h>
+
 namespace rh3t {
 
 class OncePerDevice {
@@ -18,5 +20,17 @@ class OncePerDevice {
         if (setup() && kept) done[dev].store(true, std::memory_order_release);
     }
 };
+
+// multiprocessors of device dev, asked for once
+inline int multiprocessors(int dev) {
+    constexpr int MAX = 64;
+    static std::atomic<int> known[MAX] = {};
+    const bool kept = dev >= 0 && dev < MAX;
+    int n = kept ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (n > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 1;
+    if (kept) known[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
 
 } // namespace rh3t
