@@ -652,8 +652,9 @@ class Batch(_SnapshotIO):
         return tuple(int(x) for x in a)
 
     def autotune(self, cache_path=None, reps=5):
-        """Time every admissible tile shape per (nx, ny, diffusion) class and
-        apply the fastest; returns one dict per class."""
+        """Time every admissible tile shape per (nx, ny, diffusion) class, in the
+        launches of a step, and apply the fastest where it beats the default
+        by 3%; returns one dict per class."""
         out = (_lib.TuneEntry * 64)()
         n = C.c_int32()
         path = cache_path.encode() if cache_path else None

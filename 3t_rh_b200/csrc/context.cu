@@ -128,6 +128,31 @@ int make_tiles(rh3t_ctx* c) {
     return RH3T_OK;
 }
 
+// Tile shapes of an nx x ny grid before any tuning: the default, unless another
+// shape covers the grid in a tenth fewer tiles. A cell tile counts by its time: the
+// wider it is, the more nodes its stencils reach (961 x 3841 cells: 864 us a step in
+// 16 x 16, 898 us in 8 x 32, 1206 us in 4 x 64).
+Shape default_shape(long nx, long ny) {
+    auto tiles = [](long n, long m, int area, int lg) {
+        const long rows = area >> lg, cols = 1L << lg;
+        return ((n + rows - 1) / rows) * ((m + cols - 1) / cols);
+    };
+    auto pick = [](int lo, int hi, int def, auto cost) {
+        int best = def;
+        for (int lg = lo; lg <= hi; ++lg)
+            if (cost(lg) < cost(best) && 10 * cost(lg) < 9 * cost(def)) best = lg;
+        return best;
+    };
+    Shape s;
+    s.lgx = pick(FX_LG_MIN, FX_LG_MAX, FX_LG_DEF, [&](int lg) { return tiles(nx + 1, ny, FLUX_FACES, lg); });
+    s.lgy = pick(FY_LG_MIN, FY_LG_MAX, FY_LG_DEF, [&](int lg) { return tiles(nx, ny + 1, FLUX_FACES, lg); });
+    s.lgr = pick(RHS_LG_MIN, RHS_LG_MAX, RHS_LG_DEF, [&](int lg) {
+        const int weight[] = {25, 26, 35};
+        return tiles(nx, ny, RHS_THREADS, lg) * weight[lg - RHS_LG_MIN];
+    });
+    return s;
+}
+
 // returns the number of kernels launched
 int enqueue_flux(rh3t_ctx* c, cudaStream_t s, int stage, Span r) {
     const HostInst &a = c->hi[r.k0], &b = c->hi[r.k1 - 1];
@@ -239,31 +264,6 @@ struct Built {
     int n_heavy = 0;
     bool ordered = false;       // the ghost update's order matters (kernels.cuh launch_ghosts)
 };
-
-// Tile shapes of an nx x ny grid before any tuning: the default, unless another
-// shape covers the grid in a tenth fewer tiles. A cell tile counts by its time: the
-// wider it is, the more nodes its stencils reach (961 x 3841 cells: 864 us a step in
-// 16 x 16, 898 us in 8 x 32, 1206 us in 4 x 64).
-Shape default_shape(long nx, long ny) {
-    auto tiles = [](long n, long m, int area, int lg) {
-        const long rows = area >> lg, cols = 1L << lg;
-        return ((n + rows - 1) / rows) * ((m + cols - 1) / cols);
-    };
-    auto pick = [](int lo, int hi, int def, auto cost) {
-        int best = def;
-        for (int lg = lo; lg <= hi; ++lg)
-            if (cost(lg) < cost(best) && 10 * cost(lg) < 9 * cost(def)) best = lg;
-        return best;
-    };
-    Shape s;
-    s.lgx = pick(FX_LG_MIN, FX_LG_MAX, FX_LG_DEF, [&](int lg) { return tiles(nx + 1, ny, FLUX_FACES, lg); });
-    s.lgy = pick(FY_LG_MIN, FY_LG_MAX, FY_LG_DEF, [&](int lg) { return tiles(nx, ny + 1, FLUX_FACES, lg); });
-    s.lgr = pick(RHS_LG_MIN, RHS_LG_MAX, RHS_LG_DEF, [&](int lg) {
-        const int weight[] = {25, 26, 35};
-        return tiles(nx, ny, RHS_THREADS, lg) * weight[lg - RHS_LG_MIN];
-    });
-    return s;
-}
 
 // Validates one instance description and resolves its ghost records
 // (ghost.rs:18-46, bc1.rs:50-57 and the static parts of the cheap BCs).

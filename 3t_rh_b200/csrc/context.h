@@ -80,6 +80,8 @@ struct rh3t_ctx {
 namespace rh3t {
 int set_error(rh3t_ctx* c, int code, const char* what);
 int cuda_check(rh3t_ctx* c, cudaError_t e, const char* where);
+// tile shapes of an nx x ny grid before any tuning
+Shape default_shape(long nx, long ny);
 // rebuild and upload every tile list from the instances' shapes (drops the graph)
 int make_tiles(rh3t_ctx* c);
 // x-face, y-face and RHS tiles of one instance for a given shape

@@ -241,16 +241,18 @@ int rh3t_get_tile_shapes(const rh3t_ctx* ctx, int32_t k, int32_t* lg3);
 
 /* Autotuner: instances are grouped into classes by (nx, ny, diffusion on);
  * for each class every admissible shape of each of the three tile kinds is
- * timed on the class's own instances (CUDA events, `reps` launches, the
- * minimum kept) and the fastest is applied. Results are cached per class in
- * the process and, when cache_path is not NULL, in that text file (read
- * first, rewritten after). out (may be NULL) receives up to max_out
+ * timed in the launch that a step makes (the faces of both directions, or the
+ * cells, of all the context's instances; CUDA events, `reps` launches, the
+ * minimum kept), and the fastest is applied if it beats the default by 3%.
+ * Results are cached per class in the process and, when cache_path is not
+ * NULL, in that text file (read first, unless an earlier version of the
+ * kernels wrote it; rewritten after). out (may be NULL) receives up to max_out
  * entries, one per class. Time it after uploading a state. */
 typedef struct {
     int32_t nx, ny, diffusion, n_instances;
     int32_t lg_fx, lg_fy, lg_rhs;
     int32_t from_cache;
-    double ms_fx[3], ms_fy[3], ms_rhs[3]; /* per admissible shape, ascending lg; 0 if from cache */
+    double ms_fx[3], ms_fy[3], ms_rhs[3]; /* the launch's time per admissible shape, ascending lg; 0 if from cache */
 } rh3t_tune_entry;
 int rh3t_autotune(rh3t_ctx* ctx, const char* cache_path, int32_t reps, rh3t_tune_entry* out, int32_t max_out,
                   int32_t* n_out);
