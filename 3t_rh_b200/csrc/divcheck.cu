@@ -4,8 +4,8 @@
 // next to a rounding midpoint, operands at and beyond the fast path's
 // exponent range, and special values; and the reciprocals of a face's
 // L-row divisors that roe_div (physics.cuh) forms by scaling 1/(12 c^2). The
-// branch-free routines are checked on the same operands wherever their range
-// tests accept them.
+// branch-free routines are checked on the same operands, zeros and subnormal
+// sixths among them, and on others in the widest range in which each is used.
 #include <cstdint>
 
 #include <cuda_runtime.h>
@@ -45,23 +45,44 @@ __device__ __forceinline__ bool same_bits(double x, double y) {
 
 constexpr int DIV_CATEGORIES = 7;
 
-// the branch-free quotient of case (a, b), or `want` where its range tests
-// refuse the operands (a / 3 and a / 6: any finite a, subnormals among them)
+// exponent of a normal number
+__device__ __forceinline__ int exponent(double a) { return ((__double2hiint(a) >> 20) & 0x7ff) - 1023; }
+
+// a and b within what div_near admits: b > 0 with an exponent in [-450, 450] and
+// leading fraction bits that are not all ones, a zero or of exponent -969 or more with
+// |a / b| in [2^-1000, 2^1000]
+__device__ __forceinline__ bool div_near_admits(double a, double b) {
+    if (!den_near(b)) return false;
+    if (a == 0.0) return true;
+    const int e = exponent(a) - exponent(b);
+    return isfinite(a) && exponent(a) >= -969 && e >= -999 && e <= 999;
+}
+
+// the branch-free quotient of case (a, b), or `want` where it is not used for such
+// operands (a / 3 and a / 6: any finite a, subnormals among them). Every routine's
+// range tests have to imply what is checked here.
 __device__ __forceinline__ double near_quotient(int cat, double a, double b, double want) {
     if (cat == 4 || cat == 5) {
         if (!isfinite(a)) return want;
-        // the same operand scaled into the subnormal range and its edge
-        const int sh = (int)((unsigned)__double2loint(a) % 120u) - 1070;
-        const double t = scalbn(a, sh - ilogb(a));
-        const double got3 = div3_near(t), got6 = div6_near(t);
-        if (cat == 4 && !same_bits(got3, __ddiv_rn(t, 3.0))) return got3;
-        if (cat == 5 && !same_bits(got6, __ddiv_rn(t, 6.0))) return got6;
+        if (a != 0.0) {
+            // the same operand scaled into the subnormal range and its edge, and a
+            // quotient by 6 that is a tie there
+            const unsigned w = (unsigned)__double2loint(a);
+            const int sh = (int)(w % 120u) - 1070;
+            const unsigned long long odd = 6ull * ((unsigned long long)__double_as_longlong(a) >> (14 + w % 49u)) + 3ull;
+            const double t = scalbn(a, sh - ilogb(a)), u = (double)odd * 0x1p-1074; // (below 2^53 units: exact)
+            if (cat == 4 && !same_bits(div3_near(t), __ddiv_rn(t, 3.0))) return div3_near(t);
+            if (cat == 5 && !same_bits(div6_near(t), __ddiv_rn(t, 6.0))) return div6_near(t);
+            if (cat == 5 && !same_bits(div6_near(u), __ddiv_rn(u, 6.0))) return div6_near(u);
+            if (cat == 5 && !same_bits(div6_near(-u), __ddiv_rn(-u, 6.0))) return div6_near(-u);
+        }
         return cat == 4 ? div3_near(a) : div6_near(a);
     }
-    if (!den_near(b) || !num_near(a)) return want;
+    const bool groups = (den_near(b) && num_near(a)) || (den_mid_near(b) && num_small_near(a));
+    if (!div_near_admits(a, b)) return groups ? NAN : want; // (a group's tests admit too much)
     const double q = div_near(a, recip_near(b));
     if (!same_bits(q, want)) return q;
-    return a > 0.0 ? div_once(a, b) : q;
+    return a > 0.0 && den_near(b) && num_near(a) ? div_once(a, b) : q;
 }
 
 // category of case k: 0 random, 1 all-ones divisors, 2 near-midpoint
@@ -77,13 +98,23 @@ __global__ void k_div_check(long long n, unsigned long long seed, unsigned long 
         if (cat == 0) {
             a = make_double(h1, (int)(h3 % 941) - 470);
             b = make_double(h2, (int)((h3 >> 16) % 941) - 470);
+            if ((h3 >> 40) % 3 == 0) { // small numerators, as velocities ahead of a front
+                a = make_double(h1, (int)(h3 % 540) - 980);
+                b = make_double(h2 & ~(1ull << 63), (int)((h3 >> 16) % 556) - 102);
+            }
         } else if (cat == 1) {
             a = make_double(h1, (int)(h3 % 401) - 200);
             const uint64_t frac = 0x000fffffffffffffull - (h2 & 0xffull) - (((h3 >> 40) & 1) ? ((h2 >> 8) & 0xffffull) : 0);
             b = __longlong_as_double((long long)(((uint64_t)((int)((h3 >> 16) % 401) - 200 + 1023) << 52) | frac));
         } else if (cat == 2) {
             b = make_double(h1, (int)(h3 % 201) - 100);
-            a = near_midpoint(b, h2, (int)((h3 >> 16) % 201) - 100, (int)((h3 >> 40) % 7) - 3);
+            int e = (int)((h3 >> 16) % 201) - 100;
+            if ((h3 >> 50) & 1) { // quotients down to 2^-1000, numerators to 2^-969
+                b = make_double(h1 & ~(1ull << 63), (int)(h3 % 901) - 450);
+                e = max(-1000, -969 - exponent(b)) + (int)((h3 >> 16) % 64);
+            }
+            const double scale = e < -900 ? 0x1p-200 : 1.0; // (half an ulp of 2^-1000 is no normal number)
+            a = scale * near_midpoint(b, h2, e < -900 ? e + 200 : e, (int)((h3 >> 40) % 7) - 3);
         } else if (cat == 3) {
             const double specials[12] = {0.0, -0.0, INFINITY, -INFINITY, NAN, 4.9e-324, 2.2250738585072014e-308,
                                          1.7976931348623157e308, 0x1p-450, 0x1p450, 0x1.fffffffffffffp-451,
@@ -122,12 +153,23 @@ __global__ void k_div_check(long long n, unsigned long long seed, unsigned long 
             b = cat == 4 ? 3.0 : 6.0;
             if ((h3 & 1) == 0) a = make_double(h1, (int)(h3 % 1001) - 500);
             else a = near_midpoint(b, h2, (int)((h3 >> 16) % 201) - 100, (int)((h3 >> 40) % 7) - 3);
+            if ((h3 >> 50) % 64 == 0) a = (h3 >> 56) & 1 ? -0.0 : 0.0;
         }
-        const double want = __ddiv_rn(a, b);
+        double want = __ddiv_rn(a, b);
         if (cat == 4) got = div3_rn(a);
         else if (cat == 5) got = div6_rn(a);
         else got = div_rn(a, recip(b));
         if (same_bits(got, want)) got = near_quotient(cat, a, b, want);
+        if (cat == 0 && same_bits(got, want)) { // and a WENO5's alpha, over the range of its divisors
+            const double c = h3 % 3 == 0 ? 0.1 : (h3 % 3 == 1 ? 0.6 : 0.3);
+            const double s = make_double(h2 & ~(1ull << 63), (int)((h3 >> 30) % 1412) - 960);
+            if (((unsigned)__double2hiint(s) & 0xfffffu) != 0xfffffu) {
+                a = c;
+                b = s;
+                got = div_once(c, s);
+                want = __ddiv_rn(c, s);
+            }
+        }
         if (!same_bits(got, want)) {
             atomicAdd(&bad[cat], 1ull);
             if (atomicAdd(&bad[DIV_CATEGORIES], 1ull) == 0) {
