@@ -399,7 +399,8 @@ __device__ __forceinline__ void flux_tile(const Inst& I, const Tile& t, int stag
 }
 
 constexpr int FLUX_NG3 = 2 * 148, FLUX_NG2 = 4 * 148; // tiles up to which 3 and 2 groups share a tile
-// blocks per SM (FMA build: 12 blocks of 80 registers 2% faster than 8)
+// blocks per SM (FMA build: bounds of 12, 80 registers, 2% faster than of 8; shared
+// memory admits 9 blocks of default tiles, 7 with an x tile of 4 x 16)
 constexpr int FLUX_MIN_BLOCKS = kExact ? 8 : 12;
 // x faces (blocks [0, ntx)), then y faces: in one launch the y tiles fill the
 // SMs that the last x tiles leave idle (121 x 481: two launches of 0.8 waves each
@@ -437,12 +438,17 @@ void launch_flux(cudaStream_t s, const Inst* insts, const Tile* tx, int ntx, con
     const int n = ntx + nty, smem = flux_smem(np, z.diffusion);
     // (FMA build: one instantiation, since another might contract other sums, and
     // an instance's result must not depend on what else the launch holds)
-    if (kExact && n <= FLUX_NG3)
-        k_flux<3><<<n, 3 * FLUX_FACES, smem, s>>>(insts, tx, ntx, ty, stage, z.npx, z.npy);
-    else if (kExact && n <= FLUX_NG2)
-        k_flux<2><<<n, 2 * FLUX_FACES, smem, s>>>(insts, tx, ntx, ty, stage, z.npx, z.npy);
-    else
-        k_flux<1><<<n, FLUX_FACES, smem, s>>>(insts, tx, ntx, ty, stage, z.npx, z.npy);
+    if constexpr (kExact) {
+        if (n <= FLUX_NG3) {
+            k_flux<3><<<n, 3 * FLUX_FACES, smem, s>>>(insts, tx, ntx, ty, stage, z.npx, z.npy);
+            return;
+        }
+        if (n <= FLUX_NG2) {
+            k_flux<2><<<n, 2 * FLUX_FACES, smem, s>>>(insts, tx, ntx, ty, stage, z.npx, z.npy);
+            return;
+        }
+    }
+    k_flux<1><<<n, FLUX_FACES, smem, s>>>(insts, tx, ntx, ty, stage, z.npx, z.npy);
 }
 
 int flux_launches(int ntx, int nty) { return ntx + nty > 0 ? 1 : 0; }
