@@ -15,7 +15,7 @@
 //   4. output pass: (R g)_k = sum_c R[k][c] g_c in the reference's summation
 //      order (weno.rs:793, 834-843), plus the diffusion flux for k >= 3.
 //
-// Bound by the FP64 pipe (72% busy in the no-contraction build; a loop of
+// Bound by the FP64 pipe (65-72% busy in the no-contraction build; a loop of
 // independent FMAs reaches 92%), at about 2,850 FP64 operations a face. A face
 // per thread instead of a field per warp: nothing but the staged points
 // crosses threads, so the two warps meet one barrier of equal work (with six
@@ -23,9 +23,10 @@
 // issued instruction), and the quotients a face's rows share are formed once.
 // 8 blocks of 128 registers: 10 blocks of 96 spill (3% slower), 6 blocks of 150
 // 4% slower. Without a branch per quotient (divrn.cuh), in this form and in one launch
-// the fluxes of 24 batch instances take 1.24 ms a step instead of 2.08 ms, of the
-// 961 x 3841 half-cylinder 4.67 ms instead of 7.44 ms (same bits); FMA build
-// 0.90 ms instead of 1.17 ms.
+// the fluxes of 24 batch instances take 1.25 ms a step instead of 2.08 ms, of the
+// 961 x 3841 half-cylinder 4.75 ms instead of 7.44 ms (same bits); FMA build
+// 0.89 ms instead of 1.17 ms. (A face whose state is out of the branch-free form's
+// range, physics.cuh near_face: the general form, face by face.)
 //
 // RH3T_EXACT selects the reference's expressions; otherwise the fastm forms
 // (shared reciprocals, one division per WENO5) are used.
